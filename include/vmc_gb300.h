@@ -183,6 +183,14 @@ int vmc_nnbf_local_energy(int prec, const void* const* net_ptrs, int n_sites, in
 int vmc_nnbf_logpsi_grad(int prec, const void* const* gnet, int n_sites, int nf, int hidden, double bf_scale,
                          const uint64_t* occ, int64_t B, void* O_full, int64_t ld_full, void* O_dense,
                          int64_t ld_dense, void* kron_g, void* kron_h, double* logabs, double* sign, void* stream);
+/* The FP32 adjoint (prec 0 of vmc_nnbf_logpsi_grad, same gnet and outputs) as
+ * batched stages over work_rows configurations at a time, for batches: work
+ * (16-byte aligned) of *bytes from vmc_nnbf_grad_work_bytes. */
+int vmc_nnbf_grad_work_bytes(int n_sites, int nf, int64_t work_rows, int64_t* bytes);
+int vmc_nnbf_logpsi_grad_ws(const void* const* gnet, int n_sites, int nf, int hidden, double bf_scale,
+                            const uint64_t* occ, int64_t B, float* O_full, int64_t ld_full, float* O_dense,
+                            int64_t ld_dense, float* kron_g, float* kron_h, double* logabs, double* sign, void* work,
+                            int64_t work_rows, void* stream);
 
 /* ---- Learned Metropolis-Hastings proposal (no reference counterpart: the
  * reference samples with local exchange/hop moves only, vmc_torch/GPU/sampler.py:47-137).
@@ -276,6 +284,11 @@ int vmc_nnbf_eval_noalloc(const void* const* net_ptrs, int n_sites, int nf, int 
 int vmc_check_finite(const double* amp, const double* sign, int64_t B, const void* O, int dtype, int64_t Np,
                      int64_t ldo, unsigned long long* d_counts, uint8_t* d_row_bad, uint8_t* d_col_bad,
                      unsigned long long* h_counts, void* stream);
+/* Rows r of O (B, Np, ld ldo, dtype 0 f64 / 1 f32) with logabs[r] < log_min become
+ * zero (the gradient of the reference's clamped log-amplitude,
+ * vmc_torch/GPU/models/_base.py:101-109); a NaN logabs leaves its row. */
+int vmc_floor_rows(const double* logabs, double log_min, int64_t B, void* O, int dtype, int64_t Np, int64_t ldo,
+                   void* stream);
 
 /* ---- minSR in sample space (dtype: 0 = float64, 1 = float32 for O / Oc) ---- */
 int vmc_sr_center(const void* O, int dtype, int64_t Ns, int64_t Np, int64_t ldo, void* Oc, int64_t ldc, double* mean,

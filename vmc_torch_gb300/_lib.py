@@ -48,6 +48,7 @@ SIGNATURES = {
     "vmc_nnbf_eval_noalloc": [P, I32, I32, I32, F64, P, I64, P, P, P, P],
     "vmc_nnbf_hidden_layer": [P, I64, P, P, P, U64, I32, P, P],
     "vmc_check_finite": [P, P, I64, P, I32, I64, I64, P, P, P, P, P],
+    "vmc_floor_rows": [P, F64, I64, P, I32, I64, I64, P],
     "vmc_prop_logits": [P, I32, P, I64, P, P, P, P, P, P],
     "vmc_prop_sample": [P, I32, I32, P, P, I64, U64, U64, P, P, P],
     "vmc_prop_reverse": [P, I32, I32, P, P, I64, P, P],
@@ -57,6 +58,8 @@ SIGNATURES = {
     "vmc_prop_inputs_f32": [I32, P, I64, P, P],
     "vmc_prop_collect_targets": [P, I64, P, F64, I32, I64, P, P],
     "vmc_nnbf_logpsi_grad": [I32, P, I32, I32, I32, F64, P, I64, P, I64, P, I64, P, P, P, P, P],
+    "vmc_nnbf_grad_work_bytes": [I32, I32, I64, P],
+    "vmc_nnbf_logpsi_grad_ws": [P, I32, I32, I32, F64, P, I64, P, I64, P, I64, P, P, P, P, P, I64, P],
     "vmc_nnbf_conn_count": [P, I64, I32, P, I32, P, P],
     "vmc_nnbf_conn_pairs": [P, I64, I32, P, I32, P, P, P],
     "vmc_nnbf_local_energy": [I32, P, I32, I32, I32, F64, P, I64, P, F64, F64, P, P, P, P, P, I64, I64, P, P, P, P,

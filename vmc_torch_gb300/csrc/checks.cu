@@ -59,6 +59,17 @@ __global__ void k_check_rows(const T* __restrict__ O, int64_t Np, int64_t ld, un
   }
 }
 
+// Rows of O whose log-amplitude lies below log_min become zero; the others are
+// not touched (the amplitudes decide which rows are written at all: 8 bytes read
+// per row instead of a pass over O).
+template <typename T>
+__global__ void k_floor_rows(const double* __restrict__ logabs, double log_min, T* __restrict__ O, int64_t Np,
+                             int64_t ld) {
+  const int64_t r = blockIdx.x;
+  if (!(logabs[r] < log_min)) return;
+  for (int64_t j = threadIdx.x; j < Np; j += blockDim.x) O[r * ld + j] = T(0);
+}
+
 }  // namespace
 
 extern "C" int vmc_check_finite(const double* amp, const double* sign, int64_t B, const void* O, int dtype,
@@ -85,5 +96,17 @@ extern "C" int vmc_check_finite(const double* amp, const double* sign, int64_t B
     return VMC_ERR_CUDA;
   if (h_counts[0] || h_counts[1] || h_counts[3]) return VMC_ERR_NONFINITE;
   if (h_counts[2]) return VMC_ERR_SINGULAR;
+  return VMC_OK;
+}
+
+extern "C" int vmc_floor_rows(const double* logabs, double log_min, int64_t B, void* O, int dtype, int64_t Np,
+                              int64_t ldo, void* stream) {
+  if (B < 0 || B > INT32_MAX || Np < 0 || ldo < Np || (dtype != 0 && dtype != 1)) return VMC_ERR_ARGS;
+  if (B == 0 || Np == 0) return VMC_OK;
+  if (!logabs || !O) return VMC_ERR_ARGS;
+  cudaStream_t st = (cudaStream_t)stream;
+  if (dtype == 0) k_floor_rows<double><<<(unsigned)B, 256, 0, st>>>(logabs, log_min, (double*)O, Np, ldo);
+  else k_floor_rows<float><<<(unsigned)B, 256, 0, st>>>(logabs, log_min, (float*)O, Np, ldo);
+  VMC_CUDA_CHECK_LAUNCH();
   return VMC_OK;
 }

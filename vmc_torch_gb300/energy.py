@@ -126,12 +126,12 @@ def _floor_rows(O, logabs):
     """Zero the O rows of walkers below the 1e-45 amplitude floor (the
     gradient of the reference's clamp), without a host synchronisation."""
     from .optimizer import FactoredO
-    small = (logabs < LOG_MIN).unsqueeze(1)
-    if isinstance(O, FactoredO):
-        for t in (O.dense, O.g, O.h):
-            t.masked_fill_(small, 0)
-    else:
-        O.masked_fill_(small, 0)
+    for t in (O.dense, O.g, O.h) if isinstance(O, FactoredO) else (O,):
+        if t.dtype in (torch.float64, torch.float32) and (t.shape[1] <= 1 or t.stride(1) == 1):
+            _lib.call("vmc_floor_rows", _lib.ptr(logabs), LOG_MIN, t.shape[0], _lib.ptr(t),
+                      0 if t.dtype == torch.float64 else 1, t.shape[1], t.stride(0), _lib.stream_of(t.device))
+        else:
+            t.masked_fill_((logabs < LOG_MIN).unsqueeze(1), 0)
 
 
 def compute_grads_factored(fxs, model, use_log_amp=True, **kwargs):
@@ -169,7 +169,6 @@ def compute_grads_gpu(fxs, model, batch_size=None, verbose=False, offload_to_cpu
         la = floor_log(st.logabs)
         sign = st.sign.clone()
         amps = sign * torch.exp(st.logabs)
-        small = st.logabs < LOG_MIN
         if not offload_to_cpu:
             if bs >= B:
                 O = model.logpsi_grad(st)
@@ -185,7 +184,7 @@ def compute_grads_gpu(fxs, model, batch_size=None, verbose=False, offload_to_cpu
                     else:
                         model.logpsi_grad(st.view(a, b), out=O[a:b])
             model.check_status(st, wait=True)
-            O.masked_fill_(small.unsqueeze(1), 0)
+            _floor_rows(O, st.logabs)
             _check_grads_amps(O, la if use_log_amp else amps, sign, model)
             if use_log_amp:
                 return O, (sign, la)
@@ -209,7 +208,7 @@ def compute_grads_gpu(fxs, model, batch_size=None, verbose=False, offload_to_cpu
                 bufs[i] = Oc
             if Oh is None:
                 Oh = torch.empty((B, Np), dtype=Oc.dtype, pin_memory=True)
-            Oc.masked_fill_(small[a:b].unsqueeze(1), 0)
+            _floor_rows(Oc, v.logabs)
             n_bad += _count(None, None, Oc, Np, st.device)[1][3]
             if not use_log_amp:
                 Oc.mul_(amps[a:b].to(Oc.dtype).unsqueeze(1))

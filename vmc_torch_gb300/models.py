@@ -505,29 +505,41 @@ class NNBF_GB300(WavefunctionModel_GB300):
     def n_params_out_w(self):
         return self.n_orbitals * self.n_fermions * self.hidden_dim
 
+    # configurations per pass of the batched FP32 adjoint: the orbital matrices
+    # and the output layer's cotangents of 2048 (32 + 64 MB at 8x8) stay in L2
+    GRAD_ROWS = 2048
+
+    def _adjoint(self, st, full=None, dense=None, g=None, h=None):
+        ts, arr = self.grad_net(st.device)
+        s = _lib.stream_of(st.device)
+        args = (arr, self.n_sites, self.n_fermions, self.hidden_dim, self.bf_scale, _lib.ptr(st.occ), st.B,
+                _lib.ptr(full), 0 if full is None else full.stride(0),
+                _lib.ptr(dense), 0 if dense is None else dense.stride(0), _lib.ptr(g), _lib.ptr(h), None, None)
+        if self._prec != 0:
+            _lib.call("vmc_nnbf_logpsi_grad", self._prec, *args, s)
+            return
+        rows = max(1, min(st.B, self.GRAD_ROWS))
+        nbytes = ctypes.c_int64(0)
+        _lib.call("vmc_nnbf_grad_work_bytes", self.n_sites, self.n_fermions, rows, ctypes.byref(nbytes))
+        work = torch.empty(nbytes.value, dtype=torch.uint8, device=st.device)
+        _lib.call("vmc_nnbf_logpsi_grad_ws", *args, _lib.ptr(work), rows, s)
+
     def logpsi_grad(self, st, out=None):
         """(B, Np) O rows in the reference parameter order (FP32 mixed / FP64)."""
-        ts, arr = self.grad_net(st.device)
-        dt = ts[0].dtype
         if out is None:
-            out = torch.empty((st.B, self.n_params), dtype=dt, device=st.device)
-        _lib.call("vmc_nnbf_logpsi_grad", self._prec, arr, self.n_sites, self.n_fermions, self.hidden_dim,
-                  self.bf_scale, _lib.ptr(st.occ), st.B, _lib.ptr(out), out.stride(0), None, 0, None, None, None,
-                  None, _lib.stream_of(st.device))
+            out = torch.empty((st.B, self.n_params), dtype=self._rdtype(), device=st.device)
+        self._adjoint(st, full=out)
         return out
 
     def logpsi_grad_factored(self, st):
         """O in factored form: (O_dense (B, Np - Nw), kron_g (B, 2N*nf), kron_h (B, 256))
         where the out_w block of row b is kron_g[b] (x) kron_h[b]."""
-        ts, arr = self.grad_net(st.device)
-        dt = ts[0].dtype
+        dt = self._rdtype()
         nd = self.n_params - self.n_params_out_w
         Od = torch.empty((st.B, nd), dtype=dt, device=st.device)
         kg = torch.empty((st.B, self.n_orbitals * self.n_fermions), dtype=dt, device=st.device)
         kh = torch.empty((st.B, self.hidden_dim), dtype=dt, device=st.device)
-        _lib.call("vmc_nnbf_logpsi_grad", self._prec, arr, self.n_sites, self.n_fermions, self.hidden_dim,
-                  self.bf_scale, _lib.ptr(st.occ), st.B, None, 0, _lib.ptr(Od), Od.stride(0), _lib.ptr(kg),
-                  _lib.ptr(kh), None, None, _lib.stream_of(st.device))
+        self._adjoint(st, dense=Od, g=kg, h=kh)
         return Od, kg, kh
 
     def local_energy(self, st, H):
