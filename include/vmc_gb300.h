@@ -301,6 +301,27 @@ int vmc_sr_gram(const void* Oc, int dtype, int64_t Ns, int64_t Np, int64_t ldc, 
  *   *d_info is set to 1 when a pivot is not positive or not finite (the caller
  *   zeroes it first); the factor is then not usable. */
 int vmc_sr_cholesky(double* T, int64_t n, int64_t ldt, int* d_info, void* stream);
+/* FP64 products on the tensor cores (the reference's FP64 lpg_scaled @
+ * lpg_scaled.T and its torch.linalg.solve, vmc_torch/GPU/optimizer.py:551-563).
+ * vmc_split_f64: X (rows, K, ld ldx) FP64 -> row_exp (rows_pad ints, device): E_r
+ *   with max |X[r]| < 2^E_r (INT_MIN for a row with a NaN or Inf), and seven BF16
+ *   planes of the balanced base-256 digits of x 2^(55 - E_r) rounded to an
+ *   integer, each (rows_pad, kp) row-major, rows_pad a multiple of 128 >= rows,
+ *   kp a multiple of 32 >= K, padding zeroed; planes (16-byte aligned) holds
+ *   7 * rows_pad * kp bf16.
+ * vmc_sr_gram_f64_tc: T (ns, ns, FP64, ld ldt) = [T +] X X^T [+ shift I], the
+ *   full symmetric matrix; digit products of levels 0..6 (28 of the 49; the rest
+ *   is below 2^-56 of the largest entries' product), summed as integers, added
+ *   in FP64 every 256 columns.  Rows and columns with a NaN or Inf come out NaN.
+ * vmc_sr_cholesky_tc: as vmc_sr_cholesky with the trailing updates done this
+ *   way; work (256-byte aligned) of *bytes from vmc_sr_cholesky_tc_work_bytes.
+ * d_err (device int) receives VMC_ERR_TIMEOUT if a bounded wait gave up. */
+int vmc_split_f64(const double* X, int64_t rows, int64_t K, int64_t ldx, void* planes, int64_t rows_pad, int64_t kp,
+                  int* row_exp, void* stream);
+int vmc_sr_gram_f64_tc(const void* planes, const int* row_exp, int64_t ns, int64_t rows_pad, int64_t kp, double* T,
+                       int64_t ldt, double diag_shift, int accumulate, int* d_err, void* stream);
+int vmc_sr_cholesky_tc_work_bytes(int64_t n, int64_t* bytes);
+int vmc_sr_cholesky_tc(double* T, int64_t n, int64_t ldt, int* d_info, void* work, int* d_err, void* stream);
 /* Tensor-core Gram for FP32 inputs (no reference counterpart as an operator:
  * the reference forms lpg_scaled @ lpg_scaled.T in FP64, vmc_torch/GPU/optimizer.py:551-553).
  * vmc_split_bf16x3: X (rows, K, ld ldx) FP32 -> row_exp (rows_pad ints, device):

@@ -114,6 +114,21 @@ __device__ __forceinline__ T warp_sum(T v) {
   return v;
 }
 
+// 1/d for positive finite d: FP32 seed through the bit patterns (no FP64
+// conversion), then one third-order step y (1 + e + e^2), e = 1 - d y
+// (2^-21 -> 2^-63).
+__device__ __forceinline__ double rcp_pos(double d) {
+  const int hi = __double2hiint(d), e = (hi >> 20) - 1023;
+  if (e < -1000 || e > 1000) return 1.0 / d;
+  const float m = __uint_as_float(0x3f800000u | ((unsigned)(hi & 0xfffff) << 3) | ((unsigned)__double2loint(d) >> 29));
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(m));   // in (1/2, 1]
+  const unsigned rb = __float_as_uint(r);
+  const double y = __hiloint2double((int)((rb >> 3) + ((1023 - 127 - e) << 20)), (int)(rb << 29));
+  const double t = fma(-d, y, 1.0);
+  return fma(y, fma(t, t, t), y);
+}
+
 }  // namespace vmc
 
 #define VMC_CUDA_CHECK_LAUNCH()                                   \

@@ -1,8 +1,7 @@
 // Sample-space SR (minSR) linear algebra on one GPU:
 //   column means and centring/scaling of O, the Gram matrix T = O~ O~^T + lambda I
-//   on the CUDA cores (the tensor-core Gram is in gram.cu), a blocked right-looking
-//   Cholesky of T (FP64 tiles and panels, double-float trailing updates), blocked
-//   forward/backward substitution, and dp = O~^T x.  Also the plain energy
+//   on the CUDA cores (the tensor-core ones are in gram.cu and fp64_tc.cu, with the
+//   Cholesky), blocked forward/backward substitution, and dp = O~^T x.  Also the plain energy
 //   gradient <E O> - <E><O>.
 #include "common.cuh"
 
@@ -49,18 +48,152 @@ struct TileAcc {
   }
 };
 
-// mean[p] = (1/Ns) sum_i O[i][p];  Oc[i][p] = (O[i][p] - mean[p]) * scale
-template <typename TI, typename TO>
-__global__ void k_center(const TI* __restrict__ O, int64_t Ns, int64_t Np, int64_t ldo, TO* __restrict__ Oc,
-                         int64_t ldc, double* __restrict__ mean, double scale) {
-  int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= Np) return;
-  double s = 0.0;
-  for (int64_t i = 0; i < Ns; ++i) s += (double)O[i * ldo + p];
-  const double m = s / (double)Ns;
-  if (mean) mean[p] = m;
-  if (Oc)
-    for (int64_t i = 0; i < Ns; ++i) Oc[i * ldc + p] = (TO)(((double)O[i * ldo + p] - m) * scale);
+// Column kernels: a CTA of 8 warps takes 32 NC columns, lane = column (NC of
+// them, 32 apart), warp w the rows w, w + 8, ...; the warps' sums meet in
+// shared memory.  (One thread per column leaves all but Np / 256 CTAs' worth of
+// the GPU idle and each thread waiting on one load at a time.)  NC = 4 reads 512
+// consecutive bytes of an FP32 row, which HBM pages want (one 128-byte piece a
+// row read 8192 x 115200 in 4.3 ms of centring); NC = 1 where that would leave
+// fewer CTAs than the GPU holds.  An FP64 instruction costs a warp 64 clocks
+// on GB300, so FP32 inputs are summed as double-float pairs (Knuth's TwoSum,
+// ~2^-47 of the running sum) that are added to the FP64 sum every 16 / NC rows.
+// 8192 x 115200 FP32: centring 10.7 and O~^T x 3.6 ms before; three
+// respectively one passes over 3.8 GB take 1.7 and 0.6 at the measured rate.
+constexpr int CW = 8;                    // warps a CTA
+constexpr int CB = 128;                  // rows a block of the loops below
+constexpr int64_t CWIDE = 128 * 304;     // columns from which NC = 4
+
+// s + x as s' + error
+__device__ __forceinline__ float two_sum(float& s, float x) {
+  const float t = s + x, bb = t - s;
+  const float e = (s - (t - bb)) + (x - bb);
+  s = t;
+  return e;
+}
+
+// x = h + l to 2^-48 of x, through the bit patterns where h and l are normal
+// floats (no FP64 instruction)
+__device__ __forceinline__ void split_f64(double x, float& h, float& l) {
+  const int hi = __double2hiint(x);
+  const unsigned lo = (unsigned)__double2loint(x);
+  const int e = ((hi >> 20) & 0x7ff) - 1023;
+  if (e > -70 && e < 120) {
+    h = __uint_as_float((unsigned)(hi & 0x80000000) | (unsigned)((e + 127) << 23) | ((unsigned)(hi & 0xfffff) << 3) |
+                        (lo >> 29));
+    l = (float)(lo & 0x1fffffffu) * __uint_as_float((unsigned)(hi & 0x80000000) | (unsigned)((e - 52 + 127) << 23));
+  } else {
+    h = (float)x;
+    l = (float)(x - (double)h);
+  }
+}
+
+// Sums over all rows of the lane's NC columns, in every warp.  load(i, j): the
+// value at row i, column group j; pair(i - i0, x, h, l): its term as h + l (FP32
+// inputs); begin(i0) is called by all threads before the rows [i0, i0 + CB).
+template <typename T, int NC, typename B, typename L, typename P>
+__device__ __forceinline__ void column_sums(int64_t Ns, double (*part)[NC * 32], double (&sum)[NC], B begin, L load,
+                                            P pair) {
+  constexpr int CU = 16 / NC;            // rows in flight
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+  for (int j = 0; j < NC; ++j) sum[j] = 0.0;
+  for (int64_t i0 = 0; i0 < Ns; i0 += CB) {
+    begin(i0);
+#pragma unroll 1
+    for (int u0 = 0; u0 < CB / CW; u0 += CU) {
+      T x[CU][NC];
+#pragma unroll
+      for (int u = 0; u < CU; ++u)
+#pragma unroll
+        for (int j = 0; j < NC; ++j) {
+          const int64_t i = i0 + (u0 + u) * CW + warp;
+          x[u][j] = i < Ns ? load(i, j) : T(0);
+        }
+#pragma unroll
+      for (int j = 0; j < NC; ++j) {
+        if constexpr (sizeof(T) == 4) {
+          float s = 0.f, c = 0.f;
+#pragma unroll
+          for (int u = 0; u < CU; ++u) {
+            float h, l;
+            pair((u0 + u) * CW + warp, x[u][j], h, l);
+            if (u == 0) { s = h; c = l; }
+            else c += two_sum(s, h) + l;
+          }
+          sum[j] += (double)s;
+          sum[j] += (double)c;
+        } else {
+#pragma unroll
+          for (int u = 0; u < CU; ++u) sum[j] += pair((u0 + u) * CW + warp, x[u][j]);
+        }
+      }
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < NC; ++j) part[warp][j * 32 + lane] = sum[j];
+  __syncthreads();
+#pragma unroll
+  for (int j = 0; j < NC; ++j) {
+    double t = 0.0;
+#pragma unroll
+    for (int w = 0; w < CW; ++w) t += part[w][j * 32 + lane];
+    sum[j] = t;
+  }
+}
+
+// mean[p] = (1/Ns) sum_i O[i][p];  Oc[i][p] = (O[i][p] - mean[p]) * scale, FP32
+// in double-float arithmetic: the FP64 result rounded to FP32 (but for ties to
+// 2^-20 of an ulp)
+template <typename T, int NC>
+__global__ void __launch_bounds__(32 * CW) k_center(const T* __restrict__ O, int64_t Ns, int64_t Np, int64_t ldo,
+                                                    T* __restrict__ Oc, int64_t ldc, double* __restrict__ mean,
+                                                    double scale) {
+  __shared__ double part[CW][NC * 32];
+  constexpr int CU = 16 / NC;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int64_t p0 = (int64_t)blockIdx.x * (32 * NC) + lane;
+  int64_t off[NC];       // columns past the end read the last one
+#pragma unroll
+  for (int j = 0; j < NC; ++j) off[j] = p0 + 32 * j < Np ? p0 + 32 * j : Np - 1;
+  double sum[NC];
+  auto load = [&](int64_t i, int j) { return O[i * ldo + off[j]]; };
+  if constexpr (sizeof(T) == 4)
+    column_sums<T, NC>(Ns, part, sum, [](int64_t) {}, load, [](int, float x, float& h, float& l) { h = x; l = 0.f; });
+  else
+    column_sums<T, NC>(Ns, part, sum, [](int64_t) {}, load, [](int, double x) { return x; });
+  double m[NC];
+#pragma unroll
+  for (int j = 0; j < NC; ++j) {
+    m[j] = sum[j] / (double)Ns;
+    if (mean && warp == 0 && p0 + 32 * j < Np) mean[p0 + 32 * j] = m[j];
+  }
+  if (!Oc) return;
+  float mh[NC], ml[NC];
+  const float sh = (float)scale, sl = (float)(scale - (double)sh);
+#pragma unroll
+  for (int j = 0; j < NC; ++j) { mh[j] = (float)m[j]; ml[j] = (float)(m[j] - (double)mh[j]); }
+  for (int64_t i0 = warp; i0 < Ns; i0 += CW * CU) {
+    T x[CU][NC];
+#pragma unroll
+    for (int u = 0; u < CU; ++u)
+#pragma unroll
+      for (int j = 0; j < NC; ++j) x[u][j] = i0 + u * CW < Ns ? load(i0 + u * CW, j) : T(0);
+#pragma unroll
+    for (int u = 0; u < CU; ++u)
+#pragma unroll
+      for (int j = 0; j < NC; ++j) {
+        T v;
+        if constexpr (sizeof(T) == 4) {
+          float d = x[u][j];
+          const float e = two_sum(d, -mh[j]) - ml[j];
+          const float q = d * sh;
+          v = q + fmaf(e, sh, fmaf(d, sl, fmaf(d, sh, -q)));
+        } else {
+          v = (x[u][j] - m[j]) * scale;
+        }
+        if (i0 + u * CW < Ns && p0 + 32 * j < Np) Oc[(i0 + u * CW) * ldc + p0 + 32 * j] = v;
+      }
+  }
 }
 
 // g[p] = (1/Ns) sum_i E[i] O[i][p] - Ebar * mean_i O[i][p]
@@ -129,182 +262,186 @@ __global__ void k_syrk(const TI* __restrict__ A, int64_t lda, int64_t n, int64_t
     }
 }
 
-// The Cholesky's trailing update C -= A A^T for FP64 A in double-float
-// arithmetic on the FP32 pipes (GB300's FP64 rate is 1/64 of FP32): each
-// operand is split into FP32 x = hi + lo (to 2^-48), the leading product
-// hi*hi is captured exactly (p and its FMA error term), p is summed with
-// Knuth's TwoSum into a (s, c) pair and the small terms (the error term,
-// hi*lo + lo*hi) into a third FP32 accumulator; lo*lo (2^-48) is dropped.
-// ~12 FP32 instructions per multiply-add, relative accuracy ~2^-45 over the
-// tile, far below the Gram matrix's own input rounding.  Same tiling and
-// lower-triangle semantics as k_syrk.
-__global__ void k_syrk_df(const double* __restrict__ A, int64_t lda, int64_t n, int64_t K, double* __restrict__ C,
-                          int64_t ldc, int64_t off, double sgn) {
-  const int bi = blockIdx.y, bj = blockIdx.x;
-  if (bj > bi) return;
-  __shared__ float Ah[TK][TB + 1], Al[TK][TB + 1], Bh[TK][TB + 1], Bl[TK][TB + 1];
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  const int64_t i0 = off + (int64_t)bi * TB, j0 = off + (int64_t)bj * TB;
-  float hs[4][4], hc[4][4], sm[4][4];
-#pragma unroll
-  for (int q = 0; q < 4; ++q)
-#pragma unroll
-    for (int r = 0; r < 4; ++r) { hs[q][r] = 0.f; hc[q][r] = 0.f; sm[q][r] = 0.f; }
-  for (int64_t k0 = 0; k0 < K; k0 += TK) {
-    for (int idx = threadIdx.x; idx < TB * TK; idx += 256) {
-      const int r = idx / TK, kk = idx - r * TK;
-      const int64_t gk = k0 + kk, gi = i0 + r, gj = j0 + r;
-      const double a = (gi < off + n && gk < K) ? A[gi * lda + gk] : 0.0;
-      const double b = (gj < off + n && gk < K) ? A[gj * lda + gk] : 0.0;
-      const float ah = (float)a, bh = (float)b;
-      Ah[kk][r] = ah;
-      Al[kk][r] = (float)(a - (double)ah);
-      Bh[kk][r] = bh;
-      Bl[kk][r] = (float)(b - (double)bh);
-    }
-    __syncthreads();
-#pragma unroll 4
-    for (int kk = 0; kk < TK; ++kk) {
-      float ah[4], al[4], bh[4], bl[4];
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        ah[q] = Ah[kk][ty * 4 + q]; al[q] = Al[kk][ty * 4 + q];
-        bh[q] = Bh[kk][tx * 4 + q]; bl[q] = Bl[kk][tx * 4 + q];
-      }
-#pragma unroll
-      for (int q = 0; q < 4; ++q)
-#pragma unroll
-        for (int r = 0; r < 4; ++r) {
-          const float p = ah[q] * bh[r];
-          const float e = fmaf(ah[q], bh[r], -p);
-          sm[q][r] += e + fmaf(ah[q], bl[r], al[q] * bh[r]);
-          const float s2 = hs[q][r] + p;
-          const float bb = s2 - hs[q][r];
-          hc[q][r] += (hs[q][r] - (s2 - bb)) + (p - bb);
-          hs[q][r] = s2;
-        }
-    }
-    __syncthreads();
-  }
-#pragma unroll
-  for (int q = 0; q < 4; ++q)
-#pragma unroll
-    for (int r = 0; r < 4; ++r) {
-      const int64_t gi = i0 + ty * 4 + q, gj = j0 + tx * 4 + r;
-      if (gi < off + n && gj < off + n && gj <= gi)
-        C[gi * ldc + gj] += sgn * ((double)hs[q][r] + (double)hc[q][r] + (double)sm[q][r]);
-    }
-}
-
-// Unblocked Cholesky of one diagonal tile (lower), in place; flags non-positive pivots.
-__global__ void k_potrf_tile(double* __restrict__ C, int64_t ldc, int64_t k0, int64_t nb, int* __restrict__ info) {
-  __shared__ double a[TB][TB + 1];
-  for (int idx = threadIdx.x; idx < nb * nb; idx += blockDim.x) {
-    int r = idx / nb, c = idx - r * nb;
-    a[r][c] = C[(k0 + r) * ldc + k0 + c];
-  }
-  __syncthreads();
-  for (int k = 0; k < nb; ++k) {
-    if (threadIdx.x == 0) {
-      double d = a[k][k];
-      if (!(d > 0.0) || !isfinite(d)) { atomicExch(info, 1); d = 1e-300; }
-      a[k][k] = sqrt(d);
-    }
-    __syncthreads();
-    for (int r = k + 1 + threadIdx.x; r < nb; r += blockDim.x) a[r][k] /= a[k][k];
-    __syncthreads();
-    for (int idx = threadIdx.x; idx < nb * nb; idx += blockDim.x) {
-      int r = idx / nb, c = idx - r * nb;
-      if (c > k && r >= c) a[r][c] -= a[r][k] * a[c][k];
-    }
-    __syncthreads();
-  }
-  for (int idx = threadIdx.x; idx < nb * nb; idx += blockDim.x) {
-    int r = idx / nb, c = idx - r * nb;
-    C[(k0 + r) * ldc + k0 + c] = (c <= r) ? a[r][c] : 0.0;
-  }
-}
-
-// Panel: X = A21 * L11^{-T} for the rows below the diagonal tile; one thread per row.
-__global__ void k_trsm_panel(double* __restrict__ C, int64_t ldc, int64_t n, int64_t k0, int64_t nb) {
-  __shared__ double L[TB][TB + 1];
-  for (int idx = threadIdx.x; idx < nb * nb; idx += blockDim.x) {
-    int r = idx / nb, c = idx - r * nb;
-    L[r][c] = C[(k0 + r) * ldc + k0 + c];
-  }
-  __syncthreads();
-  int64_t row = k0 + nb + (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (row >= n) return;
-  double x[TB];
-  double* a = C + row * ldc + k0;
-  for (int k = 0; k < nb; ++k) {
-    double v = a[k];
-    for (int m = 0; m < k; ++m) v -= x[m] * L[k][m];
-    x[k] = v / L[k][k];
-  }
-  for (int k = 0; k < nb; ++k) a[k] = x[k];
-}
-
-// Blocked triangular solves (panels of TRSV_NB rows): the diagonal block is
-// solved by one CTA (thread t owns row t of the block), then every remaining
-// row is updated by a coalesced dot with the panel's solved values.
+// Blocked triangular solves (panels of TRSV_NB rows), one launch per panel:
+// with the panel's solved values every remaining row is updated, and CTA 0,
+// whose rows are the next diagonal block, goes on to solve that block.  An
+// FP64 instruction takes a warp 64 clocks on GB300, so the block is solved as
+// two chains of 32 steps (one warp, a row a lane: a product with the
+// reciprocal diagonal, a shuffle and a multiply-add a step) with the 32 x 32
+// product between them spread over four warps.
 constexpr int TRSV_NB = 64;
 
-// trans = 0: solve L[k0:k0+nb, k0:k0+nb] y = b[k0:k0+nb] in place (forward);
-// trans = 1: solve L[k0:k0+nb, k0:k0+nb]^T x = b[k0:k0+nb] in place (backward).
-__global__ void k_trsv_diag(const double* __restrict__ L, int64_t ldc, int64_t k0, int nb, double* __restrict__ b,
-                            int trans) {
-  __shared__ double xs[TRSV_NB];
-  const int t = threadIdx.x;
-  double bt = t < nb ? b[k0 + t] : 0.0;
-  if (!trans) {
-    for (int j = 0; j < nb; ++j) {
-      if (t == j) xs[j] = bt / L[(k0 + j) * ldc + k0 + j];
-      __syncthreads();
-      if (t > j && t < nb) bt -= L[(k0 + t) * ldc + k0 + j] * xs[j];
+// Solves the diagonal block Ls (its rows and columns past the matrix are those
+// of the identity) for the right-hand side bs, in place; rd, part: scratch.
+// All 256 threads call it, with bs and Ls visible to all of them.
+template <bool TRANS>
+__device__ __forceinline__ void trsv_block(const double (*Ls)[TRSV_NB + 1], double* bs, double* rd,
+                                           double (*part)[TRSV_NB]) {
+  const int tid = threadIdx.x, l = tid & 31, warp = tid >> 5;
+  if (tid < TRSV_NB) rd[tid] = 1.0 / Ls[tid][tid];
+  __syncthreads();
+#pragma unroll 1
+  for (int h = 0; h < 2; ++h) {
+    const int o = (TRANS ? 1 - h : h) * 32;      // rows of this half
+    if (warp == 0) {
+      double b = bs[o + l];
+      const double r = rd[o + l];
+#pragma unroll 8
+      for (int s = 0; s < 32; ++s) {
+        const int j = TRANS ? 31 - s : s;
+        const double xj = __shfl_sync(VMC_FULL_MASK, b * r, j);
+        const double c = TRANS ? Ls[o + j][o + l] : Ls[o + l][o + j];
+        if (l == j) b = xj;
+        else if (TRANS ? l < j : l > j) b = fma(-c, xj, b);
+      }
+      bs[o + l] = b;
     }
-  } else {
-    for (int j = nb - 1; j >= 0; --j) {
-      if (t == j) xs[j] = bt / L[(k0 + j) * ldc + k0 + j];
+    __syncthreads();
+    if (h == 0) {   // the other half's right-hand side: a row a lane, eight columns a warp
+      const int p = 32 - o;
+      if (warp < 4) {
+        double acc = 0.0;
+#pragma unroll
+        for (int s = 0; s < 8; ++s) {
+          const int j = o + warp * 8 + s;
+          acc = fma(TRANS ? Ls[j][p + l] : Ls[p + l][j], bs[j], acc);
+        }
+        part[warp][l] = acc;
+      }
       __syncthreads();
-      if (t < j) bt -= L[(k0 + j) * ldc + k0 + t] * xs[j];
+      if (warp == 0) bs[p + l] -= (part[0][l] + part[1][l]) + (part[2][l] + part[3][l]);
+      __syncwarp();
     }
   }
-  if (t < nb) b[k0 + t] = xs[t];
 }
 
-// forward update: b[i] -= sum_{j < nb} L[i][k0 + j] b[k0 + j] for rows i >= k0 + nb, a warp per row
-__global__ void k_trsv_upd_fwd(const double* __restrict__ L, int64_t ldc, int64_t n, int64_t k0, int nb,
-                               double* __restrict__ b) {
-  const int64_t i = k0 + nb + (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  const int lane = threadIdx.x & 31;
-  if (i >= n) return;
-  double acc = 0.0;
-  for (int j = lane; j < nb; j += 32) acc += L[i * ldc + k0 + j] * b[k0 + j];
+__device__ __forceinline__ void trsv_load(double (*Ls)[TRSV_NB + 1], const double* __restrict__ L, int64_t ldc,
+                                          int64_t k0, int nb) {
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-  if (lane == 0) b[i] -= acc;
+  for (int q = 0; q < TRSV_NB * TRSV_NB / 256; ++q) {
+    const int idx = q * 256 + threadIdx.x, r = idx >> 6, c = idx & 63;
+    Ls[r][c] = (r < nb && c < nb) ? L[(k0 + r) * ldc + k0 + c] : (r == c ? 1.0 : 0.0);
+  }
 }
 
-// backward update: b[j] -= sum_{i < nb} L[k0 + i][j] b[k0 + i] for columns j < k0, a thread per column
-__global__ void k_trsv_upd_bwd(const double* __restrict__ L, int64_t ldc, int64_t k0, int nb,
-                               double* __restrict__ b) {
-  const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= k0) return;
+// Forward: rows i >= k1 take b[i] -= sum_j L[i][k0 + j] b[k0 + j] over the 64
+// solved values before k1 (none when k1 = 0), a warp per row, 64 rows a CTA;
+// CTA 0 then solves the block at k1.
+__global__ void __launch_bounds__(256) k_trsv_fwd(const double* __restrict__ L, int64_t ldc, int64_t n, int64_t k1,
+                                                  double* __restrict__ b) {
+  __shared__ double Ls[TRSV_NB][TRSV_NB + 1];
+  __shared__ double bs[TRSV_NB], rd[TRSV_NB];
+  __shared__ double part[4][TRSV_NB];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int64_t i0 = k1 + (int64_t)blockIdx.x * TRSV_NB;
+  const int nb = (int)(n - k1 < TRSV_NB ? n - k1 : TRSV_NB);
+  if (blockIdx.x == 0) trsv_load(Ls, L, ldc, k1, nb);
+  double x0 = 0.0, x1 = 0.0;
+  if (k1 > 0) { x0 = b[k1 - TRSV_NB + lane]; x1 = b[k1 - 32 + lane]; }
+#pragma unroll
+  for (int q = 0; q < 8; ++q) {
+    const int r = warp * 8 + q;
+    const int64_t i = i0 + r;
+    double v = 0.0;
+    if (i < n) {
+      if (k1 > 0) {
+        const double* row = L + i * ldc + k1 - TRSV_NB;
+        double acc = row[lane] * x0;
+        acc = vmc::warp_sum(fma(row[lane + 32], x1, acc));
+        v = b[i] - acc;
+      } else {
+        v = b[i];
+      }
+    }
+    if (lane == 0) {
+      if (blockIdx.x == 0) bs[r] = v;
+      else if (i < n) b[i] = v;
+    }
+  }
+  if (blockIdx.x != 0) return;
+  __syncthreads();
+  trsv_block<false>(Ls, bs, rd, part);
+  if (threadIdx.x < nb) b[k1 + threadIdx.x] = bs[threadIdx.x];
+}
+
+// Backward: columns j < k1 + 64 take b[j] -= sum_i L[k1 + 64 + i][j] b[k1 + 64 + i]
+// over the block of solved values that starts at k1 + 64 (none past n), a
+// thread per column and 16 of the block's rows, 64 columns a CTA; CTA 0 holds
+// the columns [k1, k1 + 64) and solves that block of L^T.
+__global__ void __launch_bounds__(256) k_trsv_bwd(const double* __restrict__ L, int64_t ldc, int64_t n, int64_t k1,
+                                                  double* __restrict__ b) {
+  __shared__ double Ls[TRSV_NB][TRSV_NB + 1];
+  __shared__ double bs[TRSV_NB], rd[TRSV_NB];
+  __shared__ double part[4][TRSV_NB];
+  const int64_t j0 = k1 - (int64_t)blockIdx.x * TRSV_NB;
+  const int64_t s0 = k1 + TRSV_NB;
+  const int nb = (int)(n - k1 < TRSV_NB ? n - k1 : TRSV_NB);
+  const int ns = (int)(n - s0 < TRSV_NB ? (n > s0 ? n - s0 : 0) : TRSV_NB);
+  if (blockIdx.x == 0) trsv_load(Ls, L, ldc, k1, nb);
+  const int c = threadIdx.x & 63, h = threadIdx.x >> 6;
   double acc = 0.0;
-  for (int i = 0; i < nb; ++i) acc += L[(k0 + i) * ldc + j] * b[k0 + i];
-  b[j] -= acc;
+  if (c < nb || blockIdx.x != 0) {
+#pragma unroll
+    for (int q = 0; q < 16; ++q) {
+      const int i = h * 16 + q;
+      if (i < ns) acc = fma(L[(s0 + i) * ldc + j0 + c], b[s0 + i], acc);
+    }
+  }
+  part[h][c] = acc;
+  __syncthreads();
+  if (h == 0) {
+    double v = 0.0;
+    if (c < nb || blockIdx.x != 0) v = b[j0 + c] - ((part[0][c] + part[1][c]) + (part[2][c] + part[3][c]));
+    if (blockIdx.x == 0) bs[c] = v;
+    else b[j0 + c] = v;
+  }
+  if (blockIdx.x != 0) return;
+  __syncthreads();
+  trsv_block<true>(Ls, bs, rd, part);
+  if (threadIdx.x < nb) b[k1 + threadIdx.x] = bs[threadIdx.x];
 }
 
-// dp[p] = sum_i Oc[i][p] * x[i]
-template <typename TI>
-__global__ void k_gemv_t(const TI* __restrict__ Oc, int64_t Ns, int64_t Np, int64_t ldc, const double* __restrict__ x,
-                         double* __restrict__ dp) {
-  int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= Np) return;
-  double s = 0.0;
-  for (int64_t i = 0; i < Ns; ++i) s += (double)Oc[i * ldc + p] * x[i];
-  dp[p] = s;
+// dp[p] = sum_i Oc[i][p] * x[i]; FP32 rows: the product with x = xh + xl (to
+// 2^-48, split once a CTA and block of rows) as an exact leading product and its
+// remainder
+template <typename T, int NC>
+__global__ void __launch_bounds__(32 * CW) k_gemv_t(const T* __restrict__ Oc, int64_t Ns, int64_t Np, int64_t ldc,
+                                                    const double* __restrict__ x, double* __restrict__ dp) {
+  __shared__ double part[CW][NC * 32];
+  __shared__ float2 xs[2][CB];     // two blocks: the next is written while the last is still read
+  __shared__ double xd[2][CB];
+  const int64_t p0 = (int64_t)blockIdx.x * (32 * NC) + (threadIdx.x & 31);
+  int64_t off[NC];
+#pragma unroll
+  for (int j = 0; j < NC; ++j) off[j] = p0 + 32 * j < Np ? p0 + 32 * j : Np - 1;
+  double sum[NC];
+  int buf = 1;
+  auto begin = [&](int64_t i0) {
+    buf ^= 1;
+    if (threadIdx.x < CB) {
+      const double v = i0 + threadIdx.x < Ns ? x[i0 + threadIdx.x] : 0.0;
+      if constexpr (sizeof(T) == 4) {
+        float h, l;
+        split_f64(v, h, l);
+        xs[buf][threadIdx.x] = make_float2(h, l);
+      } else {
+        xd[buf][threadIdx.x] = v;
+      }
+    }
+    __syncthreads();
+  };
+  auto load = [&](int64_t i, int j) { return Oc[i * ldc + off[j]]; };
+  if constexpr (sizeof(T) == 4)
+    column_sums<T, NC>(Ns, part, sum, begin, load, [&](int r, float o, float& h, float& l) {
+      const float2 v = xs[buf][r];
+      h = o * v.x;
+      l = fmaf(o, v.y, fmaf(o, v.x, -h));
+    });
+  else
+    column_sums<T, NC>(Ns, part, sum, begin, load, [&](int r, double o) { return o * xd[buf][r]; });
+#pragma unroll
+  for (int j = 0; j < NC; ++j)
+    if (p0 + 32 * j < Np && threadIdx.x < 32) dp[p0 + 32 * j] = sum[j];
 }
 
 __global__ void k_rhs(const double* __restrict__ E, int64_t Ns, double Ebar, double scale, double* __restrict__ b) {
@@ -327,13 +464,14 @@ int vmc_sr_center(const void* O, int dtype, int64_t Ns, int64_t Np, int64_t ldo,
                   void* stream) {
   if (Ns <= 0 || Np <= 0 || ldo < Np || ldc < Np || !O || !Oc) return VMC_ERR_ARGS;
   const double scale = 1.0 / sqrt((double)Ns);
-  unsigned grid = (unsigned)((Np + 255) / 256);
+  cudaStream_t st = (cudaStream_t)stream;
+  const unsigned g1 = (unsigned)((Np + 31) / 32), g4 = (unsigned)((Np + 127) / 128);
   if (dtype == 0)
-    k_center<double, double><<<grid, 256, 0, (cudaStream_t)stream>>>((const double*)O, Ns, Np, ldo, (double*)Oc, ldc,
-                                                                      mean, scale);
+    k_center<double, 1><<<g1, 32 * CW, 0, st>>>((const double*)O, Ns, Np, ldo, (double*)Oc, ldc, mean, scale);
+  else if (dtype == 1 && Np >= CWIDE)
+    k_center<float, 4><<<g4, 32 * CW, 0, st>>>((const float*)O, Ns, Np, ldo, (float*)Oc, ldc, mean, scale);
   else if (dtype == 1)
-    k_center<float, float><<<grid, 256, 0, (cudaStream_t)stream>>>((const float*)O, Ns, Np, ldo, (float*)Oc, ldc,
-                                                                    mean, scale);
+    k_center<float, 1><<<g1, 32 * CW, 0, st>>>((const float*)O, Ns, Np, ldo, (float*)Oc, ldc, mean, scale);
   else
     return VMC_ERR_ARGS;
   VMC_CUDA_CHECK_LAUNCH();
@@ -362,43 +500,14 @@ int vmc_sr_gram(const void* Oc, int dtype, int64_t Ns, int64_t Np, int64_t ldc, 
   return VMC_OK;
 }
 
-// In-place lower Cholesky of T: FP64 tiles and panels, double-float trailing
-// updates.  d_info set to 1 on a non-positive pivot.
-int vmc_sr_cholesky(double* T, int64_t n, int64_t ldt, int* d_info, void* stream) {
-  if (n <= 0 || ldt < n || !T || !d_info) return VMC_ERR_ARGS;
-  cudaStream_t s = (cudaStream_t)stream;
-  for (int64_t k0 = 0; k0 < n; k0 += TB) {
-    int64_t nb = (n - k0) < TB ? (n - k0) : TB;
-    k_potrf_tile<<<1, 256, 0, s>>>(T, ldt, k0, nb, d_info);
-    int64_t rest = n - k0 - nb;
-    if (rest > 0) {
-      k_trsm_panel<<<(unsigned)((rest + 63) / 64), 64, 0, s>>>(T, ldt, n, k0, nb);
-      int64_t nt = (rest + TB - 1) / TB;
-      dim3 grid((unsigned)nt, (unsigned)nt);
-      // trailing update of the lower triangle: A22 -= L21 L21^T (double-float on the FP32 pipes)
-      k_syrk_df<<<grid, 256, 0, s>>>(T + k0, ldt, rest, nb, T, ldt, k0 + nb, -1.0);
-    }
-  }
-  VMC_CUDA_CHECK_LAUNCH();
-  return VMC_OK;
-}
-
 // Solve L L^T x = b in place on b (L from vmc_sr_cholesky).
 int vmc_sr_cholesky_solve(const double* L, int64_t n, int64_t ldt, double* b, void* stream) {
   if (n <= 0 || ldt < n || !L || !b) return VMC_ERR_ARGS;
   cudaStream_t st = (cudaStream_t)stream;
-  for (int64_t k0 = 0; k0 < n; k0 += TRSV_NB) {   // L y = b
-    const int nb = (int)((n - k0) < TRSV_NB ? (n - k0) : TRSV_NB);
-    k_trsv_diag<<<1, TRSV_NB, 0, st>>>(L, ldt, k0, nb, b, 0);
-    const int64_t rest = n - k0 - nb;
-    if (rest > 0) k_trsv_upd_fwd<<<(unsigned)((rest + 7) / 8), 256, 0, st>>>(L, ldt, n, k0, nb, b);
-  }
-  const int64_t last = ((n - 1) / TRSV_NB) * TRSV_NB;
-  for (int64_t k0 = last; k0 >= 0; k0 -= TRSV_NB) {   // L^T x = y
-    const int nb = (int)((n - k0) < TRSV_NB ? (n - k0) : TRSV_NB);
-    k_trsv_diag<<<1, TRSV_NB, 0, st>>>(L, ldt, k0, nb, b, 1);
-    if (k0 > 0) k_trsv_upd_bwd<<<(unsigned)((k0 + 255) / 256), 256, 0, st>>>(L, ldt, k0, nb, b);
-  }
+  for (int64_t k1 = 0; k1 < n; k1 += TRSV_NB)   // L y = b
+    k_trsv_fwd<<<(unsigned)((n - k1 + TRSV_NB - 1) / TRSV_NB), 256, 0, st>>>(L, ldt, n, k1, b);
+  for (int64_t k1 = ((n - 1) / TRSV_NB) * TRSV_NB; k1 >= 0; k1 -= TRSV_NB)   // L^T x = y
+    k_trsv_bwd<<<(unsigned)(k1 / TRSV_NB + 1), 256, 0, st>>>(L, ldt, n, k1, b);
   VMC_CUDA_CHECK_LAUNCH();
   return VMC_OK;
 }
@@ -415,11 +524,14 @@ int vmc_sr_rhs(const double* E, int64_t Ns, double Ebar, double* b, void* stream
 int vmc_sr_update(const void* Oc, int dtype, int64_t Ns, int64_t Np, int64_t ldc, const double* x, double* dp,
                   void* stream) {
   if (Ns <= 0 || Np <= 0 || ldc < Np || !Oc || !x || !dp) return VMC_ERR_ARGS;
-  unsigned grid = (unsigned)((Np + 255) / 256);
+  cudaStream_t st = (cudaStream_t)stream;
+  const unsigned g1 = (unsigned)((Np + 31) / 32), g4 = (unsigned)((Np + 127) / 128);
   if (dtype == 0)
-    k_gemv_t<double><<<grid, 256, 0, (cudaStream_t)stream>>>((const double*)Oc, Ns, Np, ldc, x, dp);
+    k_gemv_t<double, 1><<<g1, 32 * CW, 0, st>>>((const double*)Oc, Ns, Np, ldc, x, dp);
+  else if (dtype == 1 && Np >= CWIDE)
+    k_gemv_t<float, 4><<<g4, 32 * CW, 0, st>>>((const float*)Oc, Ns, Np, ldc, x, dp);
   else if (dtype == 1)
-    k_gemv_t<float><<<grid, 256, 0, (cudaStream_t)stream>>>((const float*)Oc, Ns, Np, ldc, x, dp);
+    k_gemv_t<float, 1><<<g1, 32 * CW, 0, st>>>((const float*)Oc, Ns, Np, ldc, x, dp);
   else
     return VMC_ERR_ARGS;
   VMC_CUDA_CHECK_LAUNCH();
@@ -513,6 +625,117 @@ __global__ void k_gemm_gen(int ta, int tb, int64_t M, int64_t N, int64_t K, doub
     }
 }
 
+// The same product for FP32 inputs: the sums of k_gemm_gen<float, float> (four
+// products in FP32, then a TwoSum into the double-float accumulator, ascending
+// k; equal to the bit), tiled 64 x 64 with 8 x 4 outputs a thread and the next
+// 16 columns of K prefetched.  A multiply-add costs 2.75 FP32 instructions (the
+// fold is 7 per four), so operand traffic is amortised over 32 outputs: the
+// head's four products at 8192 samples 16.4 -> 9.2 ms.
+constexpr int DG_T = 64, DG_K = 16, DG_THREADS = 128;
+
+// operand tile of 64 rows x 16: KM: X[r][k], else X[k][r]; sk scales the columns of K
+template <bool KM>
+__device__ __forceinline__ void dg_load(const float* __restrict__ X, int64_t ld, int64_t r0, int64_t rows, int64_t k0,
+                                        int64_t K, const float* __restrict__ sk, float (&v)[8]) {
+#pragma unroll
+  for (int q = 0; q < 8; ++q) {
+    const int idx = threadIdx.x + q * DG_THREADS;
+    const int64_t r = r0 + (KM ? idx >> 4 : idx & 63), k = k0 + (KM ? idx & 15 : idx >> 6);
+    float x = 0.f;
+    if (r < rows && k < K) {
+      x = KM ? X[r * ld + k] : X[k * ld + r];
+      if (sk) x *= sk[k];
+    }
+    v[q] = x;
+  }
+}
+template <bool KM>
+__device__ __forceinline__ void dg_store(float (*s)[DG_T + 4], const float (&v)[8]) {
+#pragma unroll
+  for (int q = 0; q < 8; ++q) {
+    const int idx = threadIdx.x + q * DG_THREADS;
+    s[KM ? idx & 15 : idx >> 6][KM ? idx >> 4 : idx & 63] = v[q];
+  }
+}
+
+template <bool TA, bool TB_>
+__global__ void __launch_bounds__(DG_THREADS) k_gemm_df(int64_t M, int64_t N, int64_t K, double alpha,
+                                                        const float* __restrict__ A, int64_t lda,
+                                                        const float* __restrict__ Bm, int64_t ldb,
+                                                        const float* __restrict__ sk, double beta,
+                                                        double* __restrict__ C, int64_t ldc,
+                                                        const double* __restrict__ D, int64_t ldd, int lower) {
+  const int bi = blockIdx.y, bj = blockIdx.x;
+  if (lower && bj > bi) return;
+  __shared__ float As[2][DG_K][DG_T + 4], Bs[2][DG_K][DG_T + 4];
+  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+  const int64_t m0 = (int64_t)bi * DG_T, n0 = (int64_t)bj * DG_T;
+  float hi[8][4], lo[8][4];
+#pragma unroll
+  for (int q = 0; q < 8; ++q)
+#pragma unroll
+    for (int r = 0; r < 4; ++r) hi[q][r] = lo[q][r] = 0.f;
+  float pa[8], pb[8];
+  dg_load<!TA>(A, lda, m0, M, 0, K, sk, pa);
+  dg_load<TB_>(Bm, ldb, n0, N, 0, K, nullptr, pb);
+  dg_store<!TA>(As[0], pa);
+  dg_store<TB_>(Bs[0], pb);
+  __syncthreads();
+  int buf = 0;
+  for (int64_t k0 = 0; k0 < K; k0 += DG_K) {
+    const bool more = k0 + DG_K < K;
+    if (more) {
+      dg_load<!TA>(A, lda, m0, M, k0 + DG_K, K, sk, pa);
+      dg_load<TB_>(Bm, ldb, n0, N, k0 + DG_K, K, nullptr, pb);
+    }
+#pragma unroll
+    for (int g = 0; g < DG_K / 4; ++g) {
+      float acc[8][4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const float* ar = As[buf][g * 4 + u];
+        const float4 a0 = *reinterpret_cast<const float4*>(ar + ty * 4);
+        const float4 a1 = *reinterpret_cast<const float4*>(ar + 32 + ty * 4);
+        const float4 b0 = *reinterpret_cast<const float4*>(&Bs[buf][g * 4 + u][tx * 4]);
+        const float a[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
+        const float b[4] = {b0.x, b0.y, b0.z, b0.w};
+#pragma unroll
+        for (int q = 0; q < 8; ++q)
+#pragma unroll
+          for (int r = 0; r < 4; ++r) acc[q][r] = u == 0 ? a[q] * b[r] : fmaf(a[q], b[r], acc[q][r]);
+      }
+#pragma unroll
+      for (int q = 0; q < 8; ++q)
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+          const float x = hi[q][r], y = acc[q][r];
+          const float t = x + y, bb = t - x;
+          lo[q][r] += (x - (t - bb)) + (y - bb);
+          hi[q][r] = t;
+        }
+    }
+    if (more) {
+      dg_store<!TA>(As[buf ^ 1], pa);
+      dg_store<TB_>(Bs[buf ^ 1], pb);
+      __syncthreads();
+      buf ^= 1;
+    }
+  }
+#pragma unroll
+  for (int q = 0; q < 8; ++q)
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      const int64_t gm = m0 + (q >> 2) * 32 + ty * 4 + (q & 3), gn = n0 + tx * 4 + r;
+      if (gm >= M || gn >= N) continue;
+      if (lower && gn > gm) continue;
+      double v = alpha * ((double)hi[q][r] + (double)lo[q][r]);
+      if (D) v *= D[gm * ldd + gn];
+      const double out = (beta == 0.0 ? 0.0 : beta * C[gm * ldc + gn]) + v;
+      C[gm * ldc + gn] = out;
+      if (lower && gm != gn) C[gn * ldc + gm] = out;
+    }
+}
+
 // T[a][b] += alpha * (-v[a] - v[b] + c0)
 __global__ void k_rank_corr(int64_t n, double* __restrict__ T, int64_t ldt, const double* __restrict__ v, double c0,
                             double alpha) {
@@ -550,9 +773,18 @@ int vmc_gemm(int ta, int tb, int64_t M, int64_t N, int64_t K, double alpha, cons
   if (dtype == 0)
     k_gemm_gen<double, double><<<grid, 256, 0, s>>>(ta, tb, M, N, K, alpha, (const double*)A, lda, (const double*)B,
                                                      ldb, (const double*)sk, beta, C, ldc, D, ldd, lower);
+  else if (ta && tb)
+    k_gemm_df<true, true><<<grid, DG_THREADS, 0, s>>>(M, N, K, alpha, (const float*)A, lda, (const float*)B, ldb,
+                                                      (const float*)sk, beta, C, ldc, D, ldd, lower);
+  else if (ta)
+    k_gemm_df<true, false><<<grid, DG_THREADS, 0, s>>>(M, N, K, alpha, (const float*)A, lda, (const float*)B, ldb,
+                                                       (const float*)sk, beta, C, ldc, D, ldd, lower);
+  else if (tb)
+    k_gemm_df<false, true><<<grid, DG_THREADS, 0, s>>>(M, N, K, alpha, (const float*)A, lda, (const float*)B, ldb,
+                                                       (const float*)sk, beta, C, ldc, D, ldd, lower);
   else
-    k_gemm_gen<float, float><<<grid, 256, 0, s>>>(ta, tb, M, N, K, alpha, (const float*)A, lda, (const float*)B, ldb,
-                                                   (const float*)sk, beta, C, ldc, D, ldd, lower);
+    k_gemm_df<false, false><<<grid, DG_THREADS, 0, s>>>(M, N, K, alpha, (const float*)A, lda, (const float*)B, ldb,
+                                                        (const float*)sk, beta, C, ldc, D, ldd, lower);
   VMC_CUDA_CHECK_LAUNCH();
   return VMC_OK;
 }

@@ -27,6 +27,7 @@ is assembled without materialising it:
 which reduces the 8x8 NNBF Gram from 2 Ns^2 * 2.2e6 to 2 Ns^2 * (1.15e5 + 8192
 + 256) flops and never stores the 145 GB out_w block of O.
 """
+import ctypes
 import time
 
 import torch
@@ -140,12 +141,20 @@ class MinSRGB300(PreconditionerGB300):
         rows rounded to 2^-20 of their largest entry, positive semidefinite
         up to ~2^-32 rounding.  "cuda" forms them on the CUDA cores with
         compensated (double-float) accumulation: the exact Gram of the FP32
-        rows, ~10x slower.  FP64 O always uses FP64 arithmetic."""
+        rows, ~10x slower.  FP64 O: "tensor" uses seven base-256 digits of
+        every entry (vmc_sr_gram_f64_tc, FP64 accuracy), "cuda" the FP64 cores."""
         if gram not in ("tensor", "cuda"):
             raise ValueError("gram must be 'tensor' or 'cuda'")
         self.record_stages = record_stages
         self.last_stages = None
         self.gram = gram
+
+    # digit planes of an FP64 Gram matrix held at a time
+    SLAB_BYTES = 2 << 30
+    # order from which the Cholesky's trailing updates run on the tensor cores
+    # (vmc_sr_cholesky_tc): at 513 the two take the same time (1.13 ms: the
+    # chain of 64-column tiles), at 2049 4.4 against 5.2 ms, at 8192 29 against 85
+    CHOLESKY_TC_MIN = 513
 
     def _tc_gram(self, X, T, alpha, D, shift, accumulate, dev):
         """T [+]= alpha (X X^T) o D [+ shift I] on the tensor cores, X FP32 (Ns, K)."""
@@ -160,6 +169,27 @@ class MinSRGB300(PreconditionerGB300):
                   T.stride(0), _lib.ptr(D), float(shift), int(accumulate), _lib.ptr(err), s)
         self._tc_err = err
         del planes
+
+    def _tc_gram_f64(self, X, T, shift, dev):
+        """T = X X^T + shift I on the tensor cores, X FP64 (Ns, K); the digit
+        planes (14 bytes per entry) are made for at most SLAB_BYTES of
+        columns at a time."""
+        s = _lib.stream_of(dev)
+        Ns, K = X.shape
+        rp = -(-Ns // 128) * 128
+        slab = max(256, self.SLAB_BYTES // (14 * rp) // 256 * 256)
+        kp = -(-min(K, slab) // 32) * 32
+        planes = torch.empty(7 * rp * kp, dtype=torch.bfloat16, device=dev)
+        rexp = torch.empty(rp, dtype=torch.int32, device=dev)
+        err = torch.zeros(1, dtype=torch.int32, device=dev)
+        for a in range(0, K, slab):
+            k = min(slab, K - a)
+            kp = -(-k // 32) * 32
+            _lib.call("vmc_split_f64", _lib.ptr(X[:, a:]), Ns, k, X.stride(0), _lib.ptr(planes), rp, kp,
+                      _lib.ptr(rexp), s)
+            _lib.call("vmc_sr_gram_f64_tc", _lib.ptr(planes), _lib.ptr(rexp), Ns, rp, kp, _lib.ptr(T), T.stride(0),
+                      float(shift) if a + k == K else 0.0, int(a > 0), _lib.ptr(err), s)
+        self._tc_err = err
 
     def _check_tc(self):
         err = getattr(self, "_tc_err", None)
@@ -199,8 +229,10 @@ class MinSRGB300(PreconditionerGB300):
         self._st.mark("center")
 
         def gram(T, shift):
-            if code == 1 and self.gram == "tensor":
+            if self.gram == "tensor" and code == 1:
                 self._tc_gram(Oc, T, 1.0, None, shift, 0, dev)
+            elif self.gram == "tensor" and Np > 0:
+                self._tc_gram_f64(Oc, T, shift, dev)
             else:
                 _lib.call("vmc_sr_gram", _lib.ptr(Oc), code, Ns, Np, Oc.stride(0), _lib.ptr(T), Ns, shift, 0, s)
             self._st.mark("gram")
@@ -213,20 +245,29 @@ class MinSRGB300(PreconditionerGB300):
         return dp, time.time() - t0, info
 
     # -- shared: Gram -> FP64 Cholesky -> solve (reference fallbacks on failure) --
-    @staticmethod
-    def _factor_solve(build_gram, E, Ebar, Ns, shift, dev, stages):
+    @classmethod
+    def _factor_solve(cls, build_gram, E, Ebar, Ns, shift, dev, stages):
         s = _lib.stream_of(dev)
         T = torch.empty((Ns, Ns), dtype=torch.float64, device=dev)
         build_gram(T, shift)
-        flag = torch.zeros(1, dtype=torch.int32, device=dev)
-        _lib.call("vmc_sr_cholesky", _lib.ptr(T), Ns, Ns, _lib.ptr(flag), s)
+        flag = torch.zeros(2, dtype=torch.int32, device=dev)   # failed pivot, kernel status
+        if Ns >= cls.CHOLESKY_TC_MIN:
+            nbytes = ctypes.c_int64(0)
+            _lib.call("vmc_sr_cholesky_tc_work_bytes", Ns, ctypes.byref(nbytes))
+            work = torch.empty(nbytes.value, dtype=torch.uint8, device=dev)
+            _lib.call("vmc_sr_cholesky_tc", _lib.ptr(T), Ns, Ns, _lib.ptr(flag), _lib.ptr(work), _lib.ptr(flag[1:]), s)
+        else:
+            _lib.call("vmc_sr_cholesky", _lib.ptr(T), Ns, Ns, _lib.ptr(flag), s)
         stages.mark("cholesky")
         check = getattr(build_gram, "check", None)
         if check is not None:
             check()
         x = torch.empty(Ns, dtype=torch.float64, device=dev)
         _lib.call("vmc_sr_rhs", _lib.ptr(E), Ns, Ebar, _lib.ptr(x), s)
-        if int(flag.item()) == 0:
+        info, err = flag.tolist()
+        if err != 0:
+            raise ValueError("vmc_sr_cholesky_tc: %s" % _lib.message(err))
+        if info == 0:
             _lib.call("vmc_sr_cholesky_solve", _lib.ptr(T), Ns, Ns, _lib.ptr(x), s)
             stages.mark("solve")
             return x, 0
@@ -280,6 +321,8 @@ class MinSRGB300(PreconditionerGB300):
             tc = code == 1 and self.gram == "tensor"
             if tc:
                 self._tc_gram(Oc, T, 1.0, None, sh, 0, dev)
+            elif self.gram == "tensor" and Nd > 0:
+                self._tc_gram_f64(Oc, T, sh, dev)
             else:
                 _lib.call("vmc_sr_gram", _lib.ptr(Oc), code, Ns, Nd, Oc.stride(0), _lib.ptr(T), Ns, sh, 0, s)
             self._st.mark("gram_dense")
