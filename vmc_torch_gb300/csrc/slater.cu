@@ -20,103 +20,10 @@ namespace {
 
 constexpr int kMaxNf = 64;
 
-struct WarpSmem {
-  double* G;      // nf x (nf+1)
-  double* tmp;    // 2 x nf
-  uint8_t* slot;  // nf
-};
-
 __device__ __forceinline__ int gstride(int nf) { return nf + 1; }
 
-// Full re-inversion by Gauss-Jordan with partial pivoting on [A | I] in
-// shared memory.  Resets slots to ascending occupied order.  aug: nf x (2nf+1),
-// fac: nf.  Writes G (stride nf+1) into g_out.  Returns false if singular or
-// non-finite; a non-finite entry (NaN/Inf parameters) gives NaN sign and
-// log-amplitude, a singular matrix sign 0 and -inf.
-__device__ bool warp_refresh(const double* __restrict__ M, int nf, int N, uint64_t up, uint64_t dn, double* aug,
-                             double* fac, double* g_out, uint8_t* slot, double& sign, double& logabs) {
-  const int lane = threadIdx.x & 31;
-  const int ld = 2 * nf + 1;
-  const int gs0 = gstride(nf);
-  if (__popcll(up) + __popcll(dn) != nf) {
-    // wrong electron count for this orbital matrix: report singular, leave a
-    // well-formed (all-zero) state so later kernels never index with garbage
-    for (int k = lane; k < nf; k += 32) slot[k] = 0;
-    for (int idx = lane; idx < nf * nf; idx += 32) g_out[(idx / nf) * gs0 + idx % nf] = 0.0;
-    __syncwarp();
-    sign = 0.0;
-    logabs = -INFINITY;
-    return false;
-  }
-  // ascending occupied orbitals -> slots
-  for (int o = lane; o < 2 * N; o += 32) {
-    if (orb_occupied(up, dn, N, o)) {
-      int k = orb_prefix(up, dn, N, o);
-      if (k < nf) slot[k] = (uint8_t)o;
-    }
-  }
-  __syncwarp();
-  for (int idx = lane; idx < nf * 2 * nf; idx += 32) {
-    int r = idx / (2 * nf), c = idx - r * 2 * nf;
-    aug[r * ld + c] = (c < nf) ? M[(int)slot[r] * nf + c] : (c - nf == r ? 1.0 : 0.0);
-  }
-  __syncwarp();
-  double s = 1.0, la = 0.0;
-  bool ok = true, nonfinite = false;
-  for (int k = 0; k < nf; ++k) {
-    // pivot search over rows >= k (smallest index wins ties; NaN ranks first)
-    double best = -1.0;
-    int bi = k;
-    for (int r = k + lane; r < nf; r += 32) {
-      double v = fabs(aug[r * ld + k]);
-      if (v != v) v = INFINITY;
-      if (v > best) { best = v; bi = r; }
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      double ob = __shfl_xor_sync(VMC_FULL_MASK, best, o);
-      int oi = __shfl_xor_sync(VMC_FULL_MASK, bi, o);
-      if (ob > best || (ob == best && oi < bi)) { best = ob; bi = oi; }
-    }
-    if (!(best > 0.0) || !isfinite(best)) {
-      nonfinite = !isfinite(best);
-      ok = false;
-      break;
-    }
-    if (bi != k) {
-      for (int c = lane; c < 2 * nf; c += 32) {
-        double t0 = aug[k * ld + c];
-        aug[k * ld + c] = aug[bi * ld + c];
-        aug[bi * ld + c] = t0;
-      }
-      s = -s;
-      __syncwarp();
-    }
-    double d = aug[k * ld + k];
-    if (d < 0) s = -s;
-    la += log(fabs(d));
-    __syncwarp();
-    double inv = 1.0 / d;
-    for (int c = lane; c < 2 * nf; c += 32) aug[k * ld + c] *= inv;
-    for (int r = lane; r < nf; r += 32) fac[r] = (r == k) ? 0.0 : aug[r * ld + k];
-    __syncwarp();
-    for (int idx = lane; idx < nf * 2 * nf; idx += 32) {
-      int r = idx / (2 * nf), c = idx - r * 2 * nf;
-      if (r != k) aug[r * ld + c] -= fac[r] * aug[k * ld + c];
-    }
-    __syncwarp();
-  }
-  const int gs = gstride(nf);
-  for (int idx = lane; idx < nf * nf; idx += 32) {
-    int k = idx / nf, c = idx - k * nf;
-    g_out[k * gs + c] = ok ? aug[c * ld + nf + k] : 0.0;
-  }
-  __syncwarp();
-  const double qnan = __longlong_as_double(0x7ff8000000000000ll);
-  sign = ok ? s : (nonfinite ? qnan : 0.0);
-  logabs = ok ? la : (nonfinite ? qnan : -INFINITY);
-  return ok;
-}
+// 1/|d| for finite d != 0 (rcp_pos, common.cuh) with d's sign.
+__device__ __forceinline__ double rcp_signed(double d) { return copysign(rcp_pos(fabs(d)), d); }
 
 __device__ __forceinline__ double dot_row(const double* __restrict__ Mrow, const double* Grow, int nf) {
   double acc = 0.0;
@@ -133,32 +40,162 @@ __device__ __forceinline__ int find_slot(const uint8_t* slot, int nf, int orb) {
 }
 
 // ---------------------------------------------------------------------------
-__global__ void k_slater_refresh(const double* __restrict__ M, int nf, int N, const uint64_t* __restrict__ occ,
-                                 int64_t B, double* __restrict__ G, uint8_t* __restrict__ slot_orb,
-                                 double* __restrict__ sign, double* __restrict__ logabs, int32_t* __restrict__ n_acc,
-                                 int threshold, int* __restrict__ n_singular) {
-  extern __shared__ double sm[];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int64_t w = (int64_t)blockIdx.x * (blockDim.x >> 5) + warp;
+// Full re-inversion: in-place Gauss-Jordan exchange steps with partial
+// pivoting on the nf x nf matrix in registers (NT = nf rounded up to a tile).
+// An FP64 instruction takes a warp 64 clocks of its SM quarter on GB300, so the
+// nf^3 multiply-adds are the limit: the matrix is inverted in place (the
+// augmented [A | I] form takes twice as many), and a walker's matrix is spread
+// over NW warps so that all four quarters work on it (NT > 32: 4 warps of a
+// CTA, NT / 8 x NT / 16 elements a thread; smaller: one warp, NT / 4 x NT / 8).
+// Thread (ty, tx) holds the elements (ty + TY i, tx + TX j).  Step k exchanges
+// row variable p (the pivot row, searched over the rows not used yet) with
+// column variable k:
+//   a_ij -= a_ik v_j,  a_ik = a_ik / d,  a_pj = -v_j,  a_pk = 1 / d,
+//   v_j = a_pj / d, d = a_pk,
+// one multiply-add per element with the operands of row p and column k
+// replaced.  No rows move: with p_k the pivot row of step k the inverse is
+// A^-1[k][p_j] = a[p_k][j], and the parity of the permutation k -> p_k is
+// counted from the unused rows above each pivot row.  Resets slots to
+// ascending occupied order.  A singular matrix gives sign 0, logabs -inf and G = 0; a
+// non-finite entry (NaN or Inf parameters) NaN sign and log-amplitude.
+template <int NT, int NW>
+__global__ void __launch_bounds__(128) k_slater_refresh(
+    const double* __restrict__ M, int nf, int N, const uint64_t* __restrict__ occ, int64_t B, double* __restrict__ G,
+    uint8_t* __restrict__ slot_orb, double* __restrict__ sign, double* __restrict__ logabs, int32_t* __restrict__ n_acc,
+    int threshold, int* __restrict__ n_singular) {
+  constexpr int TX = NW == 4 ? 16 : 8, TY = 32 * NW / TX, NI = NT / TY, NJ = NT / TX;
+  constexpr int PER = NT * (NT + 1) + 4 * NT;     // doubles per walker
+  extern __shared__ __align__(16) double sm[];
+  const int tid = NW == 4 ? threadIdx.x : (threadIdx.x & 31), lane = threadIdx.x & 31;
+  const int64_t w = NW == 4 ? (int64_t)blockIdx.x : (int64_t)blockIdx.x * 4 + (threadIdx.x >> 5);
   if (w >= B) return;
   if (threshold > 0 && n_acc && n_acc[w] < threshold) return;
-  const int per = nf * (2 * nf + 1) + nf + nf * gstride(nf) + 8;
-  double* aug = sm + (size_t)warp * per;
-  double* fac = aug + nf * (2 * nf + 1);
-  double* gs = fac + nf;
-  uint8_t* sl = (uint8_t*)(gs + nf * gstride(nf));
-  double s, la;
-  bool ok = warp_refresh(M, nf, N, occ[2 * w], occ[2 * w + 1], aug, fac, gs, sl, s, la);
-  for (int idx = lane; idx < nf * nf; idx += 32) {
-    int k = idx / nf, c = idx - k * nf;
-    G[w * nf * nf + idx] = gs[k * gstride(nf) + c];
+  auto sync = [] { if (NW == 4) __syncthreads(); else __syncwarp(); };
+  double* base = sm + (NW == 4 ? 0 : (size_t)(threadIdx.x >> 5) * PER);
+  double* gst = base;                       // staged G, NT x (NT + 1)
+  double* col = gst + NT * (NT + 1);        // column k
+  double* prow = col + NT;                  // pivot row
+  double* dpiv = prow + NT;                 // pivots
+  uint8_t* pof = reinterpret_cast<uint8_t*>(dpiv + NT);   // p_k
+  uint8_t *kof = pof + NT, *sl = kof + NT;                // its inverse; the slots' orbitals
+  const uint64_t up = occ[2 * w], dn = occ[2 * w + 1];
+  const int tx = tid % TX, ty = tid / TX;
+  const double qnan = __longlong_as_double(0x7ff8000000000000ll);
+  if (__popcll(up) + __popcll(dn) != nf) {
+    // wrong electron count for this orbital matrix: report singular, leave a
+    // well-formed (all-zero) state so later kernels never index with garbage
+    for (int k = tid; k < nf; k += 32 * NW) slot_orb[w * nf + k] = 0;
+    for (int idx = tid; idx < nf * nf; idx += 32 * NW) G[w * nf * nf + idx] = 0.0;
+    if (tid == 0) {
+      sign[w] = 0.0;
+      logabs[w] = -INFINITY;
+      if (n_acc) n_acc[w] = 0;
+      if (n_singular) atomicAdd(n_singular, 1);
+    }
+    return;
   }
-  for (int k = lane; k < nf; k += 32) slot_orb[w * nf + k] = sl[k];
-  if (lane == 0) {
-    sign[w] = s;
-    logabs[w] = la;
-    if (n_acc) n_acc[w] = 0;
-    if (!ok && s == 0.0 && n_singular) atomicAdd(n_singular, 1);   // singular, not non-finite
+  for (int o = tid; o < 2 * N; o += 32 * NW)   // ascending occupied orbitals -> slots
+    if (orb_occupied(up, dn, N, o)) sl[orb_prefix(up, dn, N, o)] = (uint8_t)o;
+  sync();
+  double a[NI][NJ];
+#pragma unroll
+  for (int i = 0; i < NI; ++i)
+#pragma unroll
+    for (int j = 0; j < NJ; ++j) {
+      const int r = ty + TY * i, c = tx + TX * j;
+      a[i][j] = (r < nf && c < nf) ? M[(int)sl[r] * nf + c] : (r == c ? 1.0 : 0.0);
+    }
+  if (tx == 0)
+#pragma unroll
+    for (int i = 0; i < NI; ++i) col[ty + TY * i] = a[i][0];
+  uint64_t live = nf == 64 ? ~0ull : ((1ull << nf) - 1ull);   // rows not used as pivots yet
+  int par = 0;
+  bool ok = true, nonfinite = false;
+#pragma unroll 1
+  for (int k = 0; k < nf; ++k) {
+    sync();   // column k complete
+    // pivot: largest |a_ik| over the live rows, smallest row on a tie, from the
+    // bit patterns (a NaN ranks above every number)
+    unsigned h0 = 0, l0 = 0, h1 = 0, l1 = 0;
+    const int r0 = lane % NT, r1 = lane + 32;
+    if ((live >> r0) & 1ull) { const double v = fabs(col[r0]); h0 = (unsigned)__double2hiint(v) + 1u; l0 = (unsigned)__double2loint(v); }
+    if (NT > 32 && r1 < NT && ((live >> (r1 & 63)) & 1ull)) {
+      const double v = fabs(col[r1 < NT ? r1 : 0]);
+      h1 = (unsigned)__double2hiint(v) + 1u;
+      l1 = (unsigned)__double2loint(v);
+    }
+    const unsigned mh = __reduce_max_sync(VMC_FULL_MASK, max(h0, h1));
+    const unsigned ml = __reduce_max_sync(VMC_FULL_MASK, max(h0 == mh ? l0 : 0u, h1 == mh ? l1 : 0u));
+    const unsigned b0 = __ballot_sync(VMC_FULL_MASK, h0 == mh && l0 == ml);
+    const unsigned b1 = __ballot_sync(VMC_FULL_MASK, h1 == mh && l1 == ml);
+    const int p = b0 ? (__ffs(b0) - 1) % NT : 31 + __ffs(b1);
+    if ((mh == 1u && ml == 0u) || mh >= 0x7ff00001u) {   // zero, or NaN / Inf
+      nonfinite = mh >= 0x7ff00001u;
+      ok = false;
+      break;
+    }
+    const double d = col[p];
+    const double r = rcp_signed(d);
+    par ^= __popcll(live & ((1ull << p) - 1ull)) & 1;
+    live &= ~(1ull << p);
+    if (tid == 0) { dpiv[k] = d; pof[k] = (uint8_t)p; kof[p] = (uint8_t)k; }
+    {
+      const int pi = p / TY;
+      const bool mine = ty == p % TY;
+#pragma unroll
+      for (int j = 0; j < NJ; ++j) {   // selects: a branch per i would index the registers through local memory
+        double v = a[0][j];
+#pragma unroll
+        for (int i = 1; i < NI; ++i) v = i == pi ? a[i][j] : v;
+        if (mine) prow[tx + TX * j] = v;
+      }
+    }
+    double u[NI];
+#pragma unroll
+    for (int i = 0; i < NI; ++i) u[i] = (ty + TY * i == p) ? -1.0 : -col[ty + TY * i];
+    sync();   // pivot row complete, column k read
+    const int jn = (k + 1) / TX;
+#pragma unroll
+    for (int j = 0; j < NJ; ++j) {
+      const int c = tx + TX * j;
+      const double v = c == k ? -r : prow[c] * r;
+#pragma unroll
+      for (int i = 0; i < NI; ++i)
+        a[i][j] = fma(u[i], v, (c == k || ty + TY * i == p) ? 0.0 : a[i][j]);
+      if (j == jn && c == k + 1)
+#pragma unroll
+        for (int i = 0; i < NI; ++i) col[ty + TY * i] = a[i][j];
+    }
+  }
+  sync();
+  if (ok) {   // G[p_j][c] = A^-1[c][p_j] = a[p_c][j]
+#pragma unroll
+    for (int i = 0; i < NI; ++i)
+#pragma unroll
+      for (int j = 0; j < NJ; ++j) {
+        const int rr = ty + TY * i, c = tx + TX * j;
+        if (rr < nf && c < nf) gst[(int)pof[c] * (NT + 1) + (int)kof[rr]] = a[i][j];
+      }
+  }
+  sync();
+  for (int idx = tid; idx < nf * nf; idx += 32 * NW) {
+    const int k = idx / nf, c = idx - k * nf;
+    G[w * nf * nf + idx] = ok ? gst[k * (NT + 1) + c] : 0.0;
+  }
+  for (int k = tid; k < nf; k += 32 * NW) slot_orb[w * nf + k] = sl[k];
+  if (tid < 32) {
+    double la = 0.0;
+    int neg = 0;
+    if (ok)
+      for (int k = lane; k < nf; k += 32) { la += log(fabs(dpiv[k])); neg ^= dpiv[k] < 0.0; }
+    la = warp_sum(la);
+    neg = (__popc(__ballot_sync(VMC_FULL_MASK, neg)) & 1) ^ par;
+    if (lane == 0) {
+      sign[w] = ok ? (neg ? -1.0 : 1.0) : (nonfinite ? qnan : 0.0);
+      logabs[w] = ok ? la : (nonfinite ? qnan : -INFINITY);
+      if (n_acc) n_acc[w] = 0;
+      if (!ok && !nonfinite && n_singular) atomicAdd(n_singular, 1);
+    }
   }
 }
 
@@ -188,6 +225,9 @@ __global__ void k_slater_sweep(const double* __restrict__ M, int nf, int N, uint
   double sg = sign[w], la = logabs[w];
   int nacc = n_acc[w];
   const int j0 = lane, j1 = lane + 32;
+  const int j0c = j0 < nf ? j0 : 0, j1c = j1 < nf ? j1 : 0;   // lanes past nf compute row 0's products, unused
+  double rm = 1.0;
+  int re = 0;
   for (int s = 0; s < n_sweeps; ++s) {
     for (int e = 0; e < E; ++e) {
       const int i = edges[2 * e], j = edges[2 * e + 1];
@@ -217,16 +257,65 @@ __global__ void k_slater_sweep(const double* __restrict__ M, int nf, int N, uint
       }
       const double* m1 = M + (size_t)mv.b[0] * nf;
       const double* m2 = (mv.n == 2) ? M + (size_t)mv.b[1] * nf : m1;
+      // acceptance ratio: the products of the new orbital rows with the
+      // replaced rows of G only (lane = column); the products with every row
+      // follow on acceptance
+      double r;
+      {
+        const double* g1 = g + k1 * gsd;
+        double q0 = 0.0, q1 = 0.0, q2 = 0.0, q3 = 0.0;
+        if (mv.n == 2) {
+          const double* g2 = g + k2 * gsd;
+          for (int c = lane; c < nf; c += 32) {
+            const double x1 = m1[c], x2 = m2[c], y1 = g1[c], y2 = g2[c];
+            q0 = fma(x1, y1, q0); q1 = fma(x1, y2, q1); q2 = fma(x2, y1, q2); q3 = fma(x2, y2, q3);
+          }
+          // four sums at once: each exchange halves the values a lane carries
+          const bool hi16 = lane & 16, hi8 = lane & 8;
+          double s0 = hi16 ? q2 : q0, s1 = hi16 ? q3 : q1;
+          s0 += __shfl_xor_sync(VMC_FULL_MASK, hi16 ? q0 : q2, 16);
+          s1 += __shfl_xor_sync(VMC_FULL_MASK, hi16 ? q1 : q3, 16);
+          double t = hi8 ? s1 : s0;
+          t += __shfl_xor_sync(VMC_FULL_MASK, hi8 ? s0 : s1, 8);
+#pragma unroll
+          for (int o = 4; o > 0; o >>= 1) t += __shfl_xor_sync(VMC_FULL_MASK, t, o);
+          const double R00 = __shfl_sync(VMC_FULL_MASK, t, 0), R01 = __shfl_sync(VMC_FULL_MASK, t, 8);
+          const double R10 = __shfl_sync(VMC_FULL_MASK, t, 16), R11 = __shfl_sync(VMC_FULL_MASK, t, 24);
+          r = R00 * R11 - R01 * R10;
+        } else {
+          for (int c = lane; c < nf; c += 32) q0 = fma(m1[c], g1[c], q0);
+          r = warp_sum(q0);
+        }
+      }
+      if (!((double)u_acc < r * r)) continue;
+      // accept: rank-1 / rank-2 inverse update
       double w1a = 0, w1b = 0, w2a = 0, w2b = 0;
-      if (j0 < nf) { w1a = dot_row(m1, g + j0 * gsd, nf); if (mv.n == 2) w2a = dot_row(m2, g + j0 * gsd, nf); }
-      if (j1 < nf) { w1b = dot_row(m1, g + j1 * gsd, nf); if (mv.n == 2) w2b = dot_row(m2, g + j1 * gsd, nf); }
+      if (mv.n == 2) {
+        for (int c = 0; c < nf; ++c) {
+          const double x1 = m1[c], x2 = m2[c], ya = g[j0c * gsd + c];
+          w1a = fma(x1, ya, w1a);
+          w2a = fma(x2, ya, w2a);
+          if (nf > 32) {
+            const double yb = g[j1c * gsd + c];
+            w1b = fma(x1, yb, w1b);
+            w2b = fma(x2, yb, w2b);
+          }
+        }
+      } else {
+        for (int c = 0; c < nf; ++c) {
+          const double x1 = m1[c];
+          w1a = fma(x1, g[j0c * gsd + c], w1a);
+          if (nf > 32) w1b = fma(x1, g[j1c * gsd + c], w1b);
+        }
+      }
       // gather R entries from the owning lanes
       auto get = [&](double va, double vb, int k) {
         double a = __shfl_sync(VMC_FULL_MASK, va, k & 31);
         double b = __shfl_sync(VMC_FULL_MASK, vb, k & 31);
         return k < 32 ? a : b;
       };
-      double R00 = get(w1a, w1b, k1), R01 = 0, R10 = 0, R11 = 0, r;
+      double R01 = 0, R10 = 0, R11 = 0;
+      const double R00 = get(w1a, w1b, k1);
       if (mv.n == 2) {
         R01 = get(w1a, w1b, k2);
         R10 = get(w2a, w2b, k1);
@@ -235,15 +324,12 @@ __global__ void k_slater_sweep(const double* __restrict__ M, int nf, int N, uint
       } else {
         r = R00;
       }
-      const double prob = r * r;
-      if (!((double)u_acc < prob)) continue;
-      // accept: rank-1 / rank-2 inverse update
       for (int c = lane; c < nf; c += 32) {
         tmp[c] = g[k1 * gsd + c];
         if (mv.n == 2) tmp[nf + c] = g[k2 * gsd + c];
       }
       __syncwarp();
-      const double ir = 1.0 / r;
+      const double ir = rcp_signed(r);
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
         const int jj = h ? j1 : j0;
@@ -259,9 +345,11 @@ __global__ void k_slater_sweep(const double* __restrict__ M, int nf, int N, uint
         }
         double* row = g + jj * gsd;
         if (mv.n == 2) {
-          for (int c = 0; c < nf; ++c) row[c] -= alpha * tmp[c] + beta * tmp[nf + c];
+#pragma unroll 4
+          for (int c = 0; c < nf; ++c) row[c] = fma(-beta, tmp[nf + c], fma(-alpha, tmp[c], row[c]));
         } else {
-          for (int c = 0; c < nf; ++c) row[c] -= alpha * tmp[c];
+#pragma unroll 4
+          for (int c = 0; c < nf; ++c) row[c] = fma(-alpha, tmp[c], row[c]);
         }
       }
       __syncwarp();
@@ -272,10 +360,22 @@ __global__ void k_slater_sweep(const double* __restrict__ M, int nf, int N, uint
       __syncwarp();
       up = up1; dn = dn1;
       sg *= ((r < 0) != (par != 0)) ? -1.0 : 1.0;
-      la += log(fabs(r));
+      // log|psi| as a running product of the ratios, renormalised to a mantissa
+      // in [1, 2) and an exponent (one logarithm per launch; r is finite and
+      // not zero here, |r| > sqrt(u))
+      rm *= fabs(r);
+      const int hi = __double2hiint(rm);
+      if ((unsigned)((hi >> 20) - 1) < 0x7feu) {
+        re += (hi >> 20) - 1023;
+        rm = __hiloint2double((hi & 0xfffff) | (1023 << 20), __double2loint(rm));
+      } else {           // subnormal or overflowed product
+        la += log(rm);
+        rm = 1.0;
+      }
       ++nacc;
     }
   }
+  la += log(rm) + (double)re * 0.69314718055994530942;
   for (int idx = lane; idx < nf * nf; idx += 32) {
     int k = idx / nf, c = idx - k * nf;
     G[w * nf * nf + idx] = g[k * gsd + c];
@@ -349,8 +449,16 @@ __global__ void k_slater_grad(const double* __restrict__ G, const uint8_t* __res
   }
 }
 
-size_t refresh_smem_per_warp(int nf) {
-  return ((size_t)nf * (2 * nf + 1) + nf + (size_t)nf * (nf + 1) + 8) * sizeof(double);
+template <int NT, int NW>
+int launch_refresh(const double* M, int nf, int N, const uint64_t* occ, int64_t B, double* G, uint8_t* slot_orb,
+                   double* sign, double* logabs, int32_t* n_acc, int threshold, int* n_singular, cudaStream_t st) {
+  constexpr int wpc = NW == 4 ? 1 : 4;   // walkers per CTA
+  const size_t smem = (size_t)wpc * (NT * (NT + 1) + 4 * NT) * sizeof(double);
+  cudaFuncSetAttribute(k_slater_refresh<NT, NW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  k_slater_refresh<NT, NW><<<(unsigned)((B + wpc - 1) / wpc), 128, smem, st>>>(M, nf, N, occ, B, G, slot_orb, sign,
+                                                                              logabs, n_acc, threshold, n_singular);
+  VMC_CUDA_CHECK_LAUNCH();
+  return VMC_OK;
 }
 size_t sweep_smem_per_warp(int nf) { return ((size_t)nf * (nf + 1) + 2 * nf + 8) * sizeof(double); }
 
@@ -372,14 +480,16 @@ int vmc_slater_refresh(const double* M, int n_orb, int nf, const uint64_t* occ, 
   if (B < 0 || nf < 1 || nf > kMaxNf || n_sites < 1 || n_sites > 64 || n_orb != 2 * n_sites) return VMC_ERR_ARGS;
   if (B == 0) return VMC_OK;
   if (!M || !occ || !G || !slot_orb || !sign || !logabs) return VMC_ERR_ARGS;
-  size_t per = refresh_smem_per_warp(nf);
-  int wpb = warps_per_block(per);
-  size_t smem = per * wpb;
-  cudaFuncSetAttribute(k_slater_refresh, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  k_slater_refresh<<<(unsigned)((B + wpb - 1) / wpb), 32 * wpb, smem, (cudaStream_t)stream>>>(
-      M, nf, n_sites, occ, B, G, slot_orb, sign, logabs, n_acc, threshold, d_n_singular);
-  VMC_CUDA_CHECK_LAUNCH();
-  return VMC_OK;
+  cudaStream_t st = (cudaStream_t)stream;
+  // one warp a walker up to 32 (a barrier a step costs more than the idle
+  // quarters there), four above, the tile no wider than nf asks for
+  if (nf <= 16)
+    return launch_refresh<16, 1>(M, nf, n_sites, occ, B, G, slot_orb, sign, logabs, n_acc, threshold, d_n_singular, st);
+  if (nf <= 32)
+    return launch_refresh<32, 1>(M, nf, n_sites, occ, B, G, slot_orb, sign, logabs, n_acc, threshold, d_n_singular, st);
+  if (nf <= 48)
+    return launch_refresh<48, 4>(M, nf, n_sites, occ, B, G, slot_orb, sign, logabs, n_acc, threshold, d_n_singular, st);
+  return launch_refresh<64, 4>(M, nf, n_sites, occ, B, G, slot_orb, sign, logabs, n_acc, threshold, d_n_singular, st);
 }
 
 int vmc_slater_sweep(const double* M, int n_orb, int nf, uint64_t* occ, int64_t B, int n_sites, const int32_t* edges,
