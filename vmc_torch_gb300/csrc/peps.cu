@@ -1266,6 +1266,483 @@ __global__ void __launch_bounds__(512)
   }
 }
 
+// ---------------------------------------------------------------------------
+// The same log-derivatives for FP32, D = 4, DA = 16 (Lx = 6 at D = 4), register
+// tiled.  k_peps_grad forms one output per thread with two scalar
+// shared-memory loads per multiply-add (4.48 ms for 512 configurations of the 6x6
+// lattice, 24 GFLOP: 5 TFLOP/s).  Here 256 threads take four top-bond slices at a
+// time, every contraction gives a thread 16 outputs from 16-byte or register
+// operands (3 to 8 multiply-adds per load), the cotangent chain GX3 -> GX2 stays
+// in registers, and the sums over slices that make up dZ/dA2, dZ/dA3, dZ/dM and
+// dZ/dN are 4 x 4 register tiles over a split of the long index, folded by
+// shuffles.  Two CTAs per SM (107 KB each); the left environments are read
+// from the workspace (L1/L2).
+// ---------------------------------------------------------------------------
+namespace pg {
+
+constexpr int NT = 256, NWARP = 8;
+constexpr int RS = 272, SS = 4 * RS;    // row strides of the staged slices: [slice][r2 or u2][64], 16 floats apart in banks
+constexpr int o_Y = 0, o_X2 = o_Y + 4096, o_X3 = o_X2 + 4 * SS, o_G3 = o_X3 + 4 * SS, o_F = o_G3 + 4 * SS,
+              o_M = o_F + 4096, o_N = o_M + 1024, o_Nt = o_N + 1024, o_GM = o_Nt + 1024, o_GN = o_GM + 1024,
+              o_GA2 = o_GN + 2048, o_GA3 = o_GA2 + 256, o_GT = o_GA3 + 256, o_red = o_GT + 1024, o_col = o_red + 32;
+constexpr size_t SMEM = (size_t)(o_col + 6 * 256) * 4 + 16 * sizeof(int);
+
+// 16 partial sums over the 16 lanes that differ in lane bits 0..3 -> the total
+// of value (lane & 15) in every lane
+__device__ __forceinline__ float fold16(float (&v)[16]) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int w = 8; w > 0; w >>= 1) {
+    const bool up = lane & w;
+#pragma unroll
+    for (int i = 0; i < w; ++i) {
+      const float send = up ? v[i] : v[i + w], keep = up ? v[i + w] : v[i];
+      v[i] = keep + __shfl_xor_sync(VMC_FULL_MASK, send, w);
+    }
+  }
+  return v[0];
+}
+
+// v[i * 4 + j] += x_i . y_j over four consecutive k
+__device__ __forceinline__ void outer4(const float4 (&x)[4], const float4 (&y)[4], float (&v)[16]) {
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      v[i * 4 + j] = fmaf(x[i].x, y[j].x, fmaf(x[i].y, y[j].y, fmaf(x[i].z, y[j].z, fmaf(x[i].w, y[j].w, v[i * 4 + j]))));
+}
+__device__ __forceinline__ float4 ld4(const float* p) { return *reinterpret_cast<const float4*>(p); }
+
+// Y, X2, X3 of slices b0..b0+3 (staged; X3 also in x3[r3 * 4 + d3] of thread
+// (slice, r2, a')); E: the column's left environment (shared or global)
+__device__ __forceinline__ void forward4(float* sm, const float* E, const float* A2, const float* A3, int b0,
+                                         float (&x3)[16]) {
+  const int t = threadIdx.x;
+  float *Y = sm + o_Y, *X2 = sm + o_X2, *X3 = sm + o_X3;
+  const float* M = sm + o_M;
+  {
+    float y[4][4];   // [slice][u2] at rest = t
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int u = 0; u < 4; ++u) y[i][u] = 0.f;
+#pragma unroll
+    for (int a = 0; a < 16; ++a) {
+      const float e = E[a * 256 + t];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const float4 m = ld4(M + (a * 4 + u) * 16 + b0);
+        y[0][u] = fmaf(m.x, e, y[0][u]);
+        y[1][u] = fmaf(m.y, e, y[1][u]);
+        y[2][u] = fmaf(m.z, e, y[2][u]);
+        y[3][u] = fmaf(m.w, e, y[3][u]);
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int u = 0; u < 4; ++u) Y[i * 1024 + u * 256 + t] = y[i][u];
+  }
+  __syncthreads();
+  {
+    const int b = t >> 6, l3a = t & 63;
+    float x[16];     // [r2][d2]
+#pragma unroll
+    for (int i = 0; i < 16; ++i) x[i] = 0.f;
+#pragma unroll
+    for (int l = 0; l < 4; ++l)
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const float v = Y[b * 1024 + u * 256 + l * 64 + l3a];
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+          const float4 c = ld4(A2 + ((l * 4 + u) * 4 + r) * 4);
+          x[r * 4] = fmaf(c.x, v, x[r * 4]);
+          x[r * 4 + 1] = fmaf(c.y, v, x[r * 4 + 1]);
+          x[r * 4 + 2] = fmaf(c.z, v, x[r * 4 + 2]);
+          x[r * 4 + 3] = fmaf(c.w, v, x[r * 4 + 3]);
+        }
+      }
+#pragma unroll
+    for (int i = 0; i < 16; ++i) X2[b * SS + (i >> 2) * RS + (i & 3) * 64 + l3a] = x[i];
+  }
+  __syncthreads();
+  {
+    const int b = t >> 6, r2 = (t >> 4) & 3, ap = t & 15;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) x3[i] = 0.f;
+#pragma unroll
+    for (int l = 0; l < 4; ++l)
+#pragma unroll
+      for (int d = 0; d < 4; ++d) {
+        const float v = X2[b * SS + r2 * RS + d * 64 + l * 16 + ap];
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+          const float4 c = ld4(A3 + ((l * 4 + d) * 4 + r) * 4);
+          x3[r * 4] = fmaf(c.x, v, x3[r * 4]);
+          x3[r * 4 + 1] = fmaf(c.y, v, x3[r * 4 + 1]);
+          x3[r * 4 + 2] = fmaf(c.z, v, x3[r * 4 + 2]);
+          x3[r * 4 + 3] = fmaf(c.w, v, x3[r * 4 + 3]);
+        }
+      }
+#pragma unroll
+    for (int i = 0; i < 16; ++i) X3[b * SS + r2 * RS + (i >> 2) * 64 + (i & 3) * 16 + ap] = x3[i];
+  }
+}
+
+__global__ void __launch_bounds__(NT, 2)
+    k_peps_grad_tiled(const float* __restrict__ tens, int Ly, const uint64_t* __restrict__ occ, int64_t R,
+                      float* __restrict__ O, int64_t ldo, float* __restrict__ env) {
+  constexpr int Lx = 6, D4 = 256, ESZ = 4096;
+  extern __shared__ __align__(16) float sm[];
+  float *F = sm + o_F, *M = sm + o_M, *Nn = sm + o_N, *Nt = sm + o_Nt, *GM = sm + o_GM, *GN = sm + o_GN;
+  float *GA2 = sm + o_GA2, *GA3 = sm + o_GA3, *GT = sm + o_GT, *red = sm + o_red, *tcol = sm + o_col;
+  int* pexp = reinterpret_cast<int*>(tcol + Lx * D4);
+  const int64_t w = blockIdx.x;
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  const uint64_t up = occ[2 * w], dn = occ[2 * w + 1];
+  float* envw = env + (size_t)w * (size_t)(Ly + 1) * ESZ;
+  const float *A2 = tcol + 2 * D4, *A3 = tcol + 3 * D4;
+
+  auto load_col = [&](int c) {
+    for (int o = t; o < Lx * D4; o += NT) {
+      const int r = o >> 8, idx = o & 255;
+      const int site = r * Ly + c;
+      float v = tens[((size_t)site * 4 + site_state(up, dn, site)) * D4 + idx];
+      if (r > 0) {
+        const int l = idx >> 6, u = (idx >> 4) & 3;
+        const uint64_t m = row_mask(r, Ly, c);
+        if (u & (l ^ (__popcll(up & m) + __popcll(dn & m))) & 1) v = -v;
+      }
+      tcol[o] = v;
+    }
+    __syncthreads();
+    build_boundary<float, 4, 16>(tcol, Lx, true, M, sm + o_Y, sm + o_X2, 1.f);
+    build_boundary<float, 4, 16>(tcol, Lx, false, Nn, sm + o_Y, sm + o_X2, 1.f);
+  };
+
+  // ---------------- forward: store E^_c, exponents p_c (E in F's place, E' in G3's) ----------------
+  for (int o = t; o < ESZ; o += NT) F[o] = (o == 0) ? 1.f : 0.f;
+  int pcur = 0;
+  for (int c = 0; c < Ly; ++c) {
+    __syncthreads();
+    load_col(c);
+    for (int o = t; o < ESZ; o += NT) envw[(size_t)c * ESZ + o] = F[o];
+    if (t == 0) pexp[c] = pcur;
+    float* En = sm + o_G3;
+#pragma unroll 1
+    for (int b0 = 0; b0 < 16; b0 += 4) {
+      float x3[16];
+      __syncthreads();
+      forward4(sm, F, A2, A3, b0, x3);
+      __syncthreads();
+      // E'[b][r2 r3][b'] = sum_{d3,a'} X3 N: a thread the rows r3 and a quad of b', K = a' at one d3
+      const int nq = lane & 3, d3 = (lane >> 2) & 3, br = warp * 2 + (lane >> 4);   // br = slice * 4 + r2
+      const float* xs = sm + o_X3 + (br >> 2) * SS + (br & 3) * RS + d3 * 16;
+      float acc[16];     // [r3][b' & 3]
+#pragma unroll
+      for (int i = 0; i < 16; ++i) acc[i] = 0.f;
+#pragma unroll
+      for (int kk = 0; kk < 4; ++kk) {
+        float4 x[4];
+#pragma unroll
+        for (int r = 0; r < 4; ++r) x[r] = ld4(xs + r * 64 + kk * 4);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const float4 n = ld4(Nn + (kk * 4 + q) * 64 + d3 * 16 + nq * 4);
+#pragma unroll
+          for (int r = 0; r < 4; ++r) {
+            const float v = q == 0 ? x[r].x : (q == 1 ? x[r].y : (q == 2 ? x[r].z : x[r].w));
+            acc[r * 4] = fmaf(v, n.x, acc[r * 4]);
+            acc[r * 4 + 1] = fmaf(v, n.y, acc[r * 4 + 1]);
+            acc[r * 4 + 2] = fmaf(v, n.z, acc[r * 4 + 2]);
+            acc[r * 4 + 3] = fmaf(v, n.w, acc[r * 4 + 3]);
+          }
+        }
+      }
+      // sum over d3 (lane bits 2, 3); the lane keeps r3 = d3
+      float h[8], q4[4];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const bool hi = lane & 8;
+        h[i] = (hi ? acc[8 + i] : acc[i]) + __shfl_xor_sync(VMC_FULL_MASK, hi ? acc[i] : acc[8 + i], 8);
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const bool hi = lane & 4;
+        q4[i] = (hi ? h[4 + i] : h[i]) + __shfl_xor_sync(VMC_FULL_MASK, hi ? h[i] : h[4 + i], 4);
+      }
+      *reinterpret_cast<float4*>(&En[(b0 + (br >> 2)) * 256 + ((br & 3) * 4 + d3) * 16 + nq * 4]) =
+          make_float4(q4[0], q4[1], q4[2], q4[3]);
+    }
+    __syncthreads();
+    const int e = cta_exp_of_max<float>(En, ESZ, red);
+    if (e == INT_MIN || e == INT_MAX) return;   // psi = 0 or non-finite: the O row stays zero
+    const float s = (float)ldexp(1.0, -e);
+    for (int o = t; o < ESZ; o += NT) F[o] = En[o] * s;
+    pcur += e;
+  }
+  __syncthreads();
+  const float zhat = F[0];
+  if (zhat == 0.f) return;
+  const int Pexp = pcur;
+  __syncthreads();
+
+  // ---------------- reverse sweep ----------------
+  for (int o = t; o < ESZ; o += NT) F[o] = (o == 0) ? 1.f : 0.f;
+  int q = 0;  // F^_{c+1} = F_{c+1} 2^-q
+  for (int c = Ly - 1; c >= 0; --c) {
+    __syncthreads();
+    load_col(c);
+    const float* E = envw + (size_t)c * ESZ;
+    __syncthreads();
+    for (int o = t; o < 1024; o += NT) {   // Nt[b'][a'][d3] = N[a'][d3][b']
+      Nt[o] = Nn[((o >> 2) & 15) * 64 + (o & 3) * 16 + (o >> 6)];
+    }
+    for (int o = t; o < 2048; o += NT) GN[o] = 0.f;
+    GA2[t] = 0.f;
+    GA3[t] = 0.f;
+    float fn[16];       // F_c[a][k = t]
+#pragma unroll
+    for (int a = 0; a < 16; ++a) fn[a] = 0.f;
+#pragma unroll 1
+    for (int b0 = 0; b0 < 16; b0 += 4) {
+      float x3[16];
+      __syncthreads();
+      forward4(sm, E, A2, A3, b0, x3);
+      const int sb = t >> 6, r2 = (t >> 4) & 3, ap = t & 15;
+      // GX3[r3][d3] of (slice, r2, a') = sum_b' F[b][r2 r3][b'] N[a'][d3][b']
+      float g3[16];
+#pragma unroll
+      for (int i = 0; i < 16; ++i) g3[i] = 0.f;
+      const float* Fb = F + (b0 + sb) * 256 + r2 * 64;
+#pragma unroll
+      for (int kk = 0; kk < 4; ++kk) {
+        float4 f[4];
+#pragma unroll
+        for (int r = 0; r < 4; ++r) f[r] = ld4(Fb + r * 16 + kk * 4);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const float4 n = ld4(Nt + (kk * 4 + u) * 64 + ap * 4);
+#pragma unroll
+          for (int r = 0; r < 4; ++r) {
+            const float v = u == 0 ? f[r].x : (u == 1 ? f[r].y : (u == 2 ? f[r].z : f[r].w));
+            g3[r * 4] = fmaf(v, n.x, g3[r * 4]);
+            g3[r * 4 + 1] = fmaf(v, n.y, g3[r * 4 + 1]);
+            g3[r * 4 + 2] = fmaf(v, n.z, g3[r * 4 + 2]);
+            g3[r * 4 + 3] = fmaf(v, n.w, g3[r * 4 + 3]);
+          }
+        }
+      }
+      float* G3 = sm + o_G3;
+#pragma unroll
+      for (int i = 0; i < 16; ++i) G3[sb * SS + r2 * RS + (i >> 2) * 64 + (i & 3) * 16 + ap] = g3[i];
+      __syncthreads();
+      {  // GN[a'][d3][b'] += sum_{slice, r2 r3} X3 F: quads of a' and b' at one d3, one slice a lane half and warp half
+        const int bq = lane & 3, aq = (lane >> 2) & 3, d3 = warp & 3, sl = (warp >> 2) * 2 + (lane >> 4);
+        const float* xs = sm + o_X3 + sl * SS + d3 * 16 + aq * 4;
+        const float* fs = F + (b0 + sl) * 256 + bq * 4;
+        float v[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) v[i] = 0.f;
+#pragma unroll
+        for (int rr = 0; rr < 16; ++rr) {
+          const float4 x = ld4(xs + (rr >> 2) * RS + (rr & 3) * 64), f = ld4(fs + rr * 16);
+          const float xa[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            v[i * 4] = fmaf(xa[i], f.x, v[i * 4]);
+            v[i * 4 + 1] = fmaf(xa[i], f.y, v[i * 4 + 1]);
+            v[i * 4 + 2] = fmaf(xa[i], f.z, v[i * 4 + 2]);
+            v[i * 4 + 3] = fmaf(xa[i], f.w, v[i * 4 + 3]);
+          }
+        }
+        const bool hi = lane & 16;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {   // lower half keeps a' rows 0, 1 of the quad, upper half 2, 3
+          const float send = hi ? v[i] : v[8 + i], keep = hi ? v[8 + i] : v[i];
+          v[i] = keep + __shfl_xor_sync(VMC_FULL_MASK, send, 16);
+        }
+        float* g = GN + (warp >> 2) * 1024;
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          float4* p = reinterpret_cast<float4*>(g + (aq * 4 + (hi ? 2 : 0) + i) * 64 + d3 * 16 + bq * 4);
+          float4 o = *p;
+          o.x += v[i * 4]; o.y += v[i * 4 + 1]; o.z += v[i * 4 + 2]; o.w += v[i * 4 + 3];
+          *p = o;
+        }
+      }
+      const int kg = lane & 15, tile = warp * 2 + (lane >> 4), mt = tile >> 2, nt = tile & 3;
+      {  // GA3[l3 = mt][d2][r3 = nt][d3] += sum over (slice, r2, a') of X2 GX3
+        float v[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) v[i] = 0.f;
+        const float* xs = sm + o_X2 + (kg >> 2) * RS + mt * 16 + (kg & 3) * 4;
+        const float* gs = sm + o_G3 + (kg >> 2) * RS + nt * 64 + (kg & 3) * 4;
+#pragma unroll
+        for (int sl = 0; sl < 4; ++sl) {
+          float4 x[4], y[4];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) { x[i] = ld4(xs + sl * SS + i * 64); y[i] = ld4(gs + sl * SS + i * 16); }
+          outer4(x, y, v);
+        }
+        const float s = fold16(v);    // value (lane & 15) = d2 * 4 + d3
+        GA3[((mt * 4 + (kg >> 2)) * 4 + nt) * 4 + (kg & 3)] += s;
+      }
+      // GX2[l3][d2] of (slice, r2, a') = sum_{r3,d3} A3[l3][d2][r3][d3] GX3
+      float g2[16];
+#pragma unroll
+      for (int ld = 0; ld < 16; ++ld) {
+        float acc = 0.f;
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+          const float4 cf = ld4(A3 + (ld * 4 + r) * 4);
+          acc = fmaf(cf.x, g3[r * 4], fmaf(cf.y, g3[r * 4 + 1], fmaf(cf.z, g3[r * 4 + 2], fmaf(cf.w, g3[r * 4 + 3], acc))));
+        }
+        g2[ld] = acc;
+      }
+      __syncthreads();
+      float* G2 = sm + o_X3;    // X3's place
+#pragma unroll
+      for (int ld = 0; ld < 16; ++ld) G2[sb * SS + r2 * RS + (ld & 3) * 64 + (ld >> 2) * 16 + ap] = g2[ld];
+      __syncthreads();
+      {  // GY[u2][l2] of (slice, l3 a') = sum_{r2,d2} A2[l2][u2][r2][d2] GX2, in X2's place
+        const int l3a = t & 63;
+        float z[16], gy[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) z[i] = G2[sb * SS + (i >> 2) * RS + (i & 3) * 64 + l3a];
+#pragma unroll
+        for (int lu = 0; lu < 16; ++lu) {
+          float acc = 0.f;
+#pragma unroll
+          for (int r = 0; r < 4; ++r) {
+            const float4 cf = ld4(A2 + (lu * 4 + r) * 4);
+            acc = fmaf(cf.x, z[r * 4], fmaf(cf.y, z[r * 4 + 1], fmaf(cf.z, z[r * 4 + 2], fmaf(cf.w, z[r * 4 + 3], acc))));
+          }
+          gy[lu] = acc;
+        }
+        float* GY = sm + o_X2;
+#pragma unroll
+        for (int lu = 0; lu < 16; ++lu) GY[sb * SS + (lu & 3) * RS + (lu >> 2) * 64 + l3a] = gy[lu];
+      }
+      {  // GA2[l2 = mt][u2][r2 = nt][d2] += sum over (slice, l3, a') of Y GX2
+        float v[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) v[i] = 0.f;
+        const float* ys = sm + o_Y + mt * 64 + kg * 4;
+        const float* gs = sm + o_X3 + nt * RS + kg * 4;
+#pragma unroll
+        for (int sl = 0; sl < 4; ++sl) {
+          float4 x[4], y[4];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) { x[i] = ld4(ys + sl * 1024 + i * 256); y[i] = ld4(gs + sl * SS + i * 64); }
+          outer4(x, y, v);
+        }
+        const float s = fold16(v);
+        GA2[((mt * 4 + (kg >> 2)) * 4 + nt) * 4 + (kg & 3)] += s;
+      }
+      __syncthreads();
+      {  // GM[a][u2][b] = sum_k E[a][k] GY[b][u2][k]: a = 4 mt + i, u2 = nt, slice j
+        float v[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) v[i] = 0.f;
+        const float* gs = sm + o_X2 + nt * RS + kg * 4;
+        const float* es = E + mt * 4 * 256 + kg * 4;
+#pragma unroll
+        for (int kk = 0; kk < 4; ++kk) {
+          float4 x[4], y[4];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) { x[i] = ld4(es + i * 256 + kk * 64); y[i] = ld4(gs + i * SS + kk * 64); }
+          outer4(x, y, v);
+        }
+        const float s = fold16(v);
+        GM[((mt * 4 + (kg >> 2)) * 4 + nt) * 16 + b0 + (kg & 3)] = s;
+      }
+      // F_c[a][k] += sum_{u2, slice} M[a][u2][b] GY[b][u2][k]
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const float* gs = sm + o_X2 + u * RS + t;
+        const float z0 = gs[0], z1 = gs[SS], z2 = gs[2 * SS], z3 = gs[3 * SS];
+#pragma unroll
+        for (int a = 0; a < 16; ++a) {
+          const float4 m = ld4(M + (a * 4 + u) * 16 + b0);
+          fn[a] = fmaf(m.x, z0, fmaf(m.y, z1, fmaf(m.z, z2, fmaf(m.w, z3, fn[a]))));
+        }
+      }
+    }
+    __syncthreads();
+    for (int o = t; o < 1024; o += NT) GN[o] += GN[1024 + o];
+    __syncthreads();
+    // ---- boundary rows: dZ/dA for rows 0, 1 from GM and rows 5, 4 from GN (as in k_peps_grad) ----
+    const float *At0 = tcol, *Ab0 = tcol + 5 * D4, *A1 = tcol + D4, *A4 = tcol + 4 * D4;
+    float *gT0 = GT, *gT1 = GT + D4, *gB0 = GT + 2 * D4, *gB1 = GT + 3 * D4;
+    {
+      const int o = t, l = o >> 6, u = (o >> 4) & 3, r = (o >> 2) & 3, d = o & 3;
+      float g0 = 0.f, b0 = 0.f, g1 = 0.f, b1 = 0.f;
+      if (u == 0)
+        for (int l1 = 0; l1 < 4; ++l1)
+          for (int r1 = 0; r1 < 4; ++r1)
+            for (int d1 = 0; d1 < 4; ++d1)
+              g0 += GM[((l * 4 + l1) * 4 + d1) * 16 + (r * 4 + r1)] * A1[((l1 * 4 + d) * 4 + r1) * 4 + d1];
+      if (d == 0)
+        for (int l4 = 0; l4 < 4; ++l4)
+          for (int u4 = 0; u4 < 4; ++u4)
+            for (int r4 = 0; r4 < 4; ++r4)
+              b0 += GN[((l * 4 + l4) * 4 + u4) * 16 + (r * 4 + r4)] * A4[((l4 * 4 + u4) * 4 + r4) * 4 + u];
+      for (int l0 = 0; l0 < 4; ++l0)
+        for (int r0 = 0; r0 < 4; ++r0) {
+          g1 += GM[((l0 * 4 + l) * 4 + d) * 16 + (r0 * 4 + r)] * At0[((l0 * 4 + 0) * 4 + r0) * 4 + u];
+          b1 += GN[((l0 * 4 + l) * 4 + u) * 16 + (r0 * 4 + r)] * Ab0[((l0 * 4 + d) * 4 + r0) * 4 + 0];
+        }
+      gT0[o] = g0;
+      gB0[o] = b0;
+      gT1[o] = g1;
+      gB1[o] = b1;
+    }
+    // ---- F^_c normalised ----
+    float fm = 0.f;
+#pragma unroll
+    for (int a = 0; a < 16; ++a) fm = fmaxf(fm, fabsf(fn[a]));
+    bool bad = false;
+#pragma unroll
+    for (int a = 0; a < 16; ++a) bad |= !(fabsf(fn[a]) < INFINITY);
+    if (bad) fm = INFINITY;
+#pragma unroll
+    for (int sft = 16; sft > 0; sft >>= 1) fm = fmaxf(fm, __shfl_xor_sync(VMC_FULL_MASK, fm, sft));
+    __syncthreads();      // the slices' readers of F are done, GT is complete
+    if (lane == 0) red[warp] = fm;
+    __syncthreads();
+    // ---- write O for the column's sites ----
+    const double scl = ldexp(1.0 / (double)zhat, pexp[c] + q - Pexp);
+    float* Ow = O + (size_t)w * (size_t)ldo;
+    const float* const src[6] = {gT0, gT1, GA2, GA3, gB1, gB0};
+#pragma unroll
+    for (int r = 0; r < Lx; ++r) {
+      float v = src[r][t];
+      const int site = r * Ly + c;
+      if (r > 0) {
+        const int l = t >> 6, u = (t >> 4) & 3;
+        const uint64_t m = row_mask(r, Ly, c);
+        if (u & (l ^ (__popcll(up & m) + __popcll(dn & m))) & 1) v = -v;
+      }
+      Ow[((size_t)site * 4 + site_state(up, dn, site)) * D4 + t] = (float)((double)v * scl);
+    }
+    float mm = 0.f;
+#pragma unroll
+    for (int k = 0; k < NWARP; ++k) mm = fmaxf(mm, red[k]);
+    if (c > 0) {
+      if (mm == 0.f || !(mm < INFINITY)) return;  // nothing flows further left
+      const int e = ilogbf(mm);
+      const float s = (float)ldexp(1.0, -e);
+#pragma unroll
+      for (int a = 0; a < 16; ++a) F[a * 256 + t] = fn[a] * s;
+      q += e;
+    }
+  }
+}
+
+}  // namespace pg
+
 // ---- dispatch over the supported (D, DA) shapes ----
 enum PepsOp { OP_EVAL, OP_SWEEP, OP_TERMS, OP_SWEEP_ENV, OP_ELOC_ENV };
 
@@ -1348,6 +1825,15 @@ template <typename T, int D, int DA>
 int launch_peps_grad(int Lx, int Ly, const void* tens, const uint64_t* occ, int64_t R, void* O, int64_t ldo,
                      void* env, cudaStream_t st) {
   using G = PepsGrad<T, D, DA>;
+  if constexpr (std::is_same<T, float>::value && D == 4 && DA == 16) {   // DA = 16: Lx = 6
+    if (((uintptr_t)env & 15) == 0) {   // its 16-byte loads; the per-output kernel takes any workspace
+      cudaFuncSetAttribute(pg::k_peps_grad_tiled, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pg::SMEM);
+      pg::k_peps_grad_tiled<<<(unsigned)R, pg::NT, pg::SMEM, st>>>((const float*)tens, Ly, occ, R, (float*)O, ldo,
+                                                                 (float*)env);
+      VMC_CUDA_CHECK_LAUNCH();
+      return VMC_OK;
+    }
+  }
   const size_t smem = G::smem_bytes(Lx);
   if (smem > 227 * 1024) return VMC_ERR_UNSUPPORTED;
   cudaFuncSetAttribute(k_peps_grad<T, D, DA>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
