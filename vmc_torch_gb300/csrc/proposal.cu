@@ -25,6 +25,7 @@
 #include <cuda.h>
 #include <cudaTypedefs.h>
 #include "common.cuh"
+#include "sgemm.cuh"
 #include "tc.cuh"
 
 using namespace vmc;
@@ -380,62 +381,58 @@ __global__ void k_prop_reverse(int64_t B, Lat L, const float* __restrict__ logit
 }
 
 // ---------------------------------------------------------------------------
-// training: FP32 CUDA cores
-// C[M x N] = op(A) op(B) (+ bias[n]); row-major; EPI: 0 plain, 1 gelu(pre) with
-// pre stored in aux, 2 accumulate (C += ...), 3 split-K: block z adds the
-// partial product over k in [z kchunk, (z+1) kchunk) to C atomically (C
-// cleared beforehand; used for the weight gradients, whose K is the batch).
-template <int EPI>
-__global__ void k_sgemm(int ta, int tb, int M, int N, int K, const float* __restrict__ A, int lda,
-                        const float* __restrict__ Bm, int ldb, const float* __restrict__ bias, float* __restrict__ C,
-                        int ldc, float* __restrict__ aux, int kchunk) {
-  constexpr int T = 64, TKk = 16;
-  __shared__ float As[TKk][T + 1];
-  __shared__ float Bs[TKk][T + 1];
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  const int m0 = blockIdx.y * T, n0 = blockIdx.x * T;
-  const int kb = EPI == 3 ? blockIdx.z * kchunk : 0;
-  const int ke = EPI == 3 ? min(K, kb + kchunk) : K;
-  float acc[4][4] = {};
-  for (int k0 = kb; k0 < ke; k0 += TKk) {
-    for (int idx = threadIdx.x; idx < T * TKk; idx += 256) {
-      int r, kk;
-      if (ta) { kk = idx / T; r = idx - kk * T; } else { r = idx / TKk; kk = idx - r * TKk; }
-      const int gm = m0 + r, gk = k0 + kk;
-      As[kk][r] = (gm < M && gk < ke) ? (ta ? A[(size_t)gk * lda + gm] : A[(size_t)gm * lda + gk]) : 0.f;
+// training: FP32 CUDA cores (tiles of sgemm.cuh)
+// C[M x N] = op(A) op(B), row-major; AK: A[m][k], else A[k][m]; BK: B[n][k],
+// else B[k][n].  EPI: 0 C = v (+ bias[n]); 1 pre = v + bias[n] to aux, C =
+// gelu(pre); 2 C = v gelu'(aux) (aux may be C's own place); 3 split-K: block z
+// adds the partial product over k in [z kchunk, (z+1) kchunk) to C atomically (C
+// cleared beforehand; the weight gradients, whose K is the batch).
+// One training step of 16384 samples at 8x8 (45 GFLOP): 64 x 64 tiles with
+// 4 x 4 outputs a thread took 2.1 ms of products, and the bias gradients, two CTAs
+// walking the batch row by row, 1.2 ms; an epoch of one step 3.8 -> 1.4 ms.
+enum { MM_PLAIN = 0, MM_GELU = 1, MM_GELU_BACK = 2, MM_SPLIT = 3 };
+template <bool AK, bool BK, int EPI>
+__global__ void __launch_bounds__(sg::NTHR, 2)
+    k_mm(int M, int N, int K, const float* __restrict__ A, int lda, const float* __restrict__ Bm, int ldb,
+         const float* __restrict__ bias, float* C, int ldc, float* aux, int kchunk) {
+  __shared__ sg::Smem sm;
+  const int m0 = blockIdx.y * sg::BM, n0 = blockIdx.x * sg::BN;
+  const int kb = EPI == MM_SPLIT ? blockIdx.z * kchunk : 0;
+  const int ke = EPI == MM_SPLIT ? min(K, kb + kchunk) : K;
+  float2 acc[8][4];
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) acc[i][j] = make_float2(0.f, 0.f);
+  sg::tile<AK, BK>(A, lda, Bm, ldb, M, N, kb, ke, m0, n0, sm, acc);
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int m = m0 + sg::row_of(i);
+    if (m >= M) continue;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int n = n0 + sg::col_of(j);     // N, ldc even: pairs never straddle the edge
+      if (n >= N) continue;
+      float2 v = acc[i][j];
+      const size_t o = (size_t)m * ldc + n;
+      if (EPI == MM_SPLIT) {
+        atomicAdd(&C[o], v.x);
+        atomicAdd(&C[o + 1], v.y);
+        continue;
+      }
+      if (EPI != MM_GELU_BACK && bias) { v.x += bias[n]; v.y += bias[n + 1]; }
+      if (EPI == MM_GELU) {
+        aux[o] = v.x;        // scalar: the caller's buffers may be 4-byte aligned
+        aux[o + 1] = v.y;
+        v = make_float2(gelu_f(v.x), gelu_f(v.y));
+      }
+      if (EPI == MM_GELU_BACK) {
+        v = make_float2(v.x * gelu_df(aux[o]), v.y * gelu_df(aux[o + 1]));
+      }
+      C[o] = v.x;
+      C[o + 1] = v.y;
     }
-    for (int idx = threadIdx.x; idx < T * TKk; idx += 256) {
-      int c, kk;
-      if (tb) { c = idx / TKk; kk = idx - c * TKk; } else { kk = idx / T; c = idx - kk * T; }
-      const int gn = n0 + c, gk = k0 + kk;
-      Bs[kk][c] = (gn < N && gk < ke) ? (tb ? Bm[(size_t)gn * ldb + gk] : Bm[(size_t)gk * ldb + gn]) : 0.f;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int kk = 0; kk < TKk; ++kk) {
-      float a[4], b[4];
-#pragma unroll
-      for (int q = 0; q < 4; ++q) { a[q] = As[kk][ty * 4 + q]; b[q] = Bs[kk][tx * 4 + q]; }
-#pragma unroll
-      for (int q = 0; q < 4; ++q)
-#pragma unroll
-        for (int r = 0; r < 4; ++r) acc[q][r] = fmaf(a[q], b[r], acc[q][r]);
-    }
-    __syncthreads();
   }
-#pragma unroll
-  for (int q = 0; q < 4; ++q)
-#pragma unroll
-    for (int r = 0; r < 4; ++r) {
-      const int gm = m0 + ty * 4 + q, gn = n0 + tx * 4 + r;
-      if (gm >= M || gn >= N) continue;
-      float v = acc[q][r] + (bias ? bias[gn] : 0.f);
-      const size_t o = (size_t)gm * ldc + gn;
-      if (EPI == 1) { aux[o] = v; C[o] = gelu_f(v); }
-      else if (EPI == 2) C[o] += v;
-      else if (EPI == 3) atomicAdd(&C[o], v);
-      else C[o] = v;
-    }
 }
 
 // Masked softmax cross entropy.  Targets: hop weights w_h >= 0 (heat-bath
@@ -490,18 +487,35 @@ __global__ void k_prop_loss(int R, Lat L, const uint64_t* __restrict__ occ, cons
   }
 }
 
-// dZ = dH * gelu'(pre)
-__global__ void k_gelu_back(int64_t n, const float* __restrict__ pre, float* __restrict__ d) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) d[i] *= gelu_df(pre[i]);
+// column sums (bias gradients) of D (M, N): block (x, y) sums the y-th of
+// gridDim.y row ranges of 32 columns into part[y][n], k_colsum_fin the ranges
+__global__ void __launch_bounds__(256) k_colsum(int M, int N, const float* __restrict__ D, int ldd,
+                                                float* __restrict__ part) {
+  __shared__ float s[8][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int n = blockIdx.x * 32 + lane;
+  const int per = (M + gridDim.y - 1) / gridDim.y;
+  const int m1 = min(M, (int)(blockIdx.y + 1) * per);
+  float acc = 0.f;
+  if (n < N) {
+#pragma unroll 8
+    for (int m = blockIdx.y * per + warp; m < m1; m += 8) acc += D[(size_t)m * ldd + n];
+  }
+  s[warp][lane] = acc;
+  __syncthreads();
+  if (warp == 0 && n < N) {
+    float t = 0.f;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) t += s[w][lane];
+    part[(size_t)blockIdx.y * N + n] = t;
+  }
 }
-// column sums (bias gradients): out[n] = sum_m D[m][n]
-__global__ void k_colsum(int M, int N, const float* __restrict__ D, int ldd, float* __restrict__ out) {
+__global__ void k_colsum_fin(int N, int parts, const float* __restrict__ part, float* __restrict__ out) {
   const int n = blockIdx.x * blockDim.x + threadIdx.x;
   if (n >= N) return;
-  float s = 0.f;
-  for (int m = 0; m < M; ++m) s += D[(size_t)m * ldd + n];
-  out[n] = s;
+  float t = 0.f;
+  for (int y = 0; y < parts; ++y) t += part[(size_t)y * N + n];
+  out[n] = t;
 }
 // Adam (bias-corrected) on a flat parameter vector
 __global__ void k_adam(int64_t n, float* __restrict__ p, const float* __restrict__ g, float* __restrict__ m1,
@@ -707,33 +721,43 @@ int vmc_prop_train_step(int n_sites, const int32_t* edges, int n_edges, const ui
   float* H2 = Z2 + (size_t)R * PH;
   float* LG = H2 + (size_t)R * PH;      // R x 256 logits
   float* DL = LG + (size_t)R * PLOG;    // R x 256 dlogits
-  auto grid = [](int M, int N) { return dim3((unsigned)((N + 63) / 64), (unsigned)((M + 63) / 64)); };
-  // weight gradients: K = R (the batch), split in chunks of 256 rows so that
-  // the 512 x 512 products fill the GPU; the partial sums land atomically in
-  // the cleared gradient vector
-  const int kc = 256;
-  const unsigned nz = (unsigned)((R + kc - 1) / kc);
-  auto gridk = [nz](int M, int N) { return dim3((unsigned)((N + 63) / 64), (unsigned)((M + 63) / 64), nz); };
+  auto tiles = [](int v) { return (unsigned)((v + sg::BM - 1) / sg::BM); };
+  // weight gradients: K = R (the batch), split so that the few tiles of a
+  // 512-wide product make about four CTAs per SM; the partial sums land
+  // atomically in the cleared gradient vector
+  auto wgrad = [&](int M, int N, const float* A, int lda, const float* Bm, int ldb, float* C) {
+    const int t = (int)(tiles(M) * tiles(N));
+    int kc = (int)((((int64_t)R * t + 607) / 608 + 15) / 16 * 16);
+    kc = kc < 64 ? 64 : kc;
+    k_mm<false, false, MM_SPLIT><<<dim3(tiles(N), tiles(M), (unsigned)((R + kc - 1) / kc)), sg::NTHR, 0, st>>>(
+        M, N, R, A, lda, Bm, ldb, nullptr, C, N, nullptr, kc);
+  };
+  // bias gradients, with the logits (no longer needed) as scratch: parts * 512 <= 256 R
+  const int parts = R / 64 < 1 ? 1 : (R / 64 > 32 ? 32 : R / 64);
+  auto bgrad = [&](int N, const float* D, float* out) {
+    float* p = parts == 1 ? out : LG;
+    k_colsum<<<dim3((unsigned)((N + 31) / 32), (unsigned)parts), 256, 0, st>>>(R, N, D, N, p);
+    if (parts > 1) k_colsum_fin<<<(unsigned)((N + 255) / 256), 256, 0, st>>>(N, parts, p, out);
+  };
   if (cudaMemsetAsync(grad, 0, (size_t)np * sizeof(float), st) != cudaSuccess) return VMC_ERR_CUDA;
   // forward
-  k_sgemm<1><<<grid(R, PH), 256, 0, st>>>(0, 1, R, PH, Kin, Xf, Kin, W1, Kin, b1, H1, PH, Z1, 0);
-  k_sgemm<1><<<grid(R, PH), 256, 0, st>>>(0, 1, R, PH, PH, H1, PH, W2, PH, b2, H2, PH, Z2, 0);
-  k_sgemm<0><<<grid(R, PLOG), 256, 0, st>>>(0, 1, R, PLOG, PH, H2, PH, Wo, PH, bo, LG, PLOG, nullptr, 0);
+  const dim3 gh(tiles(PH), tiles(R)), gl(tiles(PLOG), tiles(R));
+  k_mm<true, true, MM_GELU><<<gh, sg::NTHR, 0, st>>>(R, PH, Kin, Xf, Kin, W1, Kin, b1, H1, PH, Z1, 0);
+  k_mm<true, true, MM_GELU><<<gh, sg::NTHR, 0, st>>>(R, PH, PH, H1, PH, W2, PH, b2, H2, PH, Z2, 0);
+  k_mm<true, true, MM_PLAIN><<<gl, sg::NTHR, 0, st>>>(R, PLOG, PH, H2, PH, Wo, PH, bo, LG, PLOG, nullptr, 0);
   Lat L{edges, n_edges, n_sites};
   k_prop_loss<<<(unsigned)((R * 32 + 255) / 256), 256, 0, st>>>(R, L, occ, LG, tgt, ktgt, kweight, DL, loss);
   // backward
-  k_sgemm<3><<<gridk(PLOG, PH), 256, 0, st>>>(1, 0, PLOG, PH, R, DL, PLOG, H2, PH, nullptr, gWo, PH, nullptr, kc);
-  k_colsum<<<(PLOG + 255) / 256, 256, 0, st>>>(R, PLOG, DL, PLOG, gbo);
-  // dH2 = DL Wo -> stored in H2 (H2 no longer needed), then * gelu'(Z2)
-  k_sgemm<0><<<grid(R, PH), 256, 0, st>>>(0, 0, R, PH, PLOG, DL, PLOG, Wo, PH, nullptr, H2, PH, nullptr, 0);
-  k_gelu_back<<<(unsigned)(((int64_t)R * PH + 255) / 256), 256, 0, st>>>((int64_t)R * PH, Z2, H2);
-  k_sgemm<3><<<gridk(PH, PH), 256, 0, st>>>(1, 0, PH, PH, R, H2, PH, H1, PH, nullptr, gW2, PH, nullptr, kc);
-  k_colsum<<<(PH + 255) / 256, 256, 0, st>>>(R, PH, H2, PH, gb2);
-  // dH1 = dZ2 W2 -> Z2 buffer, * gelu'(Z1)
-  k_sgemm<0><<<grid(R, PH), 256, 0, st>>>(0, 0, R, PH, PH, H2, PH, W2, PH, nullptr, Z2, PH, nullptr, 0);
-  k_gelu_back<<<(unsigned)(((int64_t)R * PH + 255) / 256), 256, 0, st>>>((int64_t)R * PH, Z1, Z2);
-  k_sgemm<3><<<gridk(PH, Kin), 256, 0, st>>>(1, 0, PH, Kin, R, Z2, PH, Xf, Kin, nullptr, gW1, Kin, nullptr, kc);
-  k_colsum<<<(PH + 255) / 256, 256, 0, st>>>(R, PH, Z2, PH, gb1);
+  wgrad(PLOG, PH, DL, PLOG, H2, PH, gWo);
+  bgrad(PLOG, DL, gbo);
+  // dZ2 = (DL Wo) gelu'(Z2) in H2's place (no longer needed)
+  k_mm<true, false, MM_GELU_BACK><<<gh, sg::NTHR, 0, st>>>(R, PH, PLOG, DL, PLOG, Wo, PH, nullptr, H2, PH, Z2, 0);
+  wgrad(PH, PH, H2, PH, H1, PH, gW2);
+  bgrad(PH, H2, gb2);
+  // dZ1 = (dZ2 W2) gelu'(Z1) in Z2's place
+  k_mm<true, false, MM_GELU_BACK><<<gh, sg::NTHR, 0, st>>>(R, PH, PH, H2, PH, W2, PH, nullptr, Z2, PH, Z1, 0);
+  wgrad(PH, Kin, Z2, PH, Xf, Kin, gW1);
+  bgrad(PH, Z2, gb1);
   // Adam
   const float c1 = 1.0f - powf(beta1, (float)t), c2 = 1.0f - powf(beta2, (float)t);
   k_adam<<<(unsigned)((np + 255) / 256), 256, 0, st>>>(np, params, grad, m1, m2, lr, beta1, beta2, eps, c1, c2);
