@@ -356,6 +356,39 @@ __device__ __forceinline__ void chi_item(int64_t item, const int32_t* cfg_idx, c
   else { ci = item >> 1; side = (int)(item & 1); }
 }
 
+// Where the side states of a launch live.  Plain (rows == 0): slot's state at
+// buf + slot * NS.  Cached (rows > 0, schedules that truncate after the last
+// row only): the state after every row a of a slot, in two buffers, at
+// ((slot * rows + a) * 2 + which); bit a of mask[slot] names the buffer that
+// holds the walker's current state, the other takes a proposal's.  A proposal
+// that changes row a0 of a side starts from the current state after row a0 - 1
+// and, on acceptance, becomes current by flipping the bits from a0 on: no
+// state is copied and no row above a move is absorbed again.
+template <typename T>
+struct ChiStates {
+  T* buf;
+  int* ex;
+  const uint32_t* mask;   // nullptr: buffer 0
+  int rows;
+  int fresh;              // 1: the buffer that is not current
+  __device__ __forceinline__ int64_t at(int64_t slot, int a, int other) const {
+    return ((slot * rows + a) * 2 + (((mask ? (mask[slot] >> a) & 1u : 0u)) ^ (unsigned)other));
+  }
+  // index (in states) of the slot's last state
+  __device__ __forceinline__ int64_t last(int64_t slot) const { return rows ? at(slot, rows - 1, fresh) : slot; }
+};
+
+// Rows of a side that a change of sites i and j leaves as they are (from the
+// lattice's edge inwards); rows: the side's.
+__device__ __forceinline__ int rows_kept(int i, int j, int side, int Lx, int Ly, int rows) {
+  int k = rows;
+  for (int q = 0; q < 2; ++q) {
+    const int r = (q ? j : i) / Ly, a = side ? Lx - 1 - r : r;
+    if (a < k) k = a;      // a row of the other side has a >= rows
+  }
+  return k;
+}
+
 // Electron parity of the first n_rows rows of a side.
 __device__ __forceinline__ int side_parity(uint64_t up, uint64_t dn, int Lx, int Ly, int side, int n_rows) {
   const int r0 = side ? Lx - n_rows : 0;
@@ -508,6 +541,44 @@ __device__ void column_adjoint(T* Wb, int NS, int stride, int par, int px, const
   }
 }
 
+// Row a of a side absorbed into W[h][idx] (whole CTA) and the state rescaled
+// by a power of two, its exponent to e2.  Returns 0, 1 (the state vanishes) or
+// 2 (not finite).  par: electron parity absorbed so far.
+template <typename T, int D>
+__device__ int absorb_row(const T* __restrict__ tens, const ChiSched& sc, uint64_t up, uint64_t dn, int side, int a,
+                          T* W, T* A2, T* red, int& par, int& e2) {
+  constexpr int H = D * D / 2;  // non-zero entries of a group
+  const int NS = sc.NS, Ly = sc.Ly;
+  const int r = side ? (sc.Lx - 1 - a) : a;
+  // the row's signed tensors, all columns at once (one global-load latency per row)
+  __syncthreads();
+  load_row_tables<T, D>(tens, up, dn, r, Ly, side, A2);
+  int stride = NS / D;
+  for (int c = 0; c < Ly; ++c, stride /= D) {
+    const int x = site_state(up, dn, r * Ly + c);
+    const int px = (x ^ (x >> 1)) & 1;
+    __syncthreads();
+    column_forward<T, D>(W, NS, stride, par, px, A2 + c * 2 * H * H);
+    par ^= px;
+  }
+  __syncthreads();
+  // rescale the state (the h != 0 slices are zero after the open right edge)
+  T m = T(0);
+  int nonfinite = 0;
+  for (int e = threadIdx.x; e < NS; e += blockDim.x) {
+    const T v = fabs(W[e]);
+    nonfinite |= !(v < T(INFINITY));
+    m = fmax(m, v);
+  }
+  if (__syncthreads_or(nonfinite)) return 2;
+  m = cta_absmax<T>(m, red);
+  if (m == T(0)) return 1;
+  e2 = (int)ilogb(m);
+  __syncthreads();
+  for (int e = threadIdx.x; e < NS; e += blockDim.x) W[e] = scalbn(W[e], -e2);
+  return 0;
+}
+
 // Absorbs rows [a0, a1) of each item's side into its boundary state (slot
 // 2 ci + side of state / expo; a0 == 0 starts from the empty boundary).  One
 // CTA per item, W[h][idx] (D x NS) in shared memory.  Z2 structure: while a
@@ -550,34 +621,12 @@ __global__ void __launch_bounds__(CHI_NT)
   }
   int par = side_parity(up, dn, Lx, Ly, side, a0);
   for (int a = a0; a < a1 && !zero && !bad; ++a) {
-    const int r = side ? (Lx - 1 - a) : a;
-    // the row's signed tensors, all columns at once (one global-load latency per row)
-    __syncthreads();
-    load_row_tables<T, D>(tens, up, dn, r, Ly, side, A2);
-    int stride = NS / D;
-    for (int c = 0; c < Ly; ++c, stride /= D) {
-      const int x = site_state(up, dn, r * Ly + c);
-      const int px = (x ^ (x >> 1)) & 1;
-      __syncthreads();
-      column_forward<T, D>(W, NS, stride, par, px, A2 + c * 2 * H * H);
-      par ^= px;
-    }
-    __syncthreads();
-    // rescale the state (the h != 0 slices are zero after the open right edge)
-    T m = T(0);
-    int nonfinite = 0;
-    for (int e = threadIdx.x; e < NS; e += blockDim.x) {
-      const T v = fabs(W[e]);
-      nonfinite |= !(v < T(INFINITY));
-      m = fmax(m, v);
-    }
-    if (__syncthreads_or(nonfinite)) { bad = true; break; }
-    m = cta_absmax<T>(m, red);
-    if (m == T(0)) { zero = true; break; }
-    const int e2 = (int)ilogb(m);
+    int e2 = 0;
+    const int rc = absorb_row<T, D>(tens, sc, up, dn, side, a, W, A2, red, par, e2);
+    zero = rc == 1;
+    bad = rc == 2;
+    if (rc) break;
     expo += e2;
-    __syncthreads();
-    for (int e = threadIdx.x; e < NS; e += blockDim.x) W[e] = scalbn(W[e], -e2);
     if (keep) {
       __syncthreads();
       T* kp = keep + (slot * sc.rows + a) * (int64_t)NS;
@@ -588,6 +637,66 @@ __global__ void __launch_bounds__(CHI_NT)
   __syncthreads();
   for (int e = threadIdx.x; e < NS; e += blockDim.x) st[e] = (zero || bad) ? T(0) : W[e];
   if (threadIdx.x == 0) expo_io[slot] = bad ? CHI_EXP_BAD : (zero ? CHI_EXP_ZERO : expo);
+}
+
+// The same with cached states: rows [a0, rows) of each item's side, from the
+// current state after row a0 - 1 of the walker's slot (a0 == 0: the empty
+// boundary), every state from a0 on (keep_rows; else the last only) written to
+// the item's place in dst.  Items as in chi_item; what changed: a sweep's edge
+// (edge >= 0, ci the walker), or a hop term's (pairs given, ci the term, its
+// walker pairs[2 ci] - w0), or everything.
+template <typename T, int D>
+__global__ void __launch_bounds__(CHI_NT)
+    k_chi_absorb_from(const T* __restrict__ tens, ChiSched sc, const uint64_t* __restrict__ cfg,
+                      const int32_t* __restrict__ cfg_idx, const uint8_t* __restrict__ sides, int64_t n_items,
+                      const int* __restrict__ count, int edge, const int32_t* __restrict__ edges,
+                      const int32_t* __restrict__ pairs, int64_t w0, ChiStates<T> cur, ChiStates<T> dst,
+                      int keep_rows) {
+  constexpr int H = D * D / 2;
+  extern __shared__ __align__(16) unsigned char smraw[];
+  const int64_t item = blockIdx.x;
+  if (item >= n_items || (count && item >= *count)) return;
+  const int NS = sc.NS, rows = sc.rows;
+  T* W = reinterpret_cast<T*>(smraw);
+  T* A2 = W + (size_t)D * NS;
+  T* red = A2 + (size_t)sc.Ly * 2 * H * H;
+  int64_t ci;
+  int side;
+  chi_item(item, cfg_idx, sides, ci, side);
+  int64_t owner = ci;
+  if (pairs) {
+    owner = pairs[2 * ci] - w0;
+    edge = pairs[2 * ci + 1] >> 1;
+  }
+  const int a0 = edge < 0 ? 0 : rows_kept(edges[2 * edge], edges[2 * edge + 1], side, sc.Lx, sc.Ly, rows);
+  const int64_t slot = 2 * ci + side;
+  const uint64_t up = cfg[2 * ci], dn = cfg[2 * ci + 1];
+  int expo = 0;
+  int rc = 0;
+  if (a0 == 0) {
+    for (int e = threadIdx.x; e < D * NS; e += blockDim.x) W[e] = (e == 0) ? T(1) : T(0);
+  } else {
+    const int64_t src = cur.at(2 * owner + side, a0 - 1, 0);
+    expo = cur.ex[src];
+    rc = expo == CHI_EXP_ZERO ? 1 : (expo == CHI_EXP_BAD ? 2 : 0);
+    const T* st = cur.buf + src * NS;
+    for (int e = threadIdx.x; e < D * NS; e += blockDim.x) W[e] = (e < NS && !rc) ? st[e] : T(0);
+  }
+  int par = side_parity(up, dn, sc.Lx, sc.Ly, side, a0);
+  for (int a = a0; a < rows; ++a) {
+    if (!rc) {
+      int e2 = 0;
+      rc = absorb_row<T, D>(tens, sc, up, dn, side, a, W, A2, red, par, e2);
+      if (!rc) expo += e2;
+    }
+    if (keep_rows || a == rows - 1) {
+      const int64_t o = dst.at(slot, a, dst.fresh);
+      T* st = dst.buf + o * NS;
+      __syncthreads();
+      for (int e = threadIdx.x; e < NS; e += blockDim.x) st[e] = rc ? T(0) : W[e];
+      if (threadIdx.x == 0) dst.ex[o] = rc == 2 ? CHI_EXP_BAD : (rc == 1 ? CHI_EXP_ZERO : expo);
+    }
+  }
 }
 
 constexpr int CHI_TRUNC_ITEMS = 2;  // items per CTA, two warps (one per parity block) each
@@ -608,7 +717,7 @@ template <typename T, int D, bool ONE_SIDED>
 __global__ void __launch_bounds__(32 * 2 * CHI_TRUNC_ITEMS)
     k_chi_trunc(ChiSched sc, int k, int n_rows, const uint64_t* __restrict__ cfg,
                 const int32_t* __restrict__ cfg_idx, const uint8_t* __restrict__ sides, int64_t n_items,
-                const int* __restrict__ count, T* __restrict__ state, const int* __restrict__ expo_io) {
+                const int* __restrict__ count, ChiStates<T> states) {
   extern __shared__ __align__(16) unsigned char smraw[];
   const int warp = threadIdx.x >> 5, ln = threadIdx.x & 31;
   const int il = warp >> 1, b = warp & 1;
@@ -633,9 +742,10 @@ __global__ void __launch_bounds__(32 * 2 * CHI_TRUNC_ITEMS)
   T* st = nullptr;
   if (live) {
     chi_item(item, cfg_idx, sides, ci, side);
-    const int ex = expo_io[2 * ci + side];
+    const int64_t o = states.last(2 * ci + side);
+    const int ex = states.ex[o];
     on = ex != CHI_EXP_ZERO && ex != CHI_EXP_BAD;
-    st = state + (2 * ci + side) * (int64_t)NS;
+    st = states.buf + o * NS;
     qcls = side_parity(cfg[2 * ci], cfg[2 * ci + 1], sc.Lx, sc.Ly, side, n_rows) ^ b;
   }
   const uint32_t pi = block_member<D>(b, ln);
@@ -713,24 +823,60 @@ __device__ __forceinline__ void chi_finish(double v, int et, int eb, uint64_t up
   }
 }
 
+// <a, b> by one warp.  FP32 states: an FP64 instruction costs a warp 64 clocks
+// on GB300 (two conversions and a multiply-add per element), so the products
+// are taken exactly as p + fma(a, b, -p) and summed in three FP32 words with
+// TwoSum (~2^-70 of the largest partial sum, finer than the FP64 sum), joined
+// in FP64 at the end.
+__device__ __forceinline__ float dot_two_sum(float& s, float x) {
+  const float t = s + x, bb = t - s;
+  const float e = (s - (t - bb)) + (x - bb);
+  s = t;
+  return e;
+}
+__device__ __forceinline__ void dot_add(float a, float b, float& s, float& c, float& d) {
+  const float p = a * b;
+  const float q = fmaf(a, b, -p);
+  const float e = dot_two_sum(s, p);
+  d += dot_two_sum(c, e);
+  d += dot_two_sum(c, q);
+}
 template <typename T>
-__device__ __forceinline__ double warp_dot(const T* a, const T* b, int NS) {
+__device__ __forceinline__ double warp_dot(const T* __restrict__ a, const T* __restrict__ b, int NS) {
+  const int ln = threadIdx.x & 31;
   double acc = 0.0;
-  for (int e = threadIdx.x & 31; e < NS; e += 32) acc += (double)a[e] * (double)b[e];
+  if constexpr (std::is_same<T, float>::value) {
+    float s = 0.f, c = 0.f, d = 0.f;
+    if ((NS & 127) == 0) {     // states start at multiples of NS elements of an aligned workspace
+#pragma unroll 4
+      for (int e = ln * 4; e < NS; e += 128) {
+        const float4 x = *reinterpret_cast<const float4*>(a + e), y = *reinterpret_cast<const float4*>(b + e);
+        dot_add(x.x, y.x, s, c, d);
+        dot_add(x.y, y.y, s, c, d);
+        dot_add(x.z, y.z, s, c, d);
+        dot_add(x.w, y.w, s, c, d);
+      }
+    } else {
+      for (int e = ln; e < NS; e += 32) dot_add(a[e], b[e], s, c, d);
+    }
+    acc = (double)s + ((double)c + (double)d);
+  } else {
+    for (int e = ln; e < NS; e += 32) acc += (double)a[e] * (double)b[e];
+  }
   return warp_sum(acc);
 }
 
-// One warp per configuration: states at st[(2w) * NS] (top), st[(2w+1) * NS].
+// One warp per configuration: top and bottom states of slots 2w and 2w + 1.
 template <typename T>
-__global__ void k_chi_dot(const T* __restrict__ st, const int* __restrict__ ex, int NS,
-                          const uint64_t* __restrict__ occ, int64_t R, double* __restrict__ sign,
-                          double* __restrict__ logabs) {
+__global__ void k_chi_dot(ChiStates<T> st, int NS, const uint64_t* __restrict__ occ, int64_t R,
+                          double* __restrict__ sign, double* __restrict__ logabs) {
   const int64_t w = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (w >= R) return;
-  const double v = warp_dot(st + 2 * w * NS, st + (2 * w + 1) * NS, NS);
+  const int64_t t = st.last(2 * w), b = st.last(2 * w + 1);
+  const double v = warp_dot(st.buf + t * NS, st.buf + b * NS, NS);
   if ((threadIdx.x & 31) == 0) {
     double s, la;
-    chi_finish(v, ex[2 * w], ex[2 * w + 1], occ[2 * w], occ[2 * w + 1], s, la);
+    chi_finish(v, st.ex[t], st.ex[b], occ[2 * w], occ[2 * w + 1], s, la);
     sign[w] = s;
     logabs[w] = la;
   }
@@ -809,10 +955,12 @@ __global__ void k_chi_propose(const uint64_t* __restrict__ occ, int64_t n, int64
 
 // Metropolis decision for every walker with a proposal: amplitude from the
 // rebuilt sides (new) and the kept ones (cur); on acceptance the new states
-// replace the current ones.  One warp per walker.
+// replace the current ones (copied; with cached states the buffers' bits flip
+// from the first changed row of each touched side on).  One warp per walker.
 template <typename T>
-__global__ void k_chi_accept(int NS, int64_t n, T* __restrict__ cur, int* __restrict__ cur_ex,
-                             const T* __restrict__ nw, const int* __restrict__ nw_ex, const uint8_t* __restrict__ flags,
+__global__ void k_chi_accept(int NS, int64_t n, ChiStates<T> cur, ChiStates<T> nw, uint32_t* __restrict__ mask,
+                             const int32_t* __restrict__ edges, int edge, int Lx, int Ly,
+                             const uint8_t* __restrict__ flags,
                              const uint64_t* __restrict__ prop, const float* __restrict__ u_acc,
                              uint64_t* __restrict__ occ, double* __restrict__ sign, double* __restrict__ logabs,
                              int32_t* __restrict__ n_acc, unsigned long long* __restrict__ n_eval) {
@@ -823,10 +971,10 @@ __global__ void k_chi_accept(int NS, int64_t n, T* __restrict__ cur, int* __rest
   const int ln = threadIdx.x & 31;
   const int f = (w < n) ? flags[w] : 0;
   if (f) {
-    const T* a = ((f & 1) ? nw : cur) + 2 * w * NS;
-    const T* b = ((f & 2) ? nw : cur) + (2 * w + 1) * NS;
-    const int et = ((f & 1) ? nw_ex : cur_ex)[2 * w], eb = ((f & 2) ? nw_ex : cur_ex)[2 * w + 1];
-    const double v = warp_dot(a, b, NS);
+    const int64_t ot = (f & 1) ? nw.last(2 * w) : cur.last(2 * w);
+    const int64_t ob = (f & 2) ? nw.last(2 * w + 1) : cur.last(2 * w + 1);
+    const int et = ((f & 1) ? nw.ex : cur.ex)[ot], eb = ((f & 2) ? nw.ex : cur.ex)[ob];
+    const double v = warp_dot(((f & 1) ? nw.buf : cur.buf) + ot * NS, ((f & 2) ? nw.buf : cur.buf) + ob * NS, NS);
     int acc = 0;
     double s1 = 0.0, la1 = 0.0;
     if (ln == 0) {
@@ -842,9 +990,14 @@ __global__ void k_chi_accept(int NS, int64_t n, T* __restrict__ cur, int* __rest
     if (acc) {
       for (int sd = 0; sd < 2; ++sd)
         if (f & (1 << sd)) {
-          const int64_t o = (2 * w + sd) * NS;
-          for (int e2 = ln; e2 < NS; e2 += 32) cur[o + e2] = nw[o + e2];
-          if (ln == 0) cur_ex[2 * w + sd] = nw_ex[2 * w + sd];
+          if (mask) {
+            const int kept = rows_kept(edges[2 * edge], edges[2 * edge + 1], sd, Lx, Ly, cur.rows);
+            if (ln == 0) mask[2 * w + sd] ^= ((1u << cur.rows) - 1u) & ~((1u << kept) - 1u);
+          } else {
+            const int64_t o = (2 * w + sd) * NS;
+            for (int e2 = ln; e2 < NS; e2 += 32) cur.buf[o + e2] = nw.buf[o + e2];
+            if (ln == 0) cur.ex[2 * w + sd] = nw.ex[2 * w + sd];
+          }
         }
       if (ln == 0) {
         occ[2 * w] = prop[2 * w];
@@ -900,19 +1053,18 @@ __global__ void k_chi_term_prep(const uint64_t* __restrict__ occ, int N, int Ly,
 template <typename T>
 __global__ void k_chi_terms(int NS, int N, const uint64_t* __restrict__ occ, const int32_t* __restrict__ pairs,
                             int64_t p0, int64_t np, int64_t w0, const int32_t* __restrict__ edges, double t,
-                            const T* __restrict__ cur, const int* __restrict__ cur_ex, const double* __restrict__ s0a,
-                            const double* __restrict__ la0a, const T* __restrict__ nw, const int* __restrict__ nw_ex,
-                            const uint8_t* __restrict__ flags, const uint64_t* __restrict__ prop,
+                            ChiStates<T> cur, const double* __restrict__ s0a, const double* __restrict__ la0a,
+                            ChiStates<T> nw, const uint8_t* __restrict__ flags, const uint64_t* __restrict__ prop,
                             double* __restrict__ term) {
   const int64_t p = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (p >= np) return;
   const int w = pairs[2 * (p0 + p)], tm = pairs[2 * (p0 + p) + 1];
   const int64_t lw = w - w0;
   const int f = flags[p];
-  const T* a = (f & 1) ? nw + 2 * p * NS : cur + 2 * lw * NS;
-  const T* b = (f & 2) ? nw + (2 * p + 1) * NS : cur + (2 * lw + 1) * NS;
-  const int et = (f & 1) ? nw_ex[2 * p] : cur_ex[2 * lw], eb = (f & 2) ? nw_ex[2 * p + 1] : cur_ex[2 * lw + 1];
-  const double v = warp_dot(a, b, NS);
+  const int64_t ot = (f & 1) ? nw.last(2 * p) : cur.last(2 * lw);
+  const int64_t ob = (f & 2) ? nw.last(2 * p + 1) : cur.last(2 * lw + 1);
+  const int et = ((f & 1) ? nw.ex : cur.ex)[ot], eb = ((f & 2) ? nw.ex : cur.ex)[ob];
+  const double v = warp_dot(((f & 1) ? nw.buf : cur.buf) + ot * NS, ((f & 2) ? nw.buf : cur.buf) + ob * NS, NS);
   if ((threadIdx.x & 31) == 0) {
     const uint64_t up = occ[2 * (int64_t)w], dn = occ[2 * (int64_t)w + 1];
     const int e = tm >> 1, sp = (tm & 1) ? 0 : 1;
@@ -1240,6 +1392,7 @@ int build_sides_d(const void* tens, const ChiSched& sc, const uint64_t* cfg, con
       cudaFuncSetAttribute(k_chi_trunc<T, D, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tsm) !=
           cudaSuccess)
     return VMC_ERR_CUDA;
+  const ChiStates<T> plain{state, ex, nullptr, 0, 0};
   int a = 0;
   while (a < sc.rows) {
     int a1 = a + 1;
@@ -1255,16 +1408,72 @@ int build_sides_d(const void* tens, const ChiSched& sc, const uint64_t* cfg, con
         const unsigned grid = (unsigned)((n_items + CHI_TRUNC_ITEMS - 1) / CHI_TRUNC_ITEMS);
         if ((sc.NS / n) / 2 <= 32)
           k_chi_trunc<T, D, true><<<grid, 64 * CHI_TRUNC_ITEMS, tsm, st>>>(sc, k, a1, cfg, cfg_idx, sides, n_items,
-                                                                            count, state, ex);
+                                                                            count, plain);
         else
           k_chi_trunc<T, D, false><<<grid, 64 * CHI_TRUNC_ITEMS, tsm, st>>>(sc, k, a1, cfg, cfg_idx, sides, n_items,
-                                                                             count, state, ex);
+                                                                             count, plain);
         VMC_CUDA_CHECK_LAUNCH();
       }
     a = a1;
   }
   return VMC_OK;
 }
+
+// Schedules whose states can be cached row by row: truncation after the last
+// row only.
+bool chi_cacheable(const ChiSched& sc) {
+  for (int a = 0; a + 1 < sc.rows; ++a)
+    if (sc.cuts[a]) return false;
+  return sc.rows < 32;
+}
+
+// Side states with cached rows (k_chi_absorb_from), then the cuts after the
+// last row.  Where items start: see k_chi_absorb_from.
+struct ChiFrom { int edge = -1; const int32_t* edges = nullptr; const int32_t* pairs = nullptr; int64_t w0 = 0; };
+
+template <typename T, int D>
+int build_sides_from_d(const void* tens, const ChiSched& sc, const uint64_t* cfg, const int32_t* cfg_idx,
+                       const uint8_t* sides, int64_t n_items, const int* count, const ChiFrom& f,
+                       const ChiStates<T>& cur, const ChiStates<T>& dst, bool keep_rows, cudaStream_t st) {
+  const size_t smem = ChiSmem<T>::bytes(sc.NS, D, sc.Ly), tsm = ChiTruncSmem<T>::bytes();
+  if (cudaFuncSetAttribute(k_chi_absorb_from<T, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
+          cudaSuccess ||
+      cudaFuncSetAttribute(k_chi_trunc<T, D, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tsm) !=
+          cudaSuccess ||
+      cudaFuncSetAttribute(k_chi_trunc<T, D, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tsm) !=
+          cudaSuccess)
+    return VMC_ERR_CUDA;
+  k_chi_absorb_from<T, D><<<(unsigned)n_items, CHI_NT, smem, st>>>((const T*)tens, sc, cfg, cfg_idx, sides, n_items,
+                                                                   count, f.edge, f.edges, f.pairs, f.w0, cur, dst,
+                                                                   keep_rows ? 1 : 0);
+  VMC_CUDA_CHECK_LAUNCH();
+  for (int k = sc.Ly - 1; k >= 1; --k)
+    if ((sc.cuts[sc.rows - 1] >> k) & 1u) {
+      int nL = 1;
+      for (int i = 0; i < k; ++i) nL *= D;
+      const int n = nL <= sc.NS / nL ? nL : sc.NS / nL;
+      const unsigned grid = (unsigned)((n_items + CHI_TRUNC_ITEMS - 1) / CHI_TRUNC_ITEMS);
+      if ((sc.NS / n) / 2 <= 32)
+        k_chi_trunc<T, D, true><<<grid, 64 * CHI_TRUNC_ITEMS, tsm, st>>>(sc, k, sc.rows, cfg, cfg_idx, sides, n_items,
+                                                                          count, dst);
+      else
+        k_chi_trunc<T, D, false><<<grid, 64 * CHI_TRUNC_ITEMS, tsm, st>>>(sc, k, sc.rows, cfg, cfg_idx, sides,
+                                                                           n_items, count, dst);
+      VMC_CUDA_CHECK_LAUNCH();
+    }
+  return VMC_OK;
+}
+
+template <typename T>
+int launch_chi_from(const void* tens, const ChiSched& sc, const uint64_t* cfg, const int32_t* cfg_idx,
+                    const uint8_t* sides, int64_t n_items, const int* count, const ChiFrom& f, const ChiStates<T>& cur,
+                    const ChiStates<T>& dst, bool keep_rows, cudaStream_t st) {
+  if (n_items <= 0) return VMC_OK;
+  return sc.D == 4
+             ? build_sides_from_d<T, 4>(tens, sc, cfg, cfg_idx, sides, n_items, count, f, cur, dst, keep_rows, st)
+             : build_sides_from_d<T, 2>(tens, sc, cfg, cfg_idx, sides, n_items, count, f, cur, dst, keep_rows, st);
+}
+
 
 // Boundary states of n_items (configuration, side) items into slots
 // 2 ci + side of state / ex: the rows of the schedule absorbed in runs that
@@ -1279,42 +1488,63 @@ int launch_chi_side(const void* tens, const ChiSched& sc, const uint64_t* cfg, c
 
 
 // Per-chunk workspace (work_rows walkers): current and new side states, their
-// exponents, proposed configurations, item lists.
+// exponents (cached: both buffers of every row, and the buffers' bits), proposed
+// configurations, item lists.
 template <typename T>
 struct ChiWork {
-  T* cur; T* nw; int* cur_ex; int* nw_ex; uint64_t* prop; int32_t* cfg_idx; uint8_t* sides; uint8_t* flags;
+  ChiStates<T> cur, nw;
+  uint32_t* mask;
+  uint64_t* prop; int32_t* cfg_idx; uint8_t* sides; uint8_t* flags;
   float* u_acc; int* count; double* s0; double* la0;
-  static int64_t bytes(int NS, int64_t rows) {
-    return rows * (4 * (int64_t)NS * (int64_t)sizeof(T) + 4 * 4 + 16 + 8 + 2 + 1 + 4 + 16) + 16 * 256;
+  int64_t cap;     // walkers (or hop terms) the workspace holds
+  static int64_t states(const ChiSched& sc) { return chi_cacheable(sc) ? 4 * sc.rows : 4; }   // per walker
+  static int64_t bytes(const ChiSched& sc, int64_t rows) {
+    const int64_t n = states(sc);
+    return rows * (n * sc.NS * (int64_t)sizeof(T) + n * 4 + 8 + 16 + 8 + 2 + 1 + 4 + 16) + 16 * 256;
   }
-  ChiWork(void* base, int NS, int64_t rows) {
+  ChiWork(void* base, const ChiSched& sc, int64_t rows) {
     char* p = (char*)base;
     auto take = [&](int64_t nbytes) { char* q = p; p += (nbytes + 255) & ~int64_t(255); return q; };
-    cur = (T*)take(2 * rows * NS * (int64_t)sizeof(T));
-    nw = (T*)take(2 * rows * NS * (int64_t)sizeof(T));
+    const bool cached = chi_cacheable(sc);
+    const int64_t n = states(sc) * rows;
+    cap = rows;
+    T* buf = (T*)take(n * sc.NS * (int64_t)sizeof(T));
     prop = (uint64_t*)take(2 * rows * 8);
     s0 = (double*)take(rows * 8);
     la0 = (double*)take(rows * 8);
-    cur_ex = (int*)take(2 * rows * 4);
-    nw_ex = (int*)take(2 * rows * 4);
+    int* ex = (int*)take(n * 4);
+    mask = (uint32_t*)take(2 * rows * 4);
     cfg_idx = (int32_t*)take(2 * rows * 4);
     u_acc = (float*)take(rows * 4);
     count = (int*)take(256);
     sides = (uint8_t*)take(2 * rows);
     flags = (uint8_t*)take(rows);
+    if (cached) {
+      cur = ChiStates<T>{buf, ex, mask, sc.rows, 0};
+      nw = ChiStates<T>{buf, ex, mask, sc.rows, 1};
+    } else {
+      cur = ChiStates<T>{buf, ex, nullptr, 0, 0};
+      nw = ChiStates<T>{buf + 2 * rows * sc.NS, ex + 2 * rows, nullptr, 0, 0};
+      mask = nullptr;
+    }
+  }
+  // current states of n walkers, built from scratch
+  int build(const void* tens, const ChiSched& sc, const uint64_t* cfg, int64_t n, cudaStream_t st) {
+    if (!mask) return launch_chi_side<T>(tens, sc, cfg, nullptr, nullptr, 2 * n, nullptr, cur.buf, cur.ex, st);
+    if (cudaMemsetAsync(mask, 0, 2 * cap * sizeof(uint32_t), st) != cudaSuccess) return VMC_ERR_CUDA;
+    return launch_chi_from<T>(tens, sc, cfg, nullptr, nullptr, 2 * n, nullptr, ChiFrom{}, cur, cur, true, st);
   }
 };
 
 template <typename T>
 int chi_eval(const void* tens, const ChiSched& sc, const uint64_t* occ, int64_t R, double* sign, double* logabs,
              void* work, int64_t work_rows, cudaStream_t st) {
-  ChiWork<T> W(work, sc.NS, work_rows);
+  ChiWork<T> W(work, sc, work_rows);
   for (int64_t w0 = 0; w0 < R; w0 += work_rows) {
     const int64_t n = (R - w0) < work_rows ? (R - w0) : work_rows;
-    int rc = launch_chi_side<T>(tens, sc, occ + 2 * w0, nullptr, nullptr, 2 * n, nullptr, W.cur, W.cur_ex, st);
+    int rc = W.build(tens, sc, occ + 2 * w0, n, st);
     if (rc) return rc;
-    k_chi_dot<T><<<(unsigned)((n + 7) / 8), 256, 0, st>>>(W.cur, W.cur_ex, sc.NS, occ + 2 * w0, n, sign + w0,
-                                                          logabs + w0);
+    k_chi_dot<T><<<(unsigned)((n + 7) / 8), 256, 0, st>>>(W.cur, sc.NS, occ + 2 * w0, n, sign + w0, logabs + w0);
     VMC_CUDA_CHECK_LAUNCH();
   }
   return VMC_OK;
@@ -1325,13 +1555,12 @@ int chi_sweep(const void* tens, const ChiSched& sc, uint64_t* occ, int64_t B, co
               int n_sweeps, float hopping_rate, uint64_t seed, uint64_t sweep_offset, const float* r_move,
               const uint8_t* r_bit, const float* r_acc, double* sign, double* logabs, int32_t* n_acc,
               unsigned long long* n_eval, void* work, int64_t work_rows, cudaStream_t st) {
-  ChiWork<T> W(work, sc.NS, work_rows);
+  ChiWork<T> W(work, sc, work_rows);
   for (int64_t w0 = 0; w0 < B; w0 += work_rows) {
     const int64_t n = (B - w0) < work_rows ? (B - w0) : work_rows;
-    int rc = launch_chi_side<T>(tens, sc, occ + 2 * w0, nullptr, nullptr, 2 * n, nullptr, W.cur, W.cur_ex, st);
+    int rc = W.build(tens, sc, occ + 2 * w0, n, st);
     if (rc) return rc;
-    k_chi_dot<T><<<(unsigned)((n + 7) / 8), 256, 0, st>>>(W.cur, W.cur_ex, sc.NS, occ + 2 * w0, n, sign + w0,
-                                                          logabs + w0);
+    k_chi_dot<T><<<(unsigned)((n + 7) / 8), 256, 0, st>>>(W.cur, sc.NS, occ + 2 * w0, n, sign + w0, logabs + w0);
     VMC_CUDA_CHECK_LAUNCH();
     for (int s = 0; s < n_sweeps; ++s)
       for (int e = 0; e < E; ++e) {
@@ -1340,10 +1569,17 @@ int chi_sweep(const void* tens, const ChiSched& sc, uint64_t* occ, int64_t B, co
             occ + 2 * w0, n, w0, B, sc.Ly, sc.rows, edges, e, E, s, hopping_rate, seed, sweep_offset, r_move, r_bit,
             r_acc, W.prop, W.flags, W.u_acc, W.cfg_idx, W.sides, W.count);
         VMC_CUDA_CHECK_LAUNCH();
-        rc = launch_chi_side<T>(tens, sc, W.prop, W.cfg_idx, W.sides, 2 * n, W.count, W.nw, W.nw_ex, st);
+        if (W.mask) {
+          ChiFrom f;
+          f.edge = e;
+          f.edges = edges;
+          rc = launch_chi_from<T>(tens, sc, W.prop, W.cfg_idx, W.sides, 2 * n, W.count, f, W.cur, W.nw, true, st);
+        } else {
+          rc = launch_chi_side<T>(tens, sc, W.prop, W.cfg_idx, W.sides, 2 * n, W.count, W.nw.buf, W.nw.ex, st);
+        }
         if (rc) return rc;
-        k_chi_accept<T><<<(unsigned)((n + 7) / 8), 256, 0, st>>>(sc.NS, n, W.cur, W.cur_ex, W.nw, W.nw_ex, W.flags,
-                                                                 W.prop, W.u_acc, occ + 2 * w0, sign + w0,
+        k_chi_accept<T><<<(unsigned)((n + 7) / 8), 256, 0, st>>>(sc.NS, n, W.cur, W.nw, W.mask, edges, e, sc.Lx, sc.Ly,
+                                                                 W.flags, W.prop, W.u_acc, occ + 2 * w0, sign + w0,
                                                                  logabs + w0, n_acc ? n_acc + w0 : nullptr, n_eval);
         VMC_CUDA_CHECK_LAUNCH();
       }
@@ -1356,13 +1592,13 @@ template <typename T>
 int chi_local_energy(const void* tens, const ChiSched& sc, const uint64_t* occ, int64_t B, const int32_t* edges,
                      double t, double U, const int32_t* pairs, const int32_t* offs, const int32_t* offs_host,
                      double* term, double* eloc, void* work, int64_t work_rows, cudaStream_t st) {
-  ChiWork<T> W(work, sc.NS, work_rows);
+  ChiWork<T> W(work, sc, work_rows);
   const int N = sc.Lx * sc.Ly;
   for (int64_t w0 = 0; w0 < B; w0 += work_rows) {
     const int64_t n = (B - w0) < work_rows ? (B - w0) : work_rows;
-    int rc = launch_chi_side<T>(tens, sc, occ + 2 * w0, nullptr, nullptr, 2 * n, nullptr, W.cur, W.cur_ex, st);
+    int rc = W.build(tens, sc, occ + 2 * w0, n, st);
     if (rc) return rc;
-    k_chi_dot<T><<<(unsigned)((n + 7) / 8), 256, 0, st>>>(W.cur, W.cur_ex, sc.NS, occ + 2 * w0, n, W.s0, W.la0);
+    k_chi_dot<T><<<(unsigned)((n + 7) / 8), 256, 0, st>>>(W.cur, sc.NS, occ + 2 * w0, n, W.s0, W.la0);
     VMC_CUDA_CHECK_LAUNCH();
     const int64_t pa = offs_host[w0], pb = offs_host[w0 + n];
     for (int64_t p0 = pa; p0 < pb; p0 += work_rows) {
@@ -1371,11 +1607,18 @@ int chi_local_energy(const void* tens, const ChiSched& sc, const uint64_t* occ, 
       k_chi_term_prep<<<(unsigned)((np + 255) / 256), 256, 0, st>>>(occ, N, sc.Ly, sc.rows, pairs, p0, np, w0, edges,
                                                                     W.prop, W.flags, W.cfg_idx, W.sides, W.count);
       VMC_CUDA_CHECK_LAUNCH();
-      rc = launch_chi_side<T>(tens, sc, W.prop, W.cfg_idx, W.sides, 2 * np, W.count, W.nw, W.nw_ex, st);
+      if (W.mask) {   // the terms' states go to the buffers that hold no walker's state
+        ChiFrom f;
+        f.edges = edges;
+        f.pairs = pairs + 2 * p0;
+        f.w0 = w0;
+        rc = launch_chi_from<T>(tens, sc, W.prop, W.cfg_idx, W.sides, 2 * np, W.count, f, W.cur, W.nw, false, st);
+      } else {
+        rc = launch_chi_side<T>(tens, sc, W.prop, W.cfg_idx, W.sides, 2 * np, W.count, W.nw.buf, W.nw.ex, st);
+      }
       if (rc) return rc;
-      k_chi_terms<T><<<(unsigned)((np + 7) / 8), 256, 0, st>>>(sc.NS, N, occ, pairs, p0, np, w0, edges, t, W.cur,
-                                                               W.cur_ex, W.s0, W.la0, W.nw, W.nw_ex, W.flags, W.prop,
-                                                               term);
+      k_chi_terms<T><<<(unsigned)((np + 7) / 8), 256, 0, st>>>(sc.NS, N, occ, pairs, p0, np, w0, edges, t, W.cur, W.s0,
+                                                               W.la0, W.nw, W.flags, W.prop, term);
       VMC_CUDA_CHECK_LAUNCH();
     }
   }
@@ -1458,7 +1701,7 @@ int vmc_peps_chi_work_bytes(int prec, int Lx, int Ly, int D, int chi, int64_t wo
   if ((prec != 0 && prec != 1) || work_rows <= 0 || !bytes) return VMC_ERR_ARGS;
   int rc = chi_plan(Lx, Ly, D, chi, sc);
   if (rc) return rc;
-  *bytes = prec == 0 ? ChiWork<float>::bytes(sc.NS, work_rows) : ChiWork<double>::bytes(sc.NS, work_rows);
+  *bytes = prec == 0 ? ChiWork<float>::bytes(sc, work_rows) : ChiWork<double>::bytes(sc, work_rows);
   return VMC_OK;
 }
 

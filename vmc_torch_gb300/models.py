@@ -789,7 +789,8 @@ class FPEPS_GB300(WavefunctionModel_GB300):
         term = torch.empty(max(P, 1), dtype=torch.float64, device=st.device)
         eloc = torch.empty(st.B, dtype=torch.float64, device=st.device)
         if self.truncated:
-            work, rows = self._chi_work(st)
+            # hop terms are built work_rows at a time: more of them than a few walkers fill the GPU
+            work, rows = self._chi_work(st, min(self.chi_rows, max(st.B, min(P, 4096))))
             offs_h = offs.cpu()
             _lib.call("vmc_peps_chi_local_energy", self._prec, _lib.ptr(T), *self._shape_args(), self.chi,
                       _lib.ptr(st.occ), st.B, _lib.ptr(edges), float(H.t), float(H.U), _lib.ptr(pairs), _lib.ptr(offs),
