@@ -431,7 +431,40 @@ __global__ void k_syrk_df(const double* __restrict__ A, int64_t lda, int64_t n, 
 // the square roots are taken for all columns at the end).  Thread (ty, tx) of
 // 8 x 16 holds the elements (ty + 8 i, tx + 16 j) in registers.  Step k: the
 // column k goes through shared memory (two buffers, one barrier a step), then
-// a_ij -= u_i (u_j / d_k); register groups left of or above k are skipped.
+// a_ij -= u_i (u_j / d_k).  Eight steps are a phase with the register groups
+// left of or above them left out at compile time: ~15 FP64 instructions a warp
+// and step (with 16 lanes a row in k_trsm64: minSR of 2049 x 8192 7.98 -> 7.31 ms).
+template <int KP>
+__device__ __forceinline__ void potrf_phase(double (&a)[8][4], double (*uc)[NB], double* dk, double* rk, int tx, int ty,
+                                            int* __restrict__ info) {
+#pragma unroll 1
+  for (int kk = 0; kk < 8; ++kk) {
+    const int k = 8 * KP + kk;
+    __syncthreads();
+    const double* u = uc[k & 1];
+    double d = u[k];
+    if (!(d > 0.0) || (__double2hiint(d) & 0x7ff00000) == 0x7ff00000) {
+      if (threadIdx.x == 0) atomicExch(info, 1);
+      d = 1e-300;
+    }
+    const double r = vmc::rcp_pos(d);
+    if (threadIdx.x == 0) { dk[k] = d; rk[k] = r; }
+    double ui[8];
+#pragma unroll
+    for (int i = KP; i < 8; ++i) ui[i] = u[ty + 8 * i];
+    const int jn = (k + 1) >> 4;
+#pragma unroll
+    for (int jj = KP / 2; jj < 4; ++jj) {   // the group of the next column comes first
+      const int c = tx + 16 * jj;
+      const double v = c > k ? u[c] * r : 0.0;
+#pragma unroll
+      for (int i = 2 * jj > KP ? 2 * jj : KP; i < 8; ++i) a[i][jj] = fma(-ui[i], v, a[i][jj]);
+      if (jj == jn && c == k + 1)
+#pragma unroll
+        for (int i = 2 * jj > KP ? 2 * jj : KP; i < 8; ++i) uc[(k + 1) & 1][ty + 8 * i] = a[i][jj];
+    }
+  }
+}
 __global__ void __launch_bounds__(128) k_potrf64(double* __restrict__ C, int64_t ldc, int nb, int* __restrict__ info) {
   __shared__ double uc[2][NB];
   __shared__ double dk[NB], rk[NB];
@@ -447,34 +480,14 @@ __global__ void __launch_bounds__(128) k_potrf64(double* __restrict__ C, int64_t
   if (tx == 0)
 #pragma unroll
     for (int i = 0; i < 8; ++i) uc[0][ty + 8 * i] = a[i][0];
-#pragma unroll 1
-  for (int k = 0; k < NB; ++k) {
-    __syncthreads();
-    const double* u = uc[k & 1];
-    double d = u[k];
-    if (!(d > 0.0) || (__double2hiint(d) & 0x7ff00000) == 0x7ff00000) {
-      if (threadIdx.x == 0) atomicExch(info, 1);
-      d = 1e-300;
-    }
-    const double r = vmc::rcp_pos(d);
-    if (threadIdx.x == 0) { dk[k] = d; rk[k] = r; }
-    double ui[8];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) ui[i] = u[ty + 8 * i];
-    const int jn = (k + 1) >> 4;    // the group of the next column comes first
-#pragma unroll
-    for (int jj = 0; jj < 4; ++jj) {
-      if (jj < jn) continue;
-      const int c = tx + 16 * jj;
-      const double v = c > k ? u[c] * r : 0.0;
-#pragma unroll
-      for (int i = 2 * jj; i < 8; ++i)
-        if (8 * i + 7 > k) a[i][jj] = fma(-ui[i], v, a[i][jj]);
-      if (jj == jn && c == k + 1)
-#pragma unroll
-        for (int i = 2 * jj; i < 8; ++i) uc[(k + 1) & 1][ty + 8 * i] = a[i][jj];
-    }
-  }
+  potrf_phase<0>(a, uc, dk, rk, tx, ty, info);
+  potrf_phase<1>(a, uc, dk, rk, tx, ty, info);
+  potrf_phase<2>(a, uc, dk, rk, tx, ty, info);
+  potrf_phase<3>(a, uc, dk, rk, tx, ty, info);
+  potrf_phase<4>(a, uc, dk, rk, tx, ty, info);
+  potrf_phase<5>(a, uc, dk, rk, tx, ty, info);
+  potrf_phase<6>(a, uc, dk, rk, tx, ty, info);
+  potrf_phase<7>(a, uc, dk, rk, tx, ty, info);
   __syncthreads();
   if (threadIdx.x < NB) {
     const double sq = sqrt(dk[threadIdx.x]);
@@ -491,25 +504,26 @@ __global__ void __launch_bounds__(128) k_potrf64(double* __restrict__ C, int64_t
     }
 }
 
-// Panel below a full 64-column diagonal tile: X = A21 L11^-T.  Four lanes a
-// row (lane q holds the columns q + 4 t), 32 rows a CTA of four warps: a row's
-// 2016 multiply-adds take 528 FP64 instructions of its warp.  The unit factor
-// L11 D^-1 is solved with, so that the divisions by the diagonal are one
-// product per entry at the end.
-constexpr int TRSM_ROWS = 32;
+// Panel below a full 64-column diagonal tile: X = A21 L11^-T.  LPR lanes a row
+// (lane q holds the columns q + LPR t), 128 / LPR rows a CTA of four warps: a
+// row's 2016 multiply-adds take 528 (LPR 4) to 160 (LPR 16) FP64 instructions of
+// its warp.  The unit factor L11 D^-1 is solved with, so that the divisions by
+// the diagonal are one product per entry at the end.
+template <int LPR>
 __global__ void __launch_bounds__(128) k_trsm64(double* __restrict__ C, int64_t ldc, int64_t rows) {
   extern __shared__ double tsm[];
   double* Lu = tsm;                  // Lu[k][c] = L11[c][k] / L11[k][k] for c > k, else 0
   double* rd = Lu + NB * NB;         // 1 / L11[k][k]
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, q = lane & 3;
-  const int64_t row = (int64_t)blockIdx.x * TRSM_ROWS + warp * 8 + (lane >> 2);
+  constexpr int NT = NB / LPR;       // entries a lane
+  const int lane = threadIdx.x & 31, q = lane % LPR;
+  const int64_t row = (int64_t)blockIdx.x * (128 / LPR) + threadIdx.x / LPR;
   double* A = C + (NB + (row < rows ? row : 0)) * ldc + q;
-  double x[NB / 4];
+  double x[NT];
 #pragma unroll
-  for (int t = 0; t < NB / 4; ++t) x[t] = A[4 * t];
+  for (int t = 0; t < NT; ++t) x[t] = A[LPR * t];
   if (threadIdx.x < NB) rd[threadIdx.x] = 1.0 / C[(int64_t)threadIdx.x * ldc + threadIdx.x];
   __syncthreads();
-#pragma unroll 8
+#pragma unroll 16
   for (int m = 0; m < NB * NB / 128; ++m) {
     const int c = m * 2 + (threadIdx.x >> 6), k = threadIdx.x & 63;   // along the rows of L11
     Lu[k * NB + c] = c > k ? C[(int64_t)c * ldc + k] * rd[k] : 0.0;
@@ -517,13 +531,13 @@ __global__ void __launch_bounds__(128) k_trsm64(double* __restrict__ C, int64_t 
   __syncthreads();
 #pragma unroll
   for (int k = 0; k < NB - 1; ++k) {
-    const double xk = __shfl_sync(VMC_FULL_MASK, x[k >> 2], (lane & 28) | (k & 3));
+    const double xk = __shfl_sync(VMC_FULL_MASK, x[k / LPR], lane - q + k % LPR);
 #pragma unroll
-    for (int t = (k + 1) >> 2; t < NB / 4; ++t) x[t] = fma(-xk, Lu[k * NB + 4 * t + q], x[t]);
+    for (int t = (k + 1) / LPR; t < NT; ++t) x[t] = fma(-xk, Lu[k * NB + LPR * t + q], x[t]);
   }
   if (row < rows) {
 #pragma unroll
-    for (int t = 0; t < NB / 4; ++t) A[4 * t] = x[t] * rd[4 * t + q];
+    for (int t = 0; t < NT; ++t) A[LPR * t] = x[t] * rd[LPR * t + q];
   }
 }
 constexpr int TRSM_SMEM = (NB * NB + NB) * 8;
@@ -538,11 +552,15 @@ int factor_step(double* T, int64_t ldt, int64_t n, int64_t k0, int* d_info, cuda
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDev) return VMC_ERR_CUDA;
     if (!g_trsm_attr[dev]) {
-      if (cudaFuncSetAttribute(k_trsm64, cudaFuncAttributeMaxDynamicSharedMemorySize, TRSM_SMEM) != cudaSuccess)
+      if (cudaFuncSetAttribute(k_trsm64<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, TRSM_SMEM) != cudaSuccess ||
+          cudaFuncSetAttribute(k_trsm64<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, TRSM_SMEM) != cudaSuccess)
         return VMC_ERR_CUDA;
       g_trsm_attr[dev] = true;
     }
-    k_trsm64<<<(unsigned)((rest + TRSM_ROWS - 1) / TRSM_ROWS), 128, TRSM_SMEM, st>>>(D, ldt, rest);
+    // a row's chain is the shorter the more lanes share it, while the CTAs fit
+    // the GPU at once: 16 lanes to two CTAs an SM
+    if (rest <= 2432) k_trsm64<16><<<(unsigned)((rest + 7) / 8), 128, TRSM_SMEM, st>>>(D, ldt, rest);
+    else k_trsm64<4><<<(unsigned)((rest + 31) / 32), 128, TRSM_SMEM, st>>>(D, ldt, rest);
   }
   return VMC_OK;
 }
