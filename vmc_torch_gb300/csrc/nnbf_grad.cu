@@ -17,6 +17,8 @@
 //
 // FP32 in bulk (vmc_nnbf_logpsi_grad_ws): the same adjoint as batched stages
 // over work_rows configurations, see "batched FP32 stages" below.
+#include <type_traits>
+
 #include "common.cuh"
 #include "sgemm.cuh"
 
@@ -370,6 +372,16 @@ __global__ void __launch_bounds__(sg::NTHR, 2) k_g_backflow(GradNet<float> net, 
   }
 }
 
+// f(I) for the compile-time I equal to the warp-uniform idx: register arrays
+// stay in registers, and only that I's instructions run
+template <int N, int I = 0, typename F>
+__device__ __forceinline__ void at_index(int idx, F f) {
+  if constexpr (I < N) {
+    if (idx == I) f(std::integral_constant<int, I>{});
+    else at_index<N, I + 1>(idx, f);
+  }
+}
+
 // A^-1 by in-place Gauss-Jordan steps in registers, NW warps a matrix (layout
 // and index algebra of k_slater_refresh).  The pivot is the largest |a| of the
 // column, on a tie the row that the elimination with row exchanges would have
@@ -435,33 +447,41 @@ __global__ void __launch_bounds__(128) k_g_invert(int N, int nf, float s, int R,
     const float ipv = 1.0f / pv;
     live &= ~(1ull << p);
     if (tid == 0) { dpiv[k] = pv; pof[k] = (uint8_t)p; kof[p] = (uint8_t)k; }
-    {
-      const int pi = p / TY;
-      const bool mine = ty == p % TY;
+    const int pi = p / TY;
+    const bool mine = ty == p % TY;    // the warp's lanes that hold row p (register row pi)
+    at_index<NI>(pi, [&](auto I) {
+      if (mine)
 #pragma unroll
-      for (int j = 0; j < NJ; ++j) {   // selects: a branch per i would index the registers through local memory
-        float v = a[0][j];
-#pragma unroll
-        for (int i = 1; i < NI; ++i) v = i == pi ? a[i][j] : v;
-        if (mine) prow[tx + TX * j] = v;
-      }
-    }
+        for (int j = 0; j < NJ; ++j) prow[tx + TX * j] = a[I][j];
+    });
     float u[NI];
 #pragma unroll
     for (int i = 0; i < NI; ++i) u[i] = col[ty + TY * i];
     sync();   // pivot row complete, column k read
-    const int jn = (k + 1) / TX;
+    float v[NJ];
 #pragma unroll
-    for (int j = 0; j < NJ; ++j) {
-      const int c = tx + TX * j;
-      const float v = c == k ? ipv : prow[c] * ipv;
+    for (int j = 0; j < NJ; ++j) v[j] = prow[tx + TX * j] * ipv;
+    at_index<NJ>(k / TX, [&](auto J) {   // column k: -a_ik / d
+      if (tx == k % TX) {
+        v[J] = ipv;
 #pragma unroll
-      for (int i = 0; i < NI; ++i)
-        a[i][j] = ty + TY * i == p ? v : fmaf(-u[i], v, c == k ? 0.f : a[i][j]);
-      if (j == jn && c == k + 1)
+        for (int i = 0; i < NI; ++i) a[i][J] = 0.f;
+      }
+    });
 #pragma unroll
-        for (int i = 0; i < NI; ++i) col[ty + TY * i] = a[i][j];
-    }
+    for (int j = 0; j < NJ; ++j)
+#pragma unroll
+      for (int i = 0; i < NI; ++i) a[i][j] = fmaf(-u[i], v[j], a[i][j]);
+    at_index<NI>(pi, [&](auto I) {
+      if (mine)
+#pragma unroll
+        for (int j = 0; j < NJ; ++j) a[I][j] = v[j];
+    });
+    at_index<NJ>((k + 1) / TX, [&](auto J) {
+      if (tx == (k + 1) % TX)
+#pragma unroll
+        for (int i = 0; i < NI; ++i) col[ty + TY * i] = a[i][J];
+    });
   }
   const bool ok = state == 1;
   sync();
