@@ -76,35 +76,46 @@ def _raise_grads(model, n_bad, B, bad_ids, n_bad_params, Np):
                      % (n_bad, B, n_bad_params, Np) + "\n".join(info))
 
 
-def _check_amps(amp, sign):
+def _queue_count(amp, sign, O):
+    """Queue vmc_check_finite on the current stream; its four counts stay on the device."""
+    ref = O if O is not None else amp
+    counts = torch.empty(4, dtype=torch.int64, device=ref.device)
+    _lib.call("vmc_check_finite", _lib.ptr(amp), _lib.ptr(sign), ref.shape[0], _lib.ptr(O),
+              0 if O is None or O.dtype == torch.float64 else 1, O.shape[1] if O is not None else 0,
+              O.stride(0) if O is not None else 0, _lib.ptr(counts), None, None, None, _lib.stream_of(ref.device))
+    return counts
+
+
+def _raise_amps(c, B):
     """First half of the reference's _check_grads_amps: NaN/Inf amplitudes
     (log mode: log|psi|) raise; zero amplitudes are counted."""
-    B = amp.shape[0]
-    _, c, _, _ = _count(amp, sign, None, 0, amp.device)
     if c[0] or c[1]:
         raise ValueError("NaN/Inf in amplitudes: %d NaN, %d Inf out of %d samples" % (c[0], c[1], B))
     last_check.clear()
     last_check.update({"zero_amplitudes": c[2], "samples": B})
 
 
-def _check_grads_amps(O, amp, sign, model):
+def _check_amps(amp, sign):
+    _raise_amps(_queue_count(amp, sign, None).tolist(), amp.shape[0])
+
+
+def _check_grads_amps(O, amp, sign, model, st):
     """The reference's _check_grads_amps on the device: amplitudes first
-    (log mode: log|psi|), then the O rows."""
-    _check_amps(amp, sign)
-    _check_O(O, model)
-
-
-def _check_O(O, model):
-    """Second half: NaN/Inf entries of O raise with the reference's message
-    (samples and parameters affected, the first bad parameters)."""
+    (log mode: log|psi|), then the O rows (NaN/Inf entries raise with the
+    reference's message: samples and parameters affected, the first bad
+    parameters).  All counts are queued before the first is read: one wait for
+    the GPU, not one per check."""
     from .optimizer import FactoredO
-    dev = O.device
-    B = O.shape[0]
+    dev, B = O.device, O.shape[0]
+    parts = [O.dense, O.g, O.h] if isinstance(O, FactoredO) else [O]
+    counts = torch.stack([_queue_count(amp if i == 0 else None, sign if i == 0 else None, t)
+                          for i, t in enumerate(parts)])
+    model.check_status(st, wait=True)
+    c = counts.tolist()
+    _raise_amps(c[0], B)
+    if not any(r[3] for r in c):
+        return
     if isinstance(O, FactoredO):
-        parts = [O.dense, O.g, O.h]
-        res = [_count(None, None, t, t.shape[1], dev) for t in parts]
-        if not any(r[1][3] for r in res):
-            return
         res = [_count(None, None, t, t.shape[1], dev, col_flags=True) for t in parts]
         rows = res[0][2].bool() | res[1][2].bool() | res[2][2].bool()
         cd, cg, ch = (r[3].bool().cpu() for r in res)
@@ -115,11 +126,9 @@ def _check_O(O, model):
         ids.sort()
         _raise_grads(model, int(rows.sum().item()), B, ids, len(ids), O.n_params)
     Np = O.shape[1]
-    st, c, _, _ = _count(None, None, O, Np, dev)
-    if c[3]:
-        _, c, _, cols = _count(None, None, O, Np, dev, col_flags=True)
-        bad = torch.nonzero(cols[:Np]).flatten()
-        _raise_grads(model, c[3], B, bad[:10].tolist(), int(bad.numel()), Np)
+    _, c, _, cols = _count(None, None, O, Np, dev, col_flags=True)
+    bad = torch.nonzero(cols[:Np]).flatten()
+    _raise_grads(model, c[3], B, bad[:10].tolist(), int(bad.numel()), Np)
 
 
 def _floor_rows(O, logabs):
@@ -145,12 +154,11 @@ def compute_grads_factored(fxs, model, use_log_amp=True, **kwargs):
     with torch.no_grad():
         st = model.bind_state(fxs)
         Od, g, h = model.logpsi_grad_factored(st)
-        model.check_status(st, wait=True)
         off = model.n_params - model.n_params_out_w - model.n_orbitals * model.n_fermions
         F = FactoredO(Od, g, h, off)
         _floor_rows(F, st.logabs)
         la = floor_log(st.logabs)
-        _check_grads_amps(F, la, st.sign, model)
+        _check_grads_amps(F, la, st.sign, model, st)
         return F, (st.sign.clone(), la)
 
 
@@ -183,9 +191,8 @@ def compute_grads_gpu(fxs, model, batch_size=None, verbose=False, offload_to_cpu
                         del Oc
                     else:
                         model.logpsi_grad(st.view(a, b), out=O[a:b])
-            model.check_status(st, wait=True)
             _floor_rows(O, st.logabs)
-            _check_grads_amps(O, la if use_log_amp else amps, sign, model)
+            _check_grads_amps(O, la if use_log_amp else amps, sign, model, st)
             if use_log_amp:
                 return O, (sign, la)
             return O.mul_(amps.to(O.dtype).unsqueeze(1)), amps

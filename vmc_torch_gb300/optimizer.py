@@ -263,14 +263,21 @@ class MinSRGB300(PreconditionerGB300):
         if check is not None:
             check()
         x = torch.empty(Ns, dtype=torch.float64, device=dev)
-        _lib.call("vmc_sr_rhs", _lib.ptr(E), Ns, Ebar, _lib.ptr(x), s)
+
+        def rhs():
+            _lib.call("vmc_sr_rhs", _lib.ptr(E), Ns, Ebar, _lib.ptr(x), s)
+
+        # the solves are queued behind the factorisation before its outcome is
+        # read, so that the GPU does not wait for the host in between
+        rhs()
+        _lib.call("vmc_sr_cholesky_solve", _lib.ptr(T), Ns, Ns, _lib.ptr(x), s)
+        stages.mark("solve")
         info, err = flag.tolist()
         if err != 0:
             raise ValueError("vmc_sr_cholesky_tc: %s" % _lib.message(err))
         if info == 0:
-            _lib.call("vmc_sr_cholesky_solve", _lib.ptr(T), Ns, Ns, _lib.ptr(x), s)
-            stages.mark("solve")
             return x, 0
+        rhs()
         # the factorisation overwrote T: rebuild it, then solve as the reference does
         build_gram(T, shift)
         T = torch.tril(T) + torch.tril(T, -1).t()   # symmetric from the lower triangle the kernels define

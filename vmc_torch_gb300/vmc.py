@@ -102,7 +102,8 @@ class VMC_GB300:
         n = local_energies.shape[0]
         m = local_energies.mean()
         var = (local_energies ** 2).mean() - m * m
-        return n, float(m.item()), float(var.item())
+        m, var = torch.stack([m, var]).tolist()
+        return n, m, var
 
     def run_vmc_loop(self, fxs, model, hamiltonian, graph, rank=0, world_size=1, config: VMCLoopConfig = None,
                      on_step_end: Optional[Callable[[Dict[str, Any]], None]] = None):
