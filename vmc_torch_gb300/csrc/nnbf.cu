@@ -33,12 +33,18 @@ using namespace vmc;
 
 namespace {
 
+// Programmatic dependent launch (single-stream sweeps): a kernel lets its
+// successor's CTAs be placed as soon as its own have started, and waits for
+// its predecessor's completion before it touches anything that one writes.  Both
+// are no-ops in a launch without the attribute.
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 constexpr int HID = 256;
 constexpr int TM = 128;          // rows per GEMM tile
 constexpr int TN = 256;          // output columns per GEMM tile
 constexpr int SMEM_A = TM * HID * 2;   // 64 KB
 constexpr int SMEM_B = TN * HID * 2;   // 128 KB
-constexpr int GEMM_SMEM = SMEM_A + SMEM_B + 1024 /*align*/ + 64 + 2 * TN * 4;
 
 __device__ __forceinline__ float gelu_f(float x) { return 0.5f * x * (1.0f + erff(x * 0.70710678118654752f)); }
 __device__ __forceinline__ double gelu_d(double x) { return 0.5 * x * (1.0 + erf(x * 0.70710678118654752440)); }
@@ -96,6 +102,8 @@ __global__ void k_prep_sweep(int64_t B, int64_t w_begin, int64_t w_end, int N, c
                              void* __restrict__ H1, int* __restrict__ cnt, int32_t* __restrict__ row_map,
                              uint64_t* __restrict__ prop_c, int* __restrict__ cnt_next) {
   const int lane = threadIdx.x & 31;
+  pdl_trigger();
+  pdl_wait();
   // the counter of the next edge: its previous users (the launches of the
   // edge before this one) have finished, as they precede this launch
   if (cnt_next && blockIdx.x == 0 && threadIdx.x == 0) *cnt_next = 0;
@@ -267,89 +275,96 @@ __global__ void k_prep_conn(int64_t P, int N, const int32_t* __restrict__ pairs 
 }
 
 // ---------------------------------------------------------------------------
-// tcgen05 GEMM: D[128 x 256] = A[128 x 256] * B[256 x 256]^T, both K-major bf16
-// in SWIZZLE_128B smem loaded by TMA; D in TMEM; fused epilogues.
+// Hidden layer: H2 = gelu(H1 W1^T + b1), a tcgen05 tile of 128 rows x 64 columns
+// a CTA (K = 256, both operands K-major bf16 in SWIZZLE_128B smem loaded by
+// TMA, D in TMEM, bias / GELU / BF16 in the epilogue).  An edge of a sweep waits
+// for this small product: a 256-column tile leaves a row tile to one CTA,
+// whose 192 KB of loads and 256 GELUs a thread take 11 us however few the rows;
+// a quarter of both runs on each of four SMs (6.44 -> 5.88 ms a
+// sweep of 112 edges for 548 walkers, with the maps encoded once a sweep).
 // ---------------------------------------------------------------------------
-enum { EPI_GELU_BF16 = 0, EPI_BACKFLOW = 1 };
+constexpr int HN = 64;                  // columns per tile
+constexpr int SMEM_HB = HN * HID * 2;   // 32 KB
+constexpr int HIDDEN_SMEM = SMEM_A + SMEM_HB + 1024 /*align*/ + 64 + HN * 4;
 
-struct EpiArgs {
-  // EPI_GELU_BF16
+struct HiddenArgs {
   const float* bias;          // (256)
   __nv_bfloat16* out;         // (rows, 256)
-  // EPI_BACKFLOW
-  const uint64_t* row_occ;    // (rows, 2)
-  const float* mbase;         // (n_orb, nf)
-  const float* outb;          // (n_orb * nf)
-  float* Aout;                // (rows, nf, nf)
-  float scale;
-  int n_sites, nf;
   // bounded wait for the operand tiles (0: 1 s); skip_loads issues no tile
   // load, so that the wait runs out with nothing in flight (self-test of the
   // timeout path, vmc_nnbf_hidden_layer)
   uint64_t wait_ns;
   int skip_loads;
+  // load the weights before the predecessor's end (launches that overlap it)
+  int early_b;
   // compacted rows: the row count is *rows_dev (device), at most `rows`
   const int* rows_dev;
 };
 
-template <int EPI>
-__global__ void __launch_bounds__(128, 1)
-    k_gemm_tc(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, int rows, EpiArgs ea,
-              int* __restrict__ err) {
+__global__ void __launch_bounds__(128, 2)
+    k_hidden_tc(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, int rows,
+                HiddenArgs ea, int* __restrict__ err) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* sm = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint8_t* sA = sm;
   uint8_t* sB = sm + SMEM_A;
-  uint64_t* bars = (uint64_t*)(sm + SMEM_A + SMEM_B);
+  uint64_t* bars = (uint64_t*)(sm + SMEM_A + SMEM_HB);   // H1 tile, MMAs; the weights' at [4]
   uint32_t* tslot = (uint32_t*)(bars + 2);
   int* sflag = (int*)(bars + 3);
-  float* sc0 = (float*)(sm + SMEM_A + SMEM_B + 64);   // bias, or M_base slice
-  float* sc1 = sc0 + TN;                               // out_b slice
+  float* bias = (float*)(sm + SMEM_A + SMEM_HB + 64);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int row0 = blockIdx.x * TM;
-  const int brow0 = blockIdx.y * TN;
-  if (ea.rows_dev) {   // uniform over the CTA, before any barrier or allocation
-    const int rr = *ea.rows_dev;
-    if (row0 >= rr) return;
-    rows = rows < rr ? rows : rr;
-  }
+  const int brow0 = blockIdx.y * HN;
+  pdl_trigger();
   if (threadIdx.x == 0) {
     tc::mbar_init(&bars[0], 1);
     tc::mbar_init(&bars[1], 1);
+    tc::mbar_init(&bars[4], 1);
     tc::fence_mbar_init();
     tc::prefetch_tmap(&tmA);
     tc::prefetch_tmap(&tmB);
     *sflag = 1;
   }
-  if (EPI == EPI_GELU_BF16) {
-    for (int q = threadIdx.x; q < TN; q += blockDim.x) sc0[q] = ea.bias[brow0 + q];
-  } else {
-    for (int q = threadIdx.x; q < TN; q += blockDim.x) {
-      sc0[q] = ea.mbase[brow0 + q];
-      sc1[q] = ea.outb[brow0 + q];
+  // the weights' tile, which no earlier kernel of the stream writes, may come
+  // before the predecessor's end
+  auto load_b = [&] {
+    tc::mbar_arrive_expect_tx(&bars[4], SMEM_HB);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) tc::tma_load_2d(sB + j * (HN * 128), &tmB, &bars[4], j * 64, brow0);
+  };
+  if (ea.early_b && threadIdx.x == 0) load_b();
+  pdl_wait();
+  if (ea.rows_dev) {   // uniform over the CTA, before any barrier or allocation
+    const int rr = *ea.rows_dev;
+    if (row0 >= rr) {
+      if (ea.early_b && threadIdx.x == 0) tc::mbar_wait(&bars[4], 0);   // nothing in flight at the exit
+      return;
     }
+    rows = rows < rr ? rows : rr;
   }
-  if (warp == 0) tc::tmem_alloc(tslot, 256);
+  if (threadIdx.x < HN) bias[threadIdx.x] = ea.bias[brow0 + threadIdx.x];
+  if (warp == 0) tc::tmem_alloc(tslot, HN);
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
   const uint32_t tbase = *tslot;
   if (threadIdx.x == 0) {
     if (!ea.skip_loads) {
-      tc::mbar_arrive_expect_tx(&bars[0], SMEM_A + SMEM_B);
+      tc::mbar_arrive_expect_tx(&bars[0], SMEM_A);
 #pragma unroll
       for (int j = 0; j < 4; ++j) tc::tma_load_2d(sA + j * (TM * 128), &tmA, &bars[0], j * 64, row0);
-#pragma unroll
-      for (int j = 0; j < 4; ++j) tc::tma_load_2d(sB + j * (TN * 128), &tmB, &bars[0], j * 64, brow0);
+      if (!ea.early_b) load_b();
     }
-    if (tc::mbar_wait(&bars[0], 0, ea.wait_ns ? ea.wait_ns : 1000000000ull)) {
+    const uint64_t lim = ea.wait_ns ? ea.wait_ns : 1000000000ull;
+    const bool a_in = tc::mbar_wait(&bars[0], 0, lim), b_in = tc::mbar_wait(&bars[4], 0, lim);
+    if (a_in && b_in) {
       tc::fence_after_sync();
-      constexpr uint32_t idesc = tc::idesc_bf16_f32(TM, TN);
+      constexpr uint32_t idesc = tc::idesc_bf16_f32(TM, HN);
 #pragma unroll
       for (int ks = 0; ks < HID / 16; ++ks) {
         const int j = ks >> 2, kk = ks & 3;
         const uint64_t ad = tc::sdesc_sw128(tc::smem_u32(sA + j * (TM * 128)) + kk * 32);
-        const uint64_t bd = tc::sdesc_sw128(tc::smem_u32(sB + j * (TN * 128)) + kk * 32);
+        const uint64_t bd = tc::sdesc_sw128(tc::smem_u32(sB + j * (HN * 128)) + kk * 32);
         tc::mma_bf16(tbase, ad, bd, idesc, ks > 0 ? 1u : 0u);
       }
       tc::mma_commit(&bars[1]);
@@ -365,55 +380,29 @@ __global__ void __launch_bounds__(128, 1)
     if (!done) {
       if (lane == 0) atomicExch(err, VMC_ERR_TIMEOUT);
     } else {
-      const int r = warp * 32 + lane;
-      const int64_t row = (int64_t)row0 + r;
+      const int64_t row = (int64_t)row0 + warp * 32 + lane;
       const bool live = row < rows;
-      uint64_t up = 0, dn = 0;
-      if (EPI == EPI_BACKFLOW && live) { up = ea.row_occ[2 * row]; dn = ea.row_occ[2 * row + 1]; }
 #pragma unroll 1
-      for (int cc = 0; cc < TN / 32; ++cc) {
+      for (int cc = 0; cc < HN / 32; ++cc) {
         float v[32];
         tc::tmem_ld32(tbase + ((uint32_t)(warp * 32) << 16) + (uint32_t)(cc * 32), v);
         if (!live) continue;
-        if (EPI == EPI_GELU_BF16) {
-          const int n0 = brow0 + cc * 32;
-          uint32_t pk[16];
+        uint32_t pk[16];
 #pragma unroll
-          for (int q = 0; q < 16; ++q) {
-            __nv_bfloat162 h2 = __floats2bfloat162_rn(gelu_f(v[2 * q] + sc0[cc * 32 + 2 * q]),
-                                                      gelu_f(v[2 * q + 1] + sc0[cc * 32 + 2 * q + 1]));
-            pk[q] = *reinterpret_cast<uint32_t*>(&h2);
-          }
-          uint4* dst = reinterpret_cast<uint4*>(ea.out + row * HID + n0);
-#pragma unroll
-          for (int q = 0; q < 4; ++q) dst[q] = make_uint4(pk[4 * q], pk[4 * q + 1], pk[4 * q + 2], pk[4 * q + 3]);
-        } else {
-          const int nf = ea.nf;
-          const int col = brow0 + cc * 32;          // flat output index = orbital * nf + c
-          const int orb = col / nf, c0 = col - orb * nf;
-          const int N = ea.n_sites;
-          if (!orb_occupied(up, dn, N, orb)) continue;
-          const int pos = orb_prefix(up, dn, N, orb);
-          if (pos >= nf) continue;
-          float* dst = ea.Aout + ((size_t)row * nf + pos) * nf + c0;
-          const float* mb = sc0 + cc * 32;   // == M_base[orb][c0 ..], staged
-          const float* ob = sc1 + cc * 32;   // == out_b[orb * nf + c0 ..], staged
-#pragma unroll
-          for (int q = 0; q < 8; ++q) {
-            float4 o;
-            o.x = mb[4 * q + 0] + ea.scale * (v[4 * q + 0] + ob[4 * q + 0]);
-            o.y = mb[4 * q + 1] + ea.scale * (v[4 * q + 1] + ob[4 * q + 1]);
-            o.z = mb[4 * q + 2] + ea.scale * (v[4 * q + 2] + ob[4 * q + 2]);
-            o.w = mb[4 * q + 3] + ea.scale * (v[4 * q + 3] + ob[4 * q + 3]);
-            reinterpret_cast<float4*>(dst)[q] = o;
-          }
+        for (int q = 0; q < 16; ++q) {
+          __nv_bfloat162 h2 = __floats2bfloat162_rn(gelu_f(v[2 * q] + bias[cc * 32 + 2 * q]),
+                                                    gelu_f(v[2 * q + 1] + bias[cc * 32 + 2 * q + 1]));
+          pk[q] = *reinterpret_cast<uint32_t*>(&h2);
         }
+        uint4* dst = reinterpret_cast<uint4*>(ea.out + row * HID + brow0 + cc * 32);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) dst[q] = make_uint4(pk[4 * q], pk[4 * q + 1], pk[4 * q + 2], pk[4 * q + 3]);
       }
     }
   }
   tc::fence_before_sync();
   __syncthreads();
-  if (warp == 0) tc::tmem_dealloc(tbase, 256);
+  if (warp == 0) tc::tmem_dealloc(tbase, HN);
 }
 
 // ---------------------------------------------------------------------------
@@ -460,17 +449,7 @@ __global__ void __launch_bounds__(PB_THREADS, 1)
   float* cM = (float*)(sm + SMEM_A + SMEM_B + 256);
   float* cO = cM + TN;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  int R = pa.R, n_tiles = pa.n_tiles, n_items = pa.n_items;
-  if (pa.rows_dev) {   // the same value in every thread: all roles walk the same items
-    const int64_t rr = (int64_t)*pa.rows_dev - pa.rows_off;
-    R = rr < 0 ? 0 : (rr < R ? (int)rr : R);
-    const int n_groups = pa.n_items / pa.n_tiles;
-    n_tiles = (R + TM - 1) / TM;
-    n_items = n_groups * n_tiles;
-  }
-  const int per = (n_items + gridDim.x - 1) / gridDim.x;
-  const int it0 = blockIdx.x * per;
-  const int it1 = min(n_items, it0 + per);
+  pdl_trigger();
   if (threadIdx.x == 0) {
     tc::mbar_init(bfull, 1);
     tc::mbar_init(bempty, 1);
@@ -486,6 +465,18 @@ __global__ void __launch_bounds__(PB_THREADS, 1)
   __syncthreads();
   tc::fence_after_sync();
   const uint32_t tbase = *tslot;
+  pdl_wait();
+  int R = pa.R, n_tiles = pa.n_tiles, n_items = pa.n_items;
+  if (pa.rows_dev) {   // the same value in every thread: all roles walk the same items
+    const int64_t rr = (int64_t)*pa.rows_dev - pa.rows_off;
+    R = rr < 0 ? 0 : (rr < R ? (int)rr : R);
+    const int n_groups = pa.n_items / pa.n_tiles;
+    n_tiles = (R + TM - 1) / TM;
+    n_items = n_groups * n_tiles;
+  }
+  const int per = (n_items + gridDim.x - 1) / gridDim.x;
+  const int it0 = blockIdx.x * per;
+  const int it1 = min(n_items, it0 + per);
   if (it0 < it1) {
     if (warp == 0) {
       if (lane == 0) {  // ---------------- TMA producer ----------------
@@ -667,7 +658,7 @@ struct Det { double logabs; double sign; };
 // Register layouts of the elimination: LU_FULL = rows lane and lane + 32 (of
 // a 64-row matrix; row lane of a 32-row one); LU_PAIRED = two matrices a
 // warp, lanes 16 h .. 16 h + 15 holding two live rows each of matrix h (see
-// warp_logdet_f32_pair).
+// lu_tail_pair).
 enum { LU_FULL = 0, LU_PAIRED = 1 };
 
 template <int NF>
@@ -911,8 +902,7 @@ __device__ __forceinline__ Det lu_det(bool ok, float mant, int expo, int neg) {
   return d;
 }
 
-// One 32 x 32 matrix a warp (64 x 64 matrices go two a warp through
-// warp_logdet_f32_pair).
+// One 32 x 32 matrix a warp (64 x 64 matrices: k_logdet_pair).
 template <int NF>
 __device__ __forceinline__ Det warp_logdet_f32(const float* __restrict__ A, float* prow) {
   static_assert(NF == 32, "one-matrix path: NF = 32");
@@ -979,81 +969,6 @@ __device__ __forceinline__ void lu_tail_pair(LuRegs<64>& S, int orow, const floa
     S.neg = unpark_neg(psw[36]);
     S.ok = (psw[36] >> 1) & 1u;
   }
-  S.half = half;
-  S.pbit[0] = 1ull << S.prow_of[0];
-  S.pbit[1] = 1ull << S.prow_of[1];
-  S.key = lu_pivot_key<64, 2, 0, 0, LU_PAIRED>(S, lane);
-  lu_phase<64, 2, 32, LU_PAIRED>(S, prow, lane);
-  lu_phase<64, 2, 16, LU_PAIRED>(S, prow, lane);
-  // each half's state -> both results
-  const float mo = __shfl_xor_sync(VMC_FULL_MASK, S.mant, 16);
-  const int eo = __shfl_xor_sync(VMC_FULL_MASK, S.expo, 16);
-  const int no = __shfl_xor_sync(VMC_FULL_MASK, S.neg, 16);
-  const bool oo = __shfl_xor_sync(VMC_FULL_MASK, (int)S.ok, 16) != 0;
-  const Det mine = lu_det(S.ok, S.mant, S.expo, S.neg), other = lu_det(oo, mo, eo, no);
-  d0 = half ? other : mine;
-  d1 = half ? mine : other;
-}
-
-// Two 64 x 64 matrices on one warp.  Each runs its first 32 pivot steps in
-// the full layout, then parks its 32 x 32 remainder in its own first 4 KB
-// (L2; the warp has consumed those rows) and its scalar state in the warp's
-// shared words, so nothing but indices stays live from one matrix to the
-// next.  The remainders then share the warp: half h (lanes 16 h .. 16 h + 15)
-// reloads live rows i and i + 16 of matrix h, and the last 32 steps of both
-// run as one instruction stream.  A row's updates are the same FMAs in either
-// layout and the pivot keys carry the original row numbers, so a matrix's
-// result does not depend on its partner or on the pairing.  The matrices
-// are rows sw[38 + h] of A; with nm = 1 both halves carry matrix 0 and the
-// second result is unused.
-__device__ __forceinline__ void warp_logdet_f32_pair(float* A, float* prow, uint32_t* sw, int nm, Det& d0,
-                                                     Det& d1) {
-  const int lane = threadIdx.x & 31;
-  LuRegs<64> S;
-#pragma unroll 1
-  for (int m = 0; m < nm; ++m) {
-    float* Am = A + (size_t)sw[38 + m] * 4096;
-    lu_load<64>(S, Am, lane);
-    lu_phase<64, 2, 64, LU_FULL>(S, prow, lane);
-    lu_phase<64, 2, 48, LU_FULL>(S, prow, lane);
-    const int orow = lu_compact<32>(S, lane);
-    __syncwarp();  // every lane's loads of the matrix precede the parking stores
-    float4* park = reinterpret_cast<float4*>(Am);
-#pragma unroll
-    for (int q = 0; q < 8; ++q)
-      __stcg(park + q * 32 + lane,
-             make_float4(S.a[0][2 * q].x, S.a[0][2 * q].y, S.a[0][2 * q + 1].x, S.a[0][2 * q + 1].y));
-    uint32_t* w = sw + 40 * m;   // [0, 32): original row held by each lane; [32, 37): scalar state
-    w[lane] = (uint32_t)orow;
-    if (lane == 0) {
-      w[32] = (uint32_t)S.U;
-      w[33] = (uint32_t)(S.U >> 32);
-      w[34] = __float_as_uint(S.mant);
-      w[35] = (uint32_t)S.expo;
-      w[36] = park_flags(S.neg, S.ok);
-    }
-  }
-  __syncwarp();  // parked rows and words visible to every lane
-  const int half = lane >> 4;
-  const int h = nm == 2 ? half : 0;   // matrix carried by this lane
-  const int i = lane & 15;
-  const uint32_t* w = sw + 40 * h;
-  const float4* park = reinterpret_cast<const float4*>(A + (size_t)sw[38 + h] * 4096);
-#pragma unroll
-  for (int q = 0; q < 8; ++q) {
-    const float4 v0 = __ldcg(park + q * 32 + i), v1 = __ldcg(park + q * 32 + i + 16);
-    S.a[0][2 * q] = make_float2(v0.x, v0.y);
-    S.a[0][2 * q + 1] = make_float2(v0.z, v0.w);
-    S.a[1][2 * q] = make_float2(v1.x, v1.y);
-    S.a[1][2 * q + 1] = make_float2(v1.z, v1.w);
-  }
-  S.prow_of[0] = (int)w[i];
-  S.prow_of[1] = (int)w[i + 16];
-  S.U = (uint64_t)w[32] | ((uint64_t)w[33] << 32);
-  S.mant = __uint_as_float(w[34]);
-  S.expo = (int)w[35];
-  S.neg = unpark_neg(w[36]);
-  S.ok = (w[36] >> 1) & 1u;
   S.half = half;
   S.pbit[0] = 1ull << S.prow_of[0];
   S.pbit[1] = 1ull << S.prow_of[1];
@@ -1257,6 +1172,8 @@ __device__ __forceinline__ void ld_finish(int64_t row, const Det& d, const LdArg
 template <typename T, int NF, int MODE>
 __global__ void __launch_bounds__(128, LU_MIN_CTAS) k_logdet(int64_t R, int64_t row0, int nf, const T* __restrict__ A, LdArgs la) {
   extern __shared__ __align__(16) uint8_t lsm[];
+  pdl_trigger();
+  pdl_wait();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int64_t local = (int64_t)blockIdx.x * (blockDim.x >> 5) + warp;
   if (local >= R) return;
@@ -1294,9 +1211,8 @@ __device__ __forceinline__ bool ld_flag(const LdArgs& la, int64_t row) {
 // scalar state in shared memory and retires; the even warp runs both tails as
 // one instruction stream (lu_tail_pair) and finishes both rows.  A warp
 // without a partner runs its tail alone in the same layout.
-// shared words per warp: 128 floats of pivot-row slots + parked state (k_logdet_dual: two 40-word blocks,
-// k_logdet_pair: one)
-constexpr int LDP_WARP_WORDS = 128 + 80;
+// shared words per warp: 128 floats of pivot-row slots + parked state
+constexpr int LDP_WARP_WORDS = 128 + 40;
 
 // Named barrier of warps 2k and 2k + 1 (ids 1 and 2; 0 is __syncthreads').
 __device__ __forceinline__ void pair_barrier(int warp) {
@@ -1306,6 +1222,8 @@ __device__ __forceinline__ void pair_barrier(int warp) {
 template <int MODE>
 __global__ void __launch_bounds__(128, LU_MIN_CTAS) k_logdet_pair(int64_t R, int64_t row0, float* A, LdArgs la) {
   extern __shared__ __align__(16) uint8_t lsm[];
+  pdl_trigger();
+  pdl_wait();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int64_t base = (int64_t)blockIdx.x * 4;
   const int64_t Reff = ld_rows(la, R);
@@ -1361,39 +1279,6 @@ __global__ void __launch_bounds__(128, LU_MIN_CTAS) k_logdet_pair(int64_t R, int
   const int nd = paired ? 2 : 1;
 #pragma unroll 1
   for (int k = 0; k < nd; ++k) ld_finish<float, MODE>(ld_row(la, row0, k ? lp : l), k ? d1 : d0, la, lane);
-}
-
-// FP32 64 x 64 rows, two matrices a warp throughout: a CTA of 4 warps takes
-// 8 rows and hands the ones that need an evaluation out in pairs (warp w: the
-// (2w)-th and (2w+1)-th; at most one warp of a CTA is left with one), see
-// warp_logdet_f32_pair.  Half as many warps as k_logdet_pair, each busy to
-// the end: the better choice when other launches (concurrent walker groups)
-// fill the SMs; alone on the GPU k_logdet_pair's warp per row wins.
-template <int MODE>
-__global__ void __launch_bounds__(128, LU_MIN_CTAS) k_logdet_dual(int64_t R, int64_t row0, float* A, LdArgs la) {
-  extern __shared__ __align__(16) uint8_t lsm[];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int64_t base = (int64_t)blockIdx.x * 8;
-  const int64_t Reff = ld_rows(la, R);
-  bool fl = false;
-  if (lane < 8 && base + lane < Reff) fl = la.rows_dev ? true : ld_flag<MODE>(la, row0 + base + lane);
-  unsigned m = __ballot_sync(VMC_FULL_MASK, fl);
-  for (int i = 0; i < 2 * warp; ++i) m &= m - 1u;
-  if (!m) return;
-  const int64_t l0 = base + (__ffs(m) - 1);
-  m &= m - 1u;
-  const int64_t l1 = m ? base + (__ffs(m) - 1) : -1;
-  if (MODE == LD_ACCEPT && la.n_eval && lane == 0) atomicAdd(la.n_eval, l1 >= 0 ? 2ull : 1ull);
-  float* prow = reinterpret_cast<float*>(lsm) + warp * LDP_WARP_WORDS;
-  uint32_t* sw = reinterpret_cast<uint32_t*>(prow + 128);
-  // the rows (local indices < 2^31) wait in shared memory during the elimination
-  if (lane == 0) { sw[38] = (uint32_t)l0; sw[39] = (uint32_t)(l1 < 0 ? l0 : l1); }
-  const int nd = l1 < 0 ? 1 : 2;
-  __syncwarp();
-  Det d0, d1;
-  warp_logdet_f32_pair(A, prow, sw, nd, d0, d1);
-#pragma unroll 1
-  for (int k = 0; k < nd; ++k) ld_finish<float, MODE>(ld_row(la, row0, (int64_t)sw[38 + k]), k ? d1 : d0, la, lane);
 }
 
 // per-walker local energy: U * doublons + segmented sum of the hop terms
@@ -1596,6 +1481,13 @@ ChunkPipe* chunk_pipe() {
   return ok ? &p : nullptr;
 }
 
+// Least walkers of a group: a group's kernels must still fill the GPU for most
+// of their time, or its second stream only adds gaps that a single stream of
+// overlapping launches does not have (64 orbitals, a 112-edge sweep of 3044
+// walkers: 11.4 ms as one group, 12.3 as two; 6000 walkers: 22.0 as one, 18.3 as
+// two; 32 orbitals, 5000 walkers: 4.7 as one, 4.1 as two, 4.5 as four).
+constexpr int64_t kLaneRows = 2048;
+
 // Walker groups per sweep (VMC_GB300_SWEEP_LANES, 1..4; default 4).  The
 // groups are independent Markov chains, so each runs its whole edge loop on
 // its own stream and the groups' GEMMs, LUs and proposal kernels overlap
@@ -1609,26 +1501,58 @@ int sweep_lanes() {
   return n;
 }
 
+// <<<grid, block, smem, st>>>, with pdl as a dependent launch that may overlap
+// the end of the kernel before it on the stream (every kernel so launched
+// calls pdl_wait before it reads or writes anything shared).
+template <typename... KArgs, typename... Args>
+void launch(bool pdl, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args&&... args) {
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = &attr;
+  cfg.numAttrs = pdl ? 1 : 0;
+  cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);   // a failure shows in VMC_CUDA_CHECK_LAUNCH
+}
+
+// Tensor maps of one workspace and network, encoded once for all edges of a
+// sweep (four driver calls an edge otherwise): H1, W1, out_w, and H2 of up to
+// kChunkRows rows.
+struct EvalMaps {
+  CUtensorMap tH1, tW1, tOW, tH2;
+  bool make(const Work& wk, const NetF32& n, int64_t R, int n_orb, int nf) {
+    return tmap_bf16(&tH1, wk.H1, (uint64_t)R, TM) && tmap_bf16(&tW1, n.w1, HID, HN) &&
+           tmap_bf16(&tOW, n.outw, (uint64_t)n_orb * nf, TN) &&
+           tmap_bf16(&tH2, wk.H2, (uint64_t)(R < kChunkRows ? R : kChunkRows), TM);
+  }
+};
+
 // d_count / row_map (mixed precision, nf = 64): the rows are compacted, their
 // number *d_count on the device (at most R) and their walkers row_map.
 int launch_eval_rows(int prec, int64_t R, int N, int nf, const uint64_t* row_occ, const void* net, double scale,
                      const Work& wk, int* err, cudaStream_t st, int ldmode, const LdArgs& la,
-                     bool allow_pipe = true, bool concurrent = false, const int* d_count = nullptr,
-                     const int32_t* row_map = nullptr) {
+                     bool allow_pipe = true, const int* d_count = nullptr,
+                     const int32_t* row_map = nullptr, const EvalMaps* maps = nullptr, bool pdl = false) {
   const int n_orb = 2 * N;
   if (prec == 0) {
     const NetF32& n = *(const NetF32*)net;
-    CUtensorMap tH1, tW1, tOW;
-    if (!tmap_bf16(&tH1, wk.H1, (uint64_t)R, TM) || !tmap_bf16(&tW1, n.w1, HID, TN) ||
-        !tmap_bf16(&tOW, n.outw, (uint64_t)n_orb * nf, TN))
-      return VMC_ERR_UNSUPPORTED;
-    EpiArgs e1{};
+    EvalMaps own;
+    if (!maps) {
+      if (!own.make(wk, n, R, n_orb, nf)) return VMC_ERR_UNSUPPORTED;
+      maps = &own;
+    }
+    HiddenArgs e1{};
     e1.bias = n.b1;
     e1.out = (__nv_bfloat16*)wk.H2;
     e1.rows_dev = d_count;
-    dim3 g1((unsigned)((R + TM - 1) / TM), 1);
+    dim3 g1((unsigned)((R + TM - 1) / TM), HID / HN);
     STAGE_BEGIN(1);
-    k_gemm_tc<EPI_GELU_BF16><<<g1, 128, GEMM_SMEM, st>>>(tH1, tW1, (int)R, e1, err);
+    e1.early_b = pdl ? 1 : 0;
+    launch(pdl, k_hidden_tc, g1, 128, HIDDEN_SMEM, st, maps->tH1, maps->tW1, (int)R, e1, err);
     STAGE_END(1);
     const int n_groups = (n_orb * nf) / TN;
     const int64_t CH = R < kChunkRows ? R : kChunkRows;
@@ -1656,8 +1580,9 @@ int launch_eval_rows(int prec, int64_t R, int N, int nf, const uint64_t* row_occ
       const int64_t Rc = (R - c0) < CH ? (R - c0) : CH;
       const int slot = pipe ? (int)(ci & 1) : 0;
       float* Ac = (float*)wk.A + (size_t)slot * (size_t)CH * nf * nf;
-      CUtensorMap tH2c;
-      if (!tmap_bf16(&tH2c, (const __nv_bfloat16*)wk.H2 + c0 * HID, (uint64_t)Rc, TM)) return fail(VMC_ERR_UNSUPPORTED);
+      CUtensorMap tH2c = maps->tH2;
+      if (ci > 0 && !tmap_bf16(&tH2c, (const __nv_bfloat16*)wk.H2 + c0 * HID, (uint64_t)Rc, TM))
+        return fail(VMC_ERR_UNSUPPORTED);
       PBArgs pa{};
       pa.row_occ = row_occ + 2 * c0; pa.mbase = n.mbase; pa.outb = n.outb; pa.Aout = Ac;
       pa.scale = (float)scale; pa.n_sites = N; pa.nf = nf; pa.R = (int)Rc;
@@ -1669,7 +1594,7 @@ int launch_eval_rows(int prec, int64_t R, int N, int nf, const uint64_t* row_occ
       cudaStream_t gs = pipe ? pipe->aux : st;
       if (pipe && ci >= 2 && cudaStreamWaitEvent(gs, pipe->lu[slot], 0) != cudaSuccess) return fail(VMC_ERR_CUDA);
       STAGE_BEGIN(2);
-      k_backflow_persistent<<<grid, PB_THREADS, PB_SMEM, gs>>>(tH2c, tOW, pa, err);
+      launch(pdl, k_backflow_persistent, grid, PB_THREADS, PB_SMEM, gs, tH2c, maps->tOW, pa, err);
       STAGE_END(2);
       if (pipe) {
         if (cudaEventRecord(pipe->g[slot], gs) != cudaSuccess || cudaStreamWaitEvent(st, pipe->g[slot], 0) != cudaSuccess)
@@ -1681,26 +1606,19 @@ int launch_eval_rows(int prec, int64_t R, int N, int nf, const uint64_t* row_occ
       lc.rows_off = c0;
       lc.row_map = row_map;
       const unsigned gl = (unsigned)((Rc + wpb - 1) / wpb);
-      if (nf == 64 && !concurrent) {  // warp pairs share the tails (the orbital-matrix slot is scratch: the LU parks in it)
+      if (nf == 64) {  // warp pairs share the tails (the orbital-matrix slot is scratch: the LU parks in it)
         const unsigned gp = (unsigned)((Rc + wpb - 1) / wpb);
         const size_t psmem = (size_t)wpb * LDP_WARP_WORDS * sizeof(float);
-        if (ldmode == LD_ACCEPT) k_logdet_pair<LD_ACCEPT><<<gp, 32 * wpb, psmem, st>>>(Rc, c0, Ac, lc);
-        else if (ldmode == LD_EVAL) k_logdet_pair<LD_EVAL><<<gp, 32 * wpb, psmem, st>>>(Rc, c0, Ac, lc);
-        else if (ldmode == LD_ACCEPT_Q) k_logdet_pair<LD_ACCEPT_Q><<<gp, 32 * wpb, psmem, st>>>(Rc, c0, Ac, lc);
-        else k_logdet_pair<LD_ELOC><<<gp, 32 * wpb, psmem, st>>>(Rc, c0, Ac, lc);
-      } else if (nf == 64) {  // two matrices a warp (concurrent walker groups fill the SMs)
-        const unsigned gp = (unsigned)((Rc + 2 * wpb - 1) / (2 * wpb));
-        const size_t psmem = (size_t)wpb * LDP_WARP_WORDS * sizeof(float);
-        if (ldmode == LD_ACCEPT) k_logdet_dual<LD_ACCEPT><<<gp, 32 * wpb, psmem, st>>>(Rc, c0, Ac, lc);
-        else if (ldmode == LD_EVAL) k_logdet_dual<LD_EVAL><<<gp, 32 * wpb, psmem, st>>>(Rc, c0, Ac, lc);
-        else if (ldmode == LD_ACCEPT_Q) k_logdet_dual<LD_ACCEPT_Q><<<gp, 32 * wpb, psmem, st>>>(Rc, c0, Ac, lc);
-        else k_logdet_dual<LD_ELOC><<<gp, 32 * wpb, psmem, st>>>(Rc, c0, Ac, lc);
+        if (ldmode == LD_ACCEPT) launch(pdl, k_logdet_pair<LD_ACCEPT>, gp, 32 * wpb, psmem, st, Rc, c0, Ac, lc);
+        else if (ldmode == LD_EVAL) launch(pdl, k_logdet_pair<LD_EVAL>, gp, 32 * wpb, psmem, st, Rc, c0, Ac, lc);
+        else if (ldmode == LD_ACCEPT_Q) launch(pdl, k_logdet_pair<LD_ACCEPT_Q>, gp, 32 * wpb, psmem, st, Rc, c0, Ac, lc);
+        else launch(pdl, k_logdet_pair<LD_ELOC>, gp, 32 * wpb, psmem, st, Rc, c0, Ac, lc);
       } else {
         // no compaction with 32 orbitals (the caller passes none)
-        if (ldmode == LD_ACCEPT) k_logdet<float, 32, LD_ACCEPT><<<gl, 32 * wpb, lsmem, st>>>(Rc, c0, nf, Ac, la);
-        else if (ldmode == LD_EVAL) k_logdet<float, 32, LD_EVAL><<<gl, 32 * wpb, lsmem, st>>>(Rc, c0, nf, Ac, la);
-        else if (ldmode == LD_ACCEPT_Q) k_logdet<float, 32, LD_ACCEPT_Q><<<gl, 32 * wpb, lsmem, st>>>(Rc, c0, nf, Ac, la);
-        else k_logdet<float, 32, LD_ELOC><<<gl, 32 * wpb, lsmem, st>>>(Rc, c0, nf, Ac, la);
+        if (ldmode == LD_ACCEPT) launch(pdl, k_logdet<float, 32, LD_ACCEPT>, gl, 32 * wpb, lsmem, st, Rc, c0, nf, Ac, la);
+        else if (ldmode == LD_EVAL) launch(pdl, k_logdet<float, 32, LD_EVAL>, gl, 32 * wpb, lsmem, st, Rc, c0, nf, Ac, la);
+        else if (ldmode == LD_ACCEPT_Q) launch(pdl, k_logdet<float, 32, LD_ACCEPT_Q>, gl, 32 * wpb, lsmem, st, Rc, c0, nf, Ac, la);
+        else launch(pdl, k_logdet<float, 32, LD_ELOC>, gl, 32 * wpb, lsmem, st, Rc, c0, nf, Ac, la);
       }
       STAGE_END(3);
       if (pipe && cudaEventRecord(pipe->lu[slot], st) != cudaSuccess) return fail(VMC_ERR_CUDA);
@@ -1736,8 +1654,7 @@ void set_attrs() {
   const int dev = current_device();
   std::lock_guard<std::mutex> lk(g_attr_mu);
   if (g_attr_done[dev]) return;
-  cudaFuncSetAttribute(k_gemm_tc<EPI_GELU_BF16>, cudaFuncAttributeMaxDynamicSharedMemorySize, GEMM_SMEM);
-  cudaFuncSetAttribute(k_gemm_tc<EPI_BACKFLOW>, cudaFuncAttributeMaxDynamicSharedMemorySize, GEMM_SMEM);
+  cudaFuncSetAttribute(k_hidden_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, HIDDEN_SMEM);
   cudaFuncSetAttribute(k_backflow_persistent, cudaFuncAttributeMaxDynamicSharedMemorySize, PB_SMEM);
   g_attr_done[dev] = true;
 }
@@ -1842,14 +1759,14 @@ int vmc_nnbf_sweep(int prec, const void* const* net_ptrs, int n_sites, int nf, i
     cprop = (uint64_t*)((char*)compact_ws + 256 + (((size_t)B * 4 + 15) & ~(size_t)15));
     if (cudaMemsetAsync(ccnt, 0, 2 * ChunkPipe::kLanes * sizeof(int), st) != cudaSuccess) return VMC_ERR_CUDA;
   }
-  // walker groups on their own streams (mixed precision, untimed stages, B >= 2 chunks)
+  // walker groups on their own streams (mixed precision, untimed stages, B >= 2 groups)
   ChunkPipe* pipe = nullptr;
   int G = 1;
-  if (prec == 0 && !stage_ms && sweep_lanes() > 1 && B >= 2 * kChunkRows) {
+  if (prec == 0 && !stage_ms && sweep_lanes() > 1 && B >= 2 * kLaneRows) {
     pipe = chunk_pipe();
     if (pipe && pipe->lanes_ok) {
       G = sweep_lanes();
-      if ((int64_t)G > B / kChunkRows) G = (int)(B / kChunkRows);
+      if ((int64_t)G > B / kLaneRows) G = (int)(B / kLaneRows);
     } else {
       pipe = nullptr;
     }
@@ -1874,6 +1791,12 @@ int vmc_nnbf_sweep(int prec, const void* const* net_ptrs, int n_sites, int nf, i
       const Work wg{(char*)H1 + (size_t)w0 * HID * 2, (char*)H2 + (size_t)w0 * HID * 2,
                     (float*)A + (size_t)w0 * nf * nf};
       const unsigned gwg = (unsigned)(((w1 - w0) * 32 + 255) / 256);
+      EvalMaps maps;
+      if (!maps.make(wg, nf32, w1 - w0, 2 * n_sites, nf)) {
+        cudaEventRecord(pipe->join[g], gs);
+        cudaStreamWaitEvent(st, pipe->join[g], 0);
+        return VMC_ERR_UNSUPPORTED;
+      }
       for (int s = 0; s < n_sweeps; ++s) {
         for (int e = 0; e < n_edges; ++e) {
           const int par = (s * n_edges + e) & 1;
@@ -1884,8 +1807,7 @@ int vmc_nnbf_sweep(int prec, const void* const* net_ptrs, int n_sites, int nf, i
                                                    (const float*)z0, nf32.w0t, prop_occ, (PropRec*)rec, H1, cn, cmap,
                                                    cprop, cx);
           int rc = launch_eval_rows(prec, w1 - w0, n_sites, nf, cn ? cprop + 2 * w0 : prop_occ + 2 * w0, net,
-                                    bf_scale, wg, d_err, gs, LD_ACCEPT, lg, /*allow_pipe=*/false,
-                                    /*concurrent=*/true, cn, cn ? cmap + w0 : nullptr);
+                                    bf_scale, wg, d_err, gs, LD_ACCEPT, lg, /*allow_pipe=*/false, cn, cn ? cmap + w0 : nullptr, &maps);
           if (rc) {
             // kernels already queued on this group's stream still write the
             // caller's buffers: the caller's stream waits for them all the same
@@ -1903,6 +1825,12 @@ int vmc_nnbf_sweep(int prec, const void* const* net_ptrs, int n_sites, int nf, i
     VMC_CUDA_CHECK_LAUNCH();
     return VMC_OK;
   }
+  // one stream: each kernel's placement overlaps the end of the one before it
+  // (an edge is four launches of 4 to 25 us: 548 walkers of 64 orbitals 5.88 ->
+  // 5.00 ms a sweep of 112 edges, 358 of 32 orbitals 1.96 -> 1.55 for 52)
+  const bool pdl = prec == 0 && !stage_ms && B <= kChunkRows;
+  EvalMaps maps;
+  if (prec == 0 && !maps.make(Work{H1, H2, A}, nf32, B, 2 * n_sites, nf)) return VMC_ERR_UNSUPPORTED;
   for (int s = 0; s < n_sweeps; ++s) {
     for (int e = 0; e < n_edges; ++e) {
       const int par = (s * n_edges + e) & 1;
@@ -1910,9 +1838,9 @@ int vmc_nnbf_sweep(int prec, const void* const* net_ptrs, int n_sites, int nf, i
       int* cx = ccnt ? ccnt + (par ^ 1) : nullptr;
       STAGE_BEGIN(0);
       if (prec == 0)
-        k_prep_sweep<float><<<gw, 256, 0, st>>>(B, 0, B, n_sites, occ, edges, e, s, n_edges, hopping_rate, seed,
-                                                sweep_offset + (uint64_t)s, r_move, r_bit, r_acc, (const float*)z0,
-                                                nf32.w0t, prop_occ, (PropRec*)rec, H1, cn, cmap, cprop, cx);
+        launch(pdl, k_prep_sweep<float>, gw, 256, 0, st, B, 0, B, n_sites, occ, edges, e, s, n_edges, hopping_rate,
+               seed, sweep_offset + (uint64_t)s, r_move, r_bit, r_acc, (const float*)z0, nf32.w0t, prop_occ,
+               (PropRec*)rec, H1, cn, cmap, cprop, cx);
       else
         k_prep_sweep<double><<<gw, 256, 0, st>>>(B, 0, B, n_sites, occ, edges, e, s, n_edges, hopping_rate, seed,
                                                  sweep_offset + (uint64_t)s, r_move, r_bit, r_acc,
@@ -1920,7 +1848,8 @@ int vmc_nnbf_sweep(int prec, const void* const* net_ptrs, int n_sites, int nf, i
                                                  nullptr, nullptr, nullptr);
       STAGE_END(0);
       int rc = launch_eval_rows(prec, B, n_sites, nf, cn ? cprop : prop_occ, net, bf_scale, Work{H1, H2, A}, d_err,
-                                st, LD_ACCEPT, la, true, false, cn, cn ? cmap : nullptr);
+                                st, LD_ACCEPT, la, true, cn, cn ? cmap : nullptr, prec == 0 ? &maps : nullptr,
+                                pdl);
       if (rc) { g_timer.acc = nullptr; return rc; }
     }
   }
@@ -2014,7 +1943,7 @@ int vmc_nnbf_local_energy(int prec, const void* const* net_ptrs, int n_sites, in
       la.sign = const_cast<double*>(sign);
       la.logabs = const_cast<double*>(logabs);
       int rc = launch_eval_rows(prec, R, n_sites, nf, ro, net, bf_scale, wg, d_err, gs, LD_ELOC, la,
-                                /*allow_pipe=*/false, /*concurrent=*/true);
+                                /*allow_pipe=*/false);
       if (rc) {
         // the caller's stream still waits for every kernel already queued on the lanes
         for (int h = 0; h < G; ++h) {
@@ -2136,14 +2065,14 @@ extern "C" int vmc_nnbf_hidden_layer(const void* H1, int64_t R, const void* W1, 
   if (R == 0) return VMC_OK;
   set_attrs();
   CUtensorMap tH1, tW1;
-  if (!tmap_bf16(&tH1, H1, (uint64_t)R, TM) || !tmap_bf16(&tW1, W1, HID, TN)) return VMC_ERR_UNSUPPORTED;
-  EpiArgs e1{};
+  if (!tmap_bf16(&tH1, H1, (uint64_t)R, TM) || !tmap_bf16(&tW1, W1, HID, HN)) return VMC_ERR_UNSUPPORTED;
+  HiddenArgs e1{};
   e1.bias = b1;
   e1.out = (__nv_bfloat16*)H2;
   e1.wait_ns = wait_limit_ns;
   e1.skip_loads = skip_loads ? 1 : 0;
-  dim3 g1((unsigned)((R + TM - 1) / TM), 1);
-  k_gemm_tc<EPI_GELU_BF16><<<g1, 128, GEMM_SMEM, (cudaStream_t)stream>>>(tH1, tW1, (int)R, e1, d_err);
+  dim3 g1((unsigned)((R + TM - 1) / TM), HID / HN);
+  k_hidden_tc<<<g1, 128, HIDDEN_SMEM, (cudaStream_t)stream>>>(tH1, tW1, (int)R, e1, d_err);
   VMC_CUDA_CHECK_LAUNCH();
   return VMC_OK;
 }

@@ -205,8 +205,8 @@ __global__ void __launch_bounds__(128) k_slater_refresh(
 // shared memory holds six 64-orbital walkers an SM: with two warps each they
 // load the four quarters evenly.  Both warps of a walker decide every proposal
 // for themselves (the acceptance ratio needs two to four products of length
-// nf) and meet only when one is accepted.  8192 walkers, nf = 64, 10 sweeps of
-// an 8x8 lattice with their refreshes: 4.84 ms with one warp a walker, 4.43 with two.
+// nf) and meet only when one is accepted.  4096 walkers, nf = 64, a step of
+// the 8x8 lattice with its refreshes: 4.84 ms with one warp a walker, 4.43 with two.
 template <int WPW>
 __global__ void k_slater_sweep(const double* __restrict__ M, int nf, int N, uint64_t* __restrict__ occ, int64_t B,
                                const int32_t* __restrict__ edges, int E, int n_sweeps, float hopping_rate,
