@@ -1803,6 +1803,11 @@ int vmc_nnbf_sweep(int prec, const void* const* net_ptrs, int n_sites, int nf, i
     if (cudaEventRecord(pipe->fork, st) != cudaSuccess) return VMC_ERR_CUDA;
     const int64_t Bg = (B + G - 1) / G;
     const size_t zrow = (size_t)HID * sizeof(float);
+    // launches of a group that overlap its own earlier ones: the CTAs that wait
+    // hold SM space, which other groups' LU tiles of 64 orbitals need (6000
+    // walkers 16.4 -> 18.2 ms) and those of 32 do not (10000 walkers 5.82 ->
+    // 5.45 ms, 5000 3.99 -> 3.47)
+    const bool lane_pdl = nf == 32;
     for (int g = 0; g < G; ++g) {
       const int64_t w0 = (int64_t)g * Bg, w1 = (w0 + Bg) < B ? (w0 + Bg) : B;
       if (w0 >= w1) continue;
@@ -1830,12 +1835,11 @@ int vmc_nnbf_sweep(int prec, const void* const* net_ptrs, int n_sites, int nf, i
           const int par = (s * n_edges + e) & 1;
           int* cn = ccnt ? ccnt + 2 * g + par : nullptr;
           int* cx = ccnt ? ccnt + 2 * g + (par ^ 1) : nullptr;
-          k_prep_sweep<float><<<gwg, 256, 0, gs>>>(B, w0, w1, n_sites, occ, edges, e, s, n_edges, hopping_rate, seed,
-                                                   sweep_offset + (uint64_t)s, r_move, r_bit, r_acc,
-                                                   (const float*)z0, nf32.w0t, prop_occ, (PropRec*)rec, H1, cn, cmap,
-                                                   cprop, cx);
+          launch(lane_pdl, k_prep_sweep<float>, gwg, 256, 0, gs, B, w0, w1, n_sites, occ, edges, e, s, n_edges,
+                 hopping_rate, seed, sweep_offset + (uint64_t)s, r_move, r_bit, r_acc, (const float*)z0, nf32.w0t,
+                 prop_occ, (PropRec*)rec, H1, cn, cmap, cprop, cx);
           int rc = launch_eval_rows(prec, w1 - w0, n_sites, nf, cn ? cprop + 2 * w0 : prop_occ + 2 * w0, net,
-                                    bf_scale, wg, d_err, gs, LD_ACCEPT, lg, /*allow_pipe=*/false, cn, cn ? cmap + w0 : nullptr, &maps);
+                                    bf_scale, wg, d_err, gs, LD_ACCEPT, lg, /*allow_pipe=*/false, cn, cn ? cmap + w0 : nullptr, &maps, lane_pdl);
           if (rc) {
             // kernels already queued on this group's stream still write the
             // caller's buffers: the caller's stream waits for them all the same
