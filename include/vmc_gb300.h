@@ -110,7 +110,8 @@ int vmc_slater_logpsi_grad(const double* G, const uint8_t* slot_orb, int64_t B, 
  *   [0] W0^T (2N, 256) f32/f64   [1] b0 (256) f32/f64   [2] W1 (256, 256) bf16/f64
  *   [3] b1 (256) f32/f64          [4] out_w (2N*nf, 256) bf16/f64
  *   [5] out_b (2N*nf) f32/f64     [6] M_base (2N, nf) f32/f64
- * Workspace for R rows (caller-owned): H1, H2 (R, 256) bf16/f64; A (R, nf, nf) f32/f64.
+ * Workspace for R rows (caller-owned): H1, H2 (R, 256) bf16/f64; A (R, nf, nf) f32/f64
+ * (scratch; the FP32 matrices are kept in blocks of 8 columns).
  * The workspace is scratch: its contents on return are unspecified (the LU
  * reuses consumed orbital-matrix rows).
  * d_err (device int) receives VMC_ERR_TIMEOUT if a bounded device wait gave up,
