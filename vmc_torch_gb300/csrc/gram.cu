@@ -17,8 +17,14 @@
 // accumulates in its own TMEM accumulator with no rounding at all.  The eight
 // small terms (2^-7 of it and below) share a second accumulator, where FP32
 // rounding is ~2^-25 of 2^-7 of the result.
-// Both are drained into the FP64 result every 2048 columns of K, scaled by
-// 2^(E_i + E_j).
+// Both are drained every 2048 columns of K into a running sum of each output,
+// two FP32 numbers in registers (exact error terms, ~2^-48 of the sum): an FP64
+// instruction holds a warp's scheduler for 64 clocks, and the drain into FP64 T
+// with its conversions, exponents and scattered read-modify-writes took as
+// long as the chunk's products (8192 samples, 2.2 million parameters in
+// Kronecker factors, with the split below: 112.7 -> 89.4 ms the solve).  The FP64 result, scaled by
+// 2^(E_i + E_j), is formed once a tile and goes through shared memory so that
+// T and D are read and written along their rows.
 //
 // Tile: 128 x 128 outputs per CTA, lower triangle of tiles only (the upper
 // triangle is written as the mirror image).  K atoms of 64 BF16 (128 bytes per
@@ -26,7 +32,7 @@
 // holds the three planes of the 128 rows of both operands (96 KB).  Warp 0
 // issues the copies, warp 1 (one thread) the tcgen05 MMAs into two TMEM
 // buffers used alternately per K chunk (each 2 x 128 columns: leading and
-// small products), warps 2..5 add each finished chunk into T.
+// small products), warps 2..9 (two a TMEM lane quadrant) hold the running sums.
 #include <cuda.h>
 #include <cudaTypedefs.h>
 #include <cuda_bf16.h>
@@ -41,44 +47,78 @@ constexpr int PLANE = GT * KA * 2;            // 16 KB: one plane of one operand
 constexpr int STAGE = 6 * PLANE;              // A hi/mid/lo + B hi/mid/lo
 constexpr int NSTAGE = 2;
 constexpr int CHUNK_ATOMS = 32;               // 2048 columns of K per FP32 accumulation
-constexpr int GR_THREADS = 192;
+constexpr int GR_THREADS = 320;
+constexpr int EC = GT / 2;                    // columns per epilogue warp
 constexpr int GR_SMEM = NSTAGE * STAGE + 1024 + 256;
 
 // Row exponents: E[r] = ilogb(max_k |X[r][k]|) + 1 (0 for a zero row or a
-// padding row), one warp per row.
-__global__ void k_row_exp(const float* __restrict__ X, int64_t rows, int64_t rows_pad, int64_t K, int64_t ldx,
-                          int* __restrict__ E) {
-  const int64_t r = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  const int lane = threadIdx.x & 31;
-  if (r >= rows_pad) return;
+// padding row), one CTA per row; eight loads a thread in flight.
+__global__ void __launch_bounds__(256) k_row_exp(const float* __restrict__ X, int64_t rows, int64_t K, int64_t ldx,
+                                                 int* __restrict__ E) {
+  __shared__ unsigned wmax[8];
+  const int64_t r = blockIdx.x;
+  const float* x = X + r * ldx;
   float m = 0.f;
-  if (r < rows)
-    for (int64_t c = lane; c < K; c += 32) m = fmaxf(m, fabsf(X[r * ldx + c]));
+  if (r < rows) {
+    int64_t c = threadIdx.x;
+    for (; c + 7 * 256 < K; c += 8 * 256) {
+      float v[8];
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(VMC_FULL_MASK, m, o));
-  if (lane == 0) E[r] = (m > 0.f && m < INFINITY) ? ilogbf(m) + 1 : 0;
+      for (int u = 0; u < 8; ++u) v[u] = x[c + u * 256];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) m = fmaxf(m, fabsf(v[u]));
+    }
+    for (; c < K; c += 256) m = fmaxf(m, fabsf(x[c]));
+  }
+  const unsigned b = __reduce_max_sync(VMC_FULL_MASK, __float_as_uint(m));   // m >= 0: ordered as its bits
+  if ((threadIdx.x & 31) == 0) wmax[threadIdx.x >> 5] = b;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    unsigned t = wmax[0];
+#pragma unroll
+    for (int w = 1; w < 8; ++w) t = max(t, wmax[w]);
+    m = __uint_as_float(t);
+    E[r] = (m > 0.f && m < INFINITY) ? ilogbf(m) + 1 : 0;
+  }
 }
 
 // x -> (hi, mid, lo) planes of the fixed-point digits of x 2^-E[r] (plane p at
 // P + p * plane), row-major with row stride kp; rows >= `rows` and columns >=
 // K are zero.  Every step below is exact in FP32: scaling by powers of two,
 // rounding to an integer, and the subtraction of that integer from a value
-// within 0.5 of it.
-__global__ void k_split3(const float* __restrict__ X, int64_t rows, int64_t rows_pad, int64_t K, int64_t ldx,
-                         int64_t kp, const int* __restrict__ E, __nv_bfloat16* __restrict__ P) {
-  const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= rows_pad * kp) return;
-  const int64_t r = idx / kp, c = idx - r * kp;
-  const float x = (r < rows && c < K) ? X[r * ldx + c] : 0.f;
-  const float y = ldexpf(x, 6 - E[r]);       // 2^6 x 2^-E, |y| < 64
-  const float a0 = rintf(y);
-  const float r1 = (y - a0) * 128.f;         // |r1| <= 64
-  const float a1 = rintf(r1);
-  const float a2 = rintf((r1 - a1) * 128.f);
-  const int64_t plane = rows_pad * kp;
-  P[idx] = __float2bfloat16_rn(ldexpf(a0, -6));
-  P[plane + idx] = __float2bfloat16_rn(ldexpf(a1, -13));
-  P[2 * plane + idx] = __float2bfloat16_rn(ldexpf(a2, -20));
+// within 0.5 of it.  HBM is the limit (10 bytes an entry): SPLIT_CU columns a
+// thread in flight, a row's blocks along x and the rows along y and z.
+constexpr int SPLIT_CU = 8;
+
+__global__ void __launch_bounds__(256) k_split3(const float* __restrict__ X, int64_t rows, int64_t rows_pad, int64_t K,
+                                                int64_t ldx, int64_t kp, const int* __restrict__ E,
+                                                __nv_bfloat16* __restrict__ P) {
+  const int64_t r = (int64_t)blockIdx.z * 65535 + blockIdx.y;
+  if (r >= rows_pad) return;
+  // 2^6 x 2^-E in two factors: 2^(6 - E) itself may lie outside FP32
+  const int k = 6 - E[r], k1 = k >> 1;
+  const float s1 = __int_as_float((127 + k1) << 23), s2 = __int_as_float((127 + k - k1) << 23);
+  const int64_t c0 = (int64_t)blockIdx.x * (256 * SPLIT_CU) + threadIdx.x, plane = rows_pad * kp;
+  float x[SPLIT_CU];
+#pragma unroll
+  for (int u = 0; u < SPLIT_CU; ++u) {
+    const int64_t c = c0 + u * 256;
+    x[u] = (r < rows && c < K) ? X[r * ldx + c] : 0.f;
+  }
+  __nv_bfloat16* p = P + r * kp;
+#pragma unroll
+  for (int u = 0; u < SPLIT_CU; ++u) {
+    const int64_t c = c0 + u * 256;
+    if (c >= kp) return;
+    const float y = x[u] * s1 * s2;            // |y| < 64
+    const float a0 = rintf(y);
+    const float r1 = (y - a0) * 128.f;         // |r1| <= 64
+    const float a1 = rintf(r1);
+    const float a2 = rintf((r1 - a1) * 128.f);
+    p[c] = __float2bfloat16_rn(a0 * 0x1p-6f);
+    p[plane + c] = __float2bfloat16_rn(a1 * 0x1p-13f);
+    p[2 * plane + c] = __float2bfloat16_rn(a2 * 0x1p-20f);
+  }
 }
 
 struct GramArgs {
@@ -101,6 +141,21 @@ __device__ __forceinline__ void tile_of(int t, int& bi, int& bj) {
   bj = t - i * (i + 1) / 2;
 }
 
+// a + b rounded into a, the rounding error returned
+__device__ __forceinline__ float two_sum(float& a, float b) {
+  const float s = __fadd_rn(a, b), bb = __fsub_rn(s, a);
+  const float e = __fadd_rn(__fsub_rn(a, __fsub_rn(s, bb)), __fsub_rn(b, bb));
+  a = s;
+  return e;
+}
+
+// t 2^e in the exponent field: t is 0, not finite, or of an exponent between
+// FP32's least and 2^31, and |e| < 300
+__device__ __forceinline__ double scale2(double t, int e) {
+  const int h = __double2hiint(t), f = (h >> 20) & 0x7ff;
+  return f == 0 || f == 0x7ff ? t : __hiloint2double(h + (e << 20), __double2loint(t));
+}
+
 __global__ void __launch_bounds__(GR_THREADS, 1)
     k_gram_bf16x3(const __grid_constant__ CUtensorMap tmX, GramArgs ga, int* __restrict__ err) {
   extern __shared__ uint8_t smem_raw[];
@@ -118,7 +173,7 @@ __global__ void __launch_bounds__(GR_THREADS, 1)
   const int n_chunks = (ga.n_atoms + CHUNK_ATOMS - 1) / CHUNK_ATOMS;
   if (threadIdx.x == 0) {
     for (int s = 0; s < NSTAGE; ++s) { tc::mbar_init(&full[s], 1); tc::mbar_init(&empty[s], 1); }
-    for (int b = 0; b < 2; ++b) { tc::mbar_init(&tfull[b], 1); tc::mbar_init(&tempty[b], 4); }
+    for (int b = 0; b < 2; ++b) { tc::mbar_init(&tfull[b], 1); tc::mbar_init(&tempty[b], 8); }
     *abort_flag = 0;
     tc::fence_mbar_init();
     tc::prefetch_tmap(&tmX);
@@ -184,42 +239,77 @@ __global__ void __launch_bounds__(GR_THREADS, 1)
         tc::mma_commit(&tfull[buf]);
       }
     }
-  } else {  // ---- epilogue: warps 2..5, TMEM lane quadrant warp % 4 ----
-    const int quad = warp & 3;
-    const int r = quad * 32 + lane;          // row of the tile
-    const int64_t gi = (int64_t)bi * GT + r;
-    const bool live = gi < ga.n;
+  } else {  // ---- epilogue: warps 2..9, TMEM lane quadrant warp % 4, half of the columns each ----
+    const int quad = warp & 3, half = (warp - 2) >> 2;
+    float hi[EC], lo[EC];
+#pragma unroll
+    for (int q = 0; q < EC; ++q) hi[q] = lo[q] = 0.f;
+    bool ok = true;
     for (int c = 0; c < n_chunks; ++c) {
       const int buf = c & 1;
-      bool ok = tc::mbar_wait(&tfull[buf], (c >> 1) & 1);
+      ok = tc::mbar_wait(&tfull[buf], (c >> 1) & 1);
       ok = __all_sync(VMC_FULL_MASK, ok);
       if (!ok) { if (lane == 0) { *abort_flag = 1; atomicExch(err, VMC_ERR_TIMEOUT); } break; }
       tc::fence_after_sync();
-      const bool first = (c == 0) && !ga.accumulate;
-      const bool last = c == n_chunks - 1;
-#pragma unroll 1
-      for (int cc = 0; cc < GT / 32; ++cc) {
-        float v[32], w[32];
-        const uint32_t ta = tbase + (uint32_t)(buf * 2 * GT) + ((uint32_t)(quad * 32) << 16) + (uint32_t)(cc * 32);
-        tc::tmem_ld32(ta, v);
-        tc::tmem_ld32(ta + GT, w);
-        if (!live) continue;
+      const uint32_t ta = tbase + (uint32_t)(buf * 2 * GT + half * EC) + ((uint32_t)(quad * 32) << 16);
 #pragma unroll
-        for (int q = 0; q < 32; ++q) {
-          const int64_t gj = (int64_t)bj * GT + cc * 32 + q;
-          if (gj >= ga.n || (bi == bj && gj > gi)) continue;
-          double* t = ga.T + gi * ga.ldt + gj;
-          double add = ga.alpha * ldexp((double)v[q] + (double)w[q], ga.E[gi] + ga.E[gj]);
-          if (ga.D) add *= ga.D[gi * ga.ldt + gj];
-          double val = first ? add : *t + add;
-          if (last && gj == gi) val += ga.shift;
-          *t = val;
-          if (last && gj != gi) ga.T[gj * ga.ldt + gi] = val;
+      for (int g = 0; g < EC / 8; ++g) {
+        float v[8], w[8];
+        tc::tmem_ld8x2(ta + (uint32_t)(g * 8), GT, v, w);
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+          float h = hi[g * 8 + q];
+          const float e = two_sum(h, v[q]), f = two_sum(h, w[q]);
+          hi[g * 8 + q] = h;
+          lo[g * 8 + q] += e + f;
         }
       }
       tc::fence_before_sync();
       __syncwarp();
       if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(tc::smem_u32(&tempty[buf])) : "memory");
+    }
+    if (ok) {
+      // the loads and MMAs of the tile are complete: their stages become the
+      // warps' transpose buffers
+      double* tb = reinterpret_cast<double*>(sm) + (warp - 2) * (32 * (EC + 1));
+      const int r0 = bi * GT + quad * 32, c0 = bj * GT + half * EC;
+      const int gi = r0 + lane;
+      const int ej[2] = {ga.E[c0 + lane], ga.E[c0 + 32 + lane]};   // padding rows have one too
+#pragma unroll
+      for (int q = 0; q < EC; ++q) reinterpret_cast<float2*>(tb)[lane * (EC + 1) + q] = make_float2(hi[q], lo[q]);
+      __syncwarp();
+#pragma unroll 1
+      for (int rb = 0; rb < 32; rb += 4) {   // four rows of T and D in flight at a time
+        double t[4][2], d[4][2];
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            const int64_t row = r0 + rb + u, col = c0 + 32 * h + lane;
+            const bool in = row < ga.n && col <= row;
+            t[u][h] = in && ga.accumulate ? ga.T[row * ga.ldt + col] : 0.0;
+            d[u][h] = in && ga.D ? ga.D[row * ga.ldt + col] : 1.0;
+          }
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            const int64_t row = r0 + rb + u, col = c0 + 32 * h + lane;
+            double* b = &tb[(rb + u) * (EC + 1) + 32 * h + lane];
+            const float2 x = *reinterpret_cast<const float2*>(b);
+            double val = ga.alpha * scale2((double)x.x + (double)x.y, ga.E[row] + ej[h]);
+            if (ga.D) val *= d[u][h];
+            if (ga.accumulate) val += t[u][h];
+            if (row == col) val += ga.shift;
+            if (row < ga.n && col <= row) ga.T[row * ga.ldt + col] = val;
+            *b = val;
+          }
+      }
+      __syncwarp();
+      for (int q = 0; q < EC; ++q) {     // along the rows of the mirror image
+        const int64_t gj = c0 + q;
+        if (gi < ga.n && gj < gi) ga.T[gj * ga.ldt + gi] = tb[lane * (EC + 1) + q];
+      }
     }
   }
   tc::fence_before_sync();
@@ -265,11 +355,13 @@ int vmc_split_bf16x3(const float* X, int64_t rows, int64_t K, int64_t ldx, void*
       (rows > 0 && (!X || !planes)) || (rows_pad > 0 && !row_exp))
     return VMC_ERR_ARGS;
   if (rows_pad == 0) return VMC_OK;
-  k_row_exp<<<(unsigned)((rows_pad + 7) / 8), 256, 0, (cudaStream_t)stream>>>(X, rows, rows_pad, K, ldx, row_exp);
+  if (rows_pad > INT32_MAX) return VMC_ERR_ARGS;
+  k_row_exp<<<(unsigned)rows_pad, 256, 0, (cudaStream_t)stream>>>(X, rows, K, ldx, row_exp);
   VMC_CUDA_CHECK_LAUNCH();
-  const int64_t n = rows_pad * kp;
-  k_split3<<<(unsigned)((n + 255) / 256), 256, 0, (cudaStream_t)stream>>>(X, rows, rows_pad, K, ldx, kp, row_exp,
-                                                                          (__nv_bfloat16*)planes);
+  if (kp == 0) return VMC_OK;
+  const dim3 grid((unsigned)((kp + 256 * SPLIT_CU - 1) / (256 * SPLIT_CU)), (unsigned)(rows_pad < 65535 ? rows_pad : 65535),
+                  (unsigned)((rows_pad + 65534) / 65535));
+  k_split3<<<grid, 256, 0, (cudaStream_t)stream>>>(X, rows, rows_pad, K, ldx, kp, row_exp, (__nv_bfloat16*)planes);
   VMC_CUDA_CHECK_LAUNCH();
   return VMC_OK;
 }

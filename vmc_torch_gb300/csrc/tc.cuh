@@ -133,6 +133,25 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float* v) {
   for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
 }
 
+// Two groups of 32 lanes x 8 columns, `step` columns apart, read in flight together.
+__device__ __forceinline__ void tmem_ld8x2(uint32_t taddr, uint32_t step, float (&v)[8], float (&w)[8]) {
+  uint32_t r[16];
+  asm volatile(
+      "{\n .reg .b32 a;\n"
+      " add.u32 a, %16, %17;\n"
+      " tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%16];\n"
+      " tcgen05.ld.sync.aligned.32x32b.x8.b32 {%8,%9,%10,%11,%12,%13,%14,%15}, [a];\n"
+      " tcgen05.wait::ld.sync.aligned;\n}\n"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+        "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr), "r"(step));
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    v[i] = __uint_as_float(r[i]);
+    w[i] = __uint_as_float(r[8 + i]);
+  }
+}
+
 // Seven groups of 32 lanes x 8 columns, `step` columns apart (one group per
 // digit level of the fixed-point products), read in flight together.
 __device__ __forceinline__ void tmem_ld8x7(uint32_t taddr, uint32_t step, uint32_t (&r)[7][8]) {
