@@ -146,7 +146,7 @@ __device__ __forceinline__ void column_sums(int64_t Ns, double (*part)[NC * 32],
 // own error (below 2^-43 of the entry and of the scaled mean) could change takes
 // the FP64 expression, so that the result is always that expression rounded:
 // about one entry in 10^5, tested for 16 entries at once (8192 samples, 115 K
-// columns: below 1 ms of 90; the FP64 expression throughout took 6 ms more).
+// columns: below 1 ms of a solve of 90).
 template <typename T, int NC>
 __global__ void __launch_bounds__(32 * CW) k_center(const T* __restrict__ O, int64_t Ns, int64_t Np, int64_t ldo,
                                                     T* __restrict__ Oc, int64_t ldc, double* __restrict__ mean,
