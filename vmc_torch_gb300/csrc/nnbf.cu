@@ -248,6 +248,8 @@ __global__ void k_prep_conn(int64_t P, int N, const int32_t* __restrict__ pairs 
                             const uint64_t* __restrict__ occ, const int32_t* __restrict__ edges, double t,
                             const T* __restrict__ z0, const T* __restrict__ w0t, uint64_t* __restrict__ row_occ,
                             double* __restrict__ coeff, void* __restrict__ H1) {
+  pdl_trigger();
+  pdl_wait();
   const int lane = threadIdx.x & 31;
   const int64_t p = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (p >= P) return;
@@ -1961,6 +1963,13 @@ int vmc_nnbf_local_energy(int prec, const void* const* net_ptrs, int n_sites, in
   }
   if (G > 1) {
     const int64_t sub = chunk / G;
+    // overlapping launches inside a lane for 32 orbitals, as in vmc_nnbf_sweep
+    const bool lane_pdl = nf == 32;
+    EvalMaps maps[ChunkPipe::kLanes];
+    for (int g = 0; g < G; ++g) {
+      const Work wg{(char*)H1 + (size_t)g * sub * HID * 2, (char*)H2 + (size_t)g * sub * HID * 2, nullptr};
+      if (!maps[g].make(wg, nf32, sub, 2 * n_sites, nf)) return VMC_ERR_UNSUPPORTED;
+    }
     if (cudaEventRecord(pipe->fork, st) != cudaSuccess) return VMC_ERR_CUDA;
     for (int g = 0; g < G; ++g)
       if (cudaStreamWaitEvent(pipe->lane[g], pipe->fork, 0) != cudaSuccess) return VMC_ERR_CUDA;
@@ -1973,8 +1982,8 @@ int vmc_nnbf_local_energy(int prec, const void* const* net_ptrs, int n_sites, in
       double* co = coeff + (size_t)g * sub;
       const Work wg{(char*)H1 + (size_t)g * sub * HID * 2, (char*)H2 + (size_t)g * sub * HID * 2,
                     (float*)A + (size_t)g * sub * nf * nf};
-      k_prep_conn<float><<<(unsigned)((R * 32 + 255) / 256), 256, 0, gs>>>(
-          R, n_sites, pairs + 2 * p0, occ, edges, t, (const float*)z0, nf32.w0t, ro, co, wg.H1);
+      launch(lane_pdl, k_prep_conn<float>, (unsigned)((R * 32 + 255) / 256), 256, 0, gs, R, n_sites, pairs + 2 * p0,
+             occ, edges, t, (const float*)z0, nf32.w0t, ro, co, wg.H1);
       LdArgs la{};
       la.pairs = pairs + 2 * p0;
       la.coeff = co;
@@ -1982,7 +1991,7 @@ int vmc_nnbf_local_energy(int prec, const void* const* net_ptrs, int n_sites, in
       la.sign = const_cast<double*>(sign);
       la.logabs = const_cast<double*>(logabs);
       int rc = launch_eval_rows(prec, R, n_sites, nf, ro, net, bf_scale, wg, d_err, gs, LD_ELOC, la,
-                                /*allow_pipe=*/false);
+                                /*allow_pipe=*/false, nullptr, nullptr, &maps[g], lane_pdl);
       if (rc) {
         // the caller's stream still waits for every kernel already queued on the lanes
         for (int h = 0; h < G; ++h) {
