@@ -335,8 +335,8 @@ int vmc_sr_cholesky_tc(double* T, int64_t n, int64_t ldt, int* d_info, void* wor
  *   with D (nullable, ld ldt) elementwise and `accumulate` selecting "+=";
  *   all nine digit products per element pair on tcgen05: the leading one summed
  *   exactly in FP32 (integer multiples of 2^-12, < 2^23 units per 2048
- *   columns), the others in a second FP32 accumulator; drained into FP64 every
- *   2048 columns and scaled by 2^(E_i + E_j); the full symmetric T is written.
+ *   columns), the others in a second FP32 accumulator; added every 2048 columns
+ *   into pairs of FP32 numbers (~2^-48), scaled by 2^(E_i + E_j) in FP64 at the end; the full symmetric T is written.
  *   d_err (device int) receives VMC_ERR_TIMEOUT if a bounded wait gave up. */
 int vmc_split_bf16x3(const float* X, int64_t rows, int64_t K, int64_t ldx, void* planes, int64_t rows_pad,
                      int64_t kp, int* row_exp, void* stream);

@@ -610,10 +610,10 @@ CholWork chol_work(int64_t n, void* base) {
 // panel solve 5 to 40) and the trailing update behind it fills the GPU.  The
 // chain runs on a stream of high priority: of a panel's update it waits for the
 // next panel's 256 columns only, and factors those while the caller's stream
-// updates the rest.  Order 8192: 28.2 -> 24.4 ms,
-// 4096: 8.72 -> 8.45, 3000: 5.78 -> 5.58, 2049: no difference.  Not under stream capture: the stream
-// and events are shared by the calls of all threads, one at a time under
-// g_look_mu, and a capture would hold them beyond the call.
+// updates the rest.  Order 8192: 28.2 -> 24.4 ms, 4096: 8.72 -> 8.45, 3000:
+// 5.78 -> 5.58, 2049: no difference.  Not under stream capture: the stream and
+// events are shared by the calls of all threads, one at a time under g_look_mu,
+// and a capture would hold them beyond the call.
 constexpr int64_t LOOK_MIN = 2560;
 struct Lookahead {
   cudaStream_t chain = nullptr;

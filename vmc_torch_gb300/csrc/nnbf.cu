@@ -9,7 +9,7 @@
 // energy, or a walker's current configuration on refresh):
 //   prep      : z0(row) from the walker's z0 plus the moved orbitals' W0
 //               columns (or from scratch), h1 = gelu(z0) -> H1 (bf16 / fp64)
-//   layer1    : H2 = gelu(H1 W1^T + b1)            tcgen05 GEMM 128x256x256
+//   layer1    : H2 = gelu(H1 W1^T + b1)            tcgen05 GEMM 128x64x256
 //   backflow  : A[row][pos] = M_base[r] + s (H2 out_w[r]^T + out_b[r]) for each
 //               occupied orbital r at ascending position pos
 //                                                   tcgen05 GEMM 128x256x256,
@@ -33,7 +33,7 @@ using namespace vmc;
 
 namespace {
 
-// Programmatic dependent launch (single-stream sweeps): a kernel lets its
+// Programmatic dependent launch (single-stream sweeps, lanes of 32 orbitals): a kernel lets its
 // successor's CTAs be placed as soon as its own have started, and waits for
 // its predecessor's completion before it touches anything that one writes.  Both
 // are no-ops in a launch without the attribute.

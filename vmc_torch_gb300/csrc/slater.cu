@@ -1,4 +1,4 @@
-// Slater-determinant walkers: one warp per walker.
+// Slater-determinant walkers: one or two warps per walker.
 //
 // Per-walker state (global memory, owned by the caller):
 //   occ[2]          packed up / down bits

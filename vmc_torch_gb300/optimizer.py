@@ -137,7 +137,7 @@ class MinSRGB300(PreconditionerGB300):
         tensor cores (vmc_sr_gram_tc: each row split
         into three 7-bit fixed-point digits under a shared power-of-two
         exponent, all nine digit products, the leading one summed exactly in
-        FP32, drained into FP64 every 2048 columns): the Gram matrix of the
+        FP32, added into pairs of FP32 numbers every 2048 columns): the Gram matrix of the
         rows rounded to 2^-20 of their largest entry, positive semidefinite
         up to ~2^-32 rounding.  "cuda" forms them on the CUDA cores with
         compensated (double-float) accumulation: the exact Gram of the FP32
