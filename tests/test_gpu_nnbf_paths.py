@@ -107,3 +107,30 @@ def test_sweep_does_not_depend_on_the_batch(Lx, Ly, nf, B):
     for x, first, last in zip(*out):
         assert torch.equal(x[:b], first)
         assert torch.equal(x[B - b:], last)
+
+
+@pytest.mark.parametrize("Lx,Ly,nf", [(8, 8, 64), (6, 6, 32)])
+@pytest.mark.parametrize("B", [257, 4096])
+def test_captured_sweep_equals_eager(Lx, Ly, nf, B):
+    """One stream of overlapping launches (257) and walker groups (4096) keep
+    their order in a CUDA graph."""
+    N = Lx * Ly
+    m = model(om.nnbf_init(N, nf, 256, 2, seed=9), N, nf)
+    g = vg.SquareLattice(Lx, Ly)
+    x0 = vg.init_walkers(B, N, nf // 2, nf // 2, seed=B, device=DEV)
+    with torch.inference_mode():   # as the sampler runs it
+        st = m.bind_state(x0)
+        occ0 = st.occ.clone()
+        m.sweep(st, g, 1, 11, 0)
+        torch.cuda.synchronize()
+        want = [t.clone() for t in (st.occ, st.sign, st.logabs, st.n_acc)]
+        assert not torch.equal(st.occ, occ0)
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            m.sweep(st, g, 1, 11, 0)
+        for _ in range(2):
+            st.occ.copy_(occ0)
+            graph.replay()
+            torch.cuda.synchronize()
+            for a, b in zip(want, (st.occ, st.sign, st.logabs, st.n_acc)):
+                assert torch.equal(a, b)
