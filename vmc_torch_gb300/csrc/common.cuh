@@ -129,6 +129,27 @@ __device__ __forceinline__ double rcp_pos(double d) {
   return fma(y, fma(t, t, t), y);
 }
 
+// s + x rounded into s, the rounding error returned (Knuth's TwoSum).  The
+// intrinsics keep a product that x came from out of the additions: contracted
+// into one of them it would leave an error that is neither.
+__device__ __forceinline__ float two_sum(float& s, float x) {
+  const float t = __fadd_rn(s, x), bb = __fsub_rn(t, s);
+  const float e = __fadd_rn(__fsub_rn(s, __fsub_rn(t, bb)), __fsub_rn(x, bb));
+  s = t;
+  return e;
+}
+
+// A sum of FP32 numbers in three FP32 words, s exact with its rounding errors
+// in c, those of c in d: ~2^-58 of the largest partial sum after 10^4 terms,
+// where a chain of FP64 additions has ~2^-47 (an FP64 instruction costs a warp
+// 64 clocks on GB300).
+struct Sum3 {
+  float s = 0.f, c = 0.f, d = 0.f;
+  __device__ __forceinline__ void low(float x) { d = __fadd_rn(d, two_sum(c, x)); }   // x below 2^-22 of the terms
+  __device__ __forceinline__ void add(float x) { low(two_sum(s, x)); }
+  __device__ __forceinline__ double value() const { return (double)s + ((double)c + (double)d); }
+};
+
 }  // namespace vmc
 
 #define VMC_CUDA_CHECK_LAUNCH()                                   \

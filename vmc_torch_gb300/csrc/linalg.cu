@@ -55,50 +55,50 @@ struct TileAcc {
 // consecutive bytes of an FP32 row, which HBM pages want (one 128-byte piece a
 // row read 8192 x 115200 in 4.3 ms of centring); NC = 1 where that would leave
 // fewer CTAs than the GPU holds.  An FP64 instruction costs a warp 64 clocks
-// on GB300, so FP32 inputs are summed as double-float pairs (Knuth's TwoSum,
-// ~2^-47 of the running sum) that are added to the FP64 sum every 16 / NC rows.
+// on GB300, so FP32 inputs are summed in three FP32 words (Sum3), which become
+// one FP64 number at the end; rows whose terms leave the range in which that
+// is finer than FP64 sums are added in FP64.
 // 8192 x 115200 FP32: centring 10.7 and O~^T x 3.6 ms before; three
 // respectively one passes over 3.8 GB take 1.7 and 0.6 at the measured rate.
 constexpr int CW = 8;                    // warps a CTA
 constexpr int CB = 128;                  // rows a block of the loops below
 constexpr int64_t CWIDE = 128 * 304;     // columns from which NC = 4
 
-// s + x as s' + error
-__device__ __forceinline__ float two_sum(float& s, float x) {
-  const float t = s + x, bb = t - s;
-  const float e = (s - (t - bb)) + (x - bb);
-  s = t;
-  return e;
-}
+// Terms of a group of rows are summed in FP32 words while the largest lies in
+// [2^-85, 2^96): sums of 2^28 rows stay below FP32's largest number, and what
+// the parts of a product lose below FP32's least (2^-149 each) stays below
+// 2^-60 of that term.
+constexpr unsigned TERM_LO = (127u - 85u) << 23, TERM_HI = (127u + 96u) << 23;
 
-// x = h + l to 2^-48 of x, through the bit patterns where h and l are normal
-// floats (no FP64 instruction)
-__device__ __forceinline__ void split_f64(double x, float& h, float& l) {
+// x = h + m + l exactly, 24 + 24 + 5 bits, for |x| in [2^-70, 2^70) or 0: the
+// parts are normal floats or 0.  False for any other x.
+__device__ __forceinline__ bool split_f64(double x, float& h, float& m, float& l) {
   const int hi = __double2hiint(x);
-  const unsigned lo = (unsigned)__double2loint(x);
+  const unsigned lo = (unsigned)__double2loint(x), sg = (unsigned)hi & 0x80000000u;
   const int e = ((hi >> 20) & 0x7ff) - 1023;
-  if (e > -70 && e < 120) {
-    h = __uint_as_float((unsigned)(hi & 0x80000000) | (unsigned)((e + 127) << 23) | ((unsigned)(hi & 0xfffff) << 3) |
-                        (lo >> 29));
-    l = (float)(lo & 0x1fffffffu) * __uint_as_float((unsigned)(hi & 0x80000000) | (unsigned)((e - 52 + 127) << 23));
-  } else {
-    h = (float)x;
-    l = (float)(x - (double)h);
-  }
+  h = m = l = 0.f;
+  if (e < -70 || e >= 70) return x == 0.0;
+  h = __uint_as_float(sg | (unsigned)(e + 127) << 23 | ((unsigned)(hi & 0xfffff) << 3) | (lo >> 29));
+  m = __uint2float_rn((lo >> 5) & 0xffffffu) * __uint_as_float(sg | (unsigned)(e - 47 + 127) << 23);
+  l = __uint2float_rn(lo & 31u) * __uint_as_float(sg | (unsigned)(e - 52 + 127) << 23);
+  return true;
 }
 
 // Sums over all rows of the lane's NC columns, in every warp.  load(i, j): the
-// value at row i, column group j; pair(i - i0, x, h, l): its term as h + l (FP32
-// inputs); begin(i0) is called by all threads before the rows [i0, i0 + CB).
-template <typename T, int NC, typename B, typename L, typename P>
+// value at row i, column group j; begin(i0), called by all threads before the
+// rows [i0, i0 + CB): whether they may be summed in FP32 words; add(S, i - i0,
+// x): adds x's term to S and returns its leading part (FP32 inputs; LOW: terms
+// below TERM_LO are inexact); term(i - i0, x): the term in FP64.
+template <typename T, int NC, bool LOW, typename B, typename L, typename A, typename F>
 __device__ __forceinline__ void column_sums(int64_t Ns, double (*part)[NC * 32], double (&sum)[NC], B begin, L load,
-                                            P pair) {
+                                            A add, F term) {
   constexpr int CU = 16 / NC;            // rows in flight
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  vmc::Sum3 acc[NC];
 #pragma unroll
   for (int j = 0; j < NC; ++j) sum[j] = 0.0;
   for (int64_t i0 = 0; i0 < Ns; i0 += CB) {
-    begin(i0);
+    const bool words = begin(i0);
 #pragma unroll 1
     for (int u0 = 0; u0 < CB / CW; u0 += CU) {
       T x[CU][NC];
@@ -111,26 +111,29 @@ __device__ __forceinline__ void column_sums(int64_t Ns, double (*part)[NC * 32],
         }
 #pragma unroll
       for (int j = 0; j < NC; ++j) {
+        bool f64 = true;
         if constexpr (sizeof(T) == 4) {
-          float s = 0.f, c = 0.f;
+          if (words) {
+            const vmc::Sum3 was = acc[j];
+            unsigned mx = 0;
 #pragma unroll
-          for (int u = 0; u < CU; ++u) {
-            float h, l;
-            pair((u0 + u) * CW + warp, x[u][j], h, l);
-            if (u == 0) { s = h; c = l; }
-            else c += two_sum(s, h) + l;
+            for (int u = 0; u < CU; ++u)
+              mx = max(mx, __float_as_uint(add(acc[j], (u0 + u) * CW + warp, x[u][j])) & 0x7fffffffu);
+            f64 = mx >= TERM_HI;
+            if (LOW && mx < TERM_LO)
+#pragma unroll
+              for (int u = 0; u < CU; ++u) f64 |= x[u][j] != T(0);   // all zero: nothing is lost
+            if (f64) acc[j] = was;
           }
-          sum[j] += (double)s;
-          sum[j] += (double)c;
-        } else {
-#pragma unroll
-          for (int u = 0; u < CU; ++u) sum[j] += pair((u0 + u) * CW + warp, x[u][j]);
         }
+        if (f64)
+#pragma unroll
+          for (int u = 0; u < CU; ++u) sum[j] += term((u0 + u) * CW + warp, x[u][j]);
       }
     }
   }
 #pragma unroll
-  for (int j = 0; j < NC; ++j) part[warp][j * 32 + lane] = sum[j];
+  for (int j = 0; j < NC; ++j) part[warp][j * 32 + lane] = sizeof(T) == 4 ? sum[j] + acc[j].value() : sum[j];
   __syncthreads();
 #pragma unroll
   for (int j = 0; j < NC; ++j) {
@@ -161,10 +164,13 @@ __global__ void __launch_bounds__(32 * CW) k_center(const T* __restrict__ O, int
   for (int j = 0; j < NC; ++j) off[j] = p0 + 32 * j < Np ? p0 + 32 * j : Np - 1;
   double sum[NC];
   auto load = [&](int64_t i, int j) { return O[i * ldo + off[j]]; };
-  if constexpr (sizeof(T) == 4)
-    column_sums<T, NC>(Ns, part, sum, [](int64_t) {}, load, [](int, float x, float& h, float& l) { h = x; l = 0.f; });
-  else
-    column_sums<T, NC>(Ns, part, sum, [](int64_t) {}, load, [](int, double x) { return x; });
+  column_sums<T, NC, false>(
+      Ns, part, sum, [](int64_t) { return true; }, load,
+      [](vmc::Sum3& S, int, T v) {
+        S.add((float)v);
+        return (float)v;
+      },
+      [](int, T v) { return (double)v; });
   double m[NC];
 #pragma unroll
   for (int j = 0; j < NC; ++j) {
@@ -193,7 +199,7 @@ __global__ void __launch_bounds__(32 * CW) k_center(const T* __restrict__ O, int
         T v;
         if constexpr (sizeof(T) == 4) {
           float d = x[u][j];
-          const float e = two_sum(d, -mh[j]) - ml[j];
+          const float e = vmc::two_sum(d, -mh[j]) - ml[j];
           const float q = d * sh;
           const float r = fmaf(e, sh, fmaf(d, sl, fmaf(d, sh, -q)));
           const float w = fmaf(fabsf(q), 0x1p-43f, dm[j]);
@@ -429,14 +435,13 @@ __global__ void __launch_bounds__(256) k_trsv_bwd(const double* __restrict__ L, 
   if (threadIdx.x < nb) b[k1 + threadIdx.x] = bs[threadIdx.x];
 }
 
-// dp[p] = sum_i Oc[i][p] * x[i]; FP32 rows: the product with x = xh + xl (to
-// 2^-48, split once a CTA and block of rows) as an exact leading product and its
-// remainder
+// dp[p] = sum_i Oc[i][p] * x[i]; FP32 rows: the product with x = h + m + l (exact,
+// split once a CTA and block of rows) as two exact products and the last bits'
 template <typename T, int NC>
 __global__ void __launch_bounds__(32 * CW) k_gemv_t(const T* __restrict__ Oc, int64_t Ns, int64_t Np, int64_t ldc,
                                                     const double* __restrict__ x, double* __restrict__ dp) {
   __shared__ double part[CW][NC * 32];
-  __shared__ float2 xs[2][CB];     // two blocks: the next is written while the last is still read
+  __shared__ float4 xs[2][CB];     // two blocks: the next is written while the last is still read
   __shared__ double xd[2][CB];
   const int64_t p0 = (int64_t)blockIdx.x * (32 * NC) + (threadIdx.x & 31);
   int64_t off[NC];
@@ -446,27 +451,32 @@ __global__ void __launch_bounds__(32 * CW) k_gemv_t(const T* __restrict__ Oc, in
   int buf = 1;
   auto begin = [&](int64_t i0) {
     buf ^= 1;
+    bool out = false;
     if (threadIdx.x < CB) {
       const double v = i0 + threadIdx.x < Ns ? x[i0 + threadIdx.x] : 0.0;
+      xd[buf][threadIdx.x] = v;
       if constexpr (sizeof(T) == 4) {
-        float h, l;
-        split_f64(v, h, l);
-        xs[buf][threadIdx.x] = make_float2(h, l);
-      } else {
-        xd[buf][threadIdx.x] = v;
+        float h, m, l;
+        out = !split_f64(v, h, m, l);
+        xs[buf][threadIdx.x] = make_float4(h, m, l, 0.f);
       }
     }
-    __syncthreads();
+    return __syncthreads_or(out) == 0;
   };
   auto load = [&](int64_t i, int j) { return Oc[i * ldc + off[j]]; };
-  if constexpr (sizeof(T) == 4)
-    column_sums<T, NC>(Ns, part, sum, begin, load, [&](int r, float o, float& h, float& l) {
-      const float2 v = xs[buf][r];
-      h = o * v.x;
-      l = fmaf(o, v.y, fmaf(o, v.x, -h));
-    });
-  else
-    column_sums<T, NC>(Ns, part, sum, begin, load, [&](int r, double o) { return o * xd[buf][r]; });
+  column_sums<T, NC, true>(
+      Ns, part, sum, begin, load,
+      [&](vmc::Sum3& S, int r, T v) {
+        const float o = (float)v;
+        const float4 f = xs[buf][r];
+        const float p = __fmul_rn(o, f.x), q = __fmul_rn(o, f.y);
+        S.add(p);
+        S.low(fmaf(o, f.x, -p));
+        S.low(q);
+        S.d += fmaf(o, f.z, fmaf(o, f.y, -q));
+        return p;
+      },
+      [&](int r, T v) { return (double)v * xd[buf][r]; });
 #pragma unroll
   for (int j = 0; j < NC; ++j)
     if (p0 + 32 * j < Np && threadIdx.x < 32) dp[p0 + 32 * j] = sum[j];
