@@ -109,3 +109,18 @@ def test_infinite_entries_stay_in_their_columns():
     for v in (dp, mean):
         assert v[3] == np.inf and np.isnan(v[5]) and np.isnan(v[7])
         assert np.isfinite(np.delete(v, [3, 5, 7])).all()
+
+
+@pytest.mark.parametrize("f", [1e-44, 1e-38, 1e-30, 1e-25, 1e30, 2e38])
+@pytest.mark.parametrize("ns,npar", [(3, 20), (100, 33), (129, 38915)])
+def test_centring_over_the_range(f, ns, npar):
+    """Means that FP32 cannot sum (entries near its largest) and entries whose
+    scaled remainder underflows it: the FP64 expression rounded, as elsewhere."""
+    rng = np.random.default_rng(ns)
+    O = (rng.uniform(0.1, 1.5, (ns, npar)) * f).astype(np.float32)
+    O[:, ::3] = (rng.uniform(-1.5, 1.5, (ns, len(range(0, npar, 3)))) * f).astype(np.float32)
+    out, mean = center(torch.as_tensor(O, device=DEV))
+    ref = O.astype(np.float64).mean(0)
+    assert (np.abs(mean - ref) <= (ns + 2) * U * np.abs(O.astype(np.float64)).mean(0)).all()
+    want = ((O.astype(np.float64) - mean) * (1.0 / ns ** 0.5)).astype(np.float32)
+    assert np.array_equal(out, want)

@@ -149,7 +149,10 @@ __device__ __forceinline__ void column_sums(int64_t Ns, double (*part)[NC * 32],
 // own error (below 2^-43 of the entry and of the scaled mean) could change takes
 // the FP64 expression, so that the result is always that expression rounded:
 // about one entry in 10^5, tested for 16 entries at once (8192 samples, 115 K
-// columns: below 1 ms of a solve of 90).
+// columns: below 1 ms of a solve of 90).  So do entries whose distance from the
+// mean leaves [2^-80, 2^120): below it the remainders underflow FP32 (where the
+// mean is that small too: a larger one widens the test), above it the
+// difference overflows.
 template <typename T, int NC>
 __global__ void __launch_bounds__(32 * CW) k_center(const T* __restrict__ O, int64_t Ns, int64_t Np, int64_t ldo,
                                                     T* __restrict__ Oc, int64_t ldc, double* __restrict__ mean,
@@ -182,9 +185,13 @@ __global__ void __launch_bounds__(32 * CW) k_center(const T* __restrict__ O, int
   const float sh = (float)scale, sl = (float)(scale - (double)sh);
 #pragma unroll
   for (int j = 0; j < NC; ++j) { mh[j] = (float)m[j]; ml[j] = (float)(m[j] - (double)mh[j]); }
-  float dm[NC];
+  float dm[NC], d0[NC], d1[NC];     // |d| in [d0, d1): too small (an exact 0 - 0 is not)
 #pragma unroll
-  for (int j = 0; j < NC; ++j) dm[j] = fabsf(mh[j] * sh) * 0x1p-43f;
+  for (int j = 0; j < NC; ++j) {
+    dm[j] = fabsf(mh[j] * sh) * 0x1p-43f;
+    d0[j] = mh[j] == 0.f ? 0x1p-149f : 0.f;
+    d1[j] = fabsf(mh[j]) < 0x1p-80f ? 0x1p-80f : 0.f;
+  }
   for (int64_t i0 = warp; i0 < Ns; i0 += CW * CU) {
     T x[CU][NC];
 #pragma unroll
@@ -204,7 +211,7 @@ __global__ void __launch_bounds__(32 * CW) k_center(const T* __restrict__ O, int
           const float r = fmaf(e, sh, fmaf(d, sl, fmaf(d, sh, -q)));
           const float w = fmaf(fabsf(q), 0x1p-43f, dm[j]);
           v = q + (r + w);
-          unsure |= v != q + (r - w);
+          unsure |= v != q + (r - w) || !(fabsf(d) < 0x1p120f) || (fabsf(d) < d1[j] && fabsf(d) >= d0[j]);
         } else {
           v = (x[u][j] - m[j]) * scale;
         }
