@@ -153,10 +153,11 @@ __device__ __forceinline__ void column_sums(int64_t Ns, double (*part)[NC * 32],
 // mean leaves [2^-80, 2^120): below it the remainders underflow FP32 (where the
 // mean is that small too: a larger one widens the test), above it the
 // difference overflows.
+// O may be Oc (neither is __restrict__): a warp has read its rows before it
+// writes them, and no other warp of any CTA reads their columns' entries again.
 template <typename T, int NC>
-__global__ void __launch_bounds__(32 * CW) k_center(const T* __restrict__ O, int64_t Ns, int64_t Np, int64_t ldo,
-                                                    T* __restrict__ Oc, int64_t ldc, double* __restrict__ mean,
-                                                    double scale) {
+__global__ void __launch_bounds__(32 * CW) k_center(const T* O, int64_t Ns, int64_t Np, int64_t ldo, T* Oc,
+                                                    int64_t ldc, double* __restrict__ mean, double scale) {
   __shared__ double part[CW][NC * 32];
   __shared__ float again[sizeof(T) == 4 ? 16 : 1][32 * CW];
   constexpr int CU = 16 / NC;
