@@ -713,7 +713,7 @@ __global__ void __launch_bounds__(DG_THREADS) k_gemm_df(int64_t M, int64_t N, in
                                                         const double* __restrict__ D, int64_t ldd, int lower) {
   const int bi = blockIdx.y, bj = blockIdx.x;
   if (lower && bj > bi) return;
-  __shared__ float As[2][DG_K][DG_T + 4], Bs[2][DG_K][DG_T + 4];
+  __shared__ alignas(16) float As[2][DG_K][DG_T + 4], Bs[2][DG_K][DG_T + 4];
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
   const int64_t m0 = (int64_t)bi * DG_T, n0 = (int64_t)bj * DG_T;
   float hi[8][4], lo[8][4];

@@ -578,7 +578,7 @@ __global__ void __launch_bounds__(sg::NTHR, 2) k_g_dz0(GradNet<float> net, int R
 // the 8x8 model); 16-byte stores where the rows are aligned.
 __global__ void __launch_bounds__(256) k_g_write(int N, int nf, float s, const uint64_t* __restrict__ occ, GradWork w,
                                                  float* __restrict__ O, int64_t ld, int full) {
-  __shared__ float h1[HID], h2[HID], oc[128];
+  __shared__ alignas(16) float h1[HID], h2[HID], oc[128];
   const int64_t b = blockIdx.x;
   const int tid = threadIdx.x, lane = tid & 31;
   const int n_orb = 2 * N, nout = n_orb * nf;

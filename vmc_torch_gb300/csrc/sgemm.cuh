@@ -15,7 +15,7 @@ namespace sg {
 
 constexpr int BM = 128, BN = 128, BK = 16, NTHR = 256;
 constexpr int LDS_ = BM + 4;
-struct Smem { float a[2][BK][LDS_]; float b[2][BK][LDS_]; };
+struct alignas(16) Smem { float a[2][BK][LDS_]; float b[2][BK][LDS_]; };
 
 // Operand tile of 128 rows (of the output dimension) x BK.  KMAJ: X[r][k]
 // (ld between r), else X[k][r] (ld between k).  vec: 16-byte loads are
