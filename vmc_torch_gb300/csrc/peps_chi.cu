@@ -235,7 +235,8 @@ __device__ void warp_hestenes(T (&u)[32], T* V, T* lam) {
 // goes through shared memory (lane k holds column k of L), its rows are made
 // orthogonal (no rotation matrix is kept: A A^T = L L^T, whose eigenvectors
 // are the normalised final rows), and lam[k] = |row k|^2, V[k * 33 + i] =
-// row k / |row k| (zero for a zero row).  S: a 32 x 33 scratch.
+// row k / |row k| (zero for a zero row and one of rounding noise).  S: a 32 x
+// 33 scratch.
 template <typename T>
 __device__ void warp_lq_jacobi(T (&u)[32], int nq, T* S, T* V, T* lam) {
   const int ln = threadIdx.x & 31;
@@ -328,7 +329,14 @@ __device__ void warp_lq_jacobi(T (&u)[32], int nq, T* S, T* V, T* lam) {
 #pragma unroll
   for (int j = 0; j < 32; ++j) nrm = fma(u[j], u[j], nrm);
   lam[ln] = nrm;
-  const T inv = nrm > T(0) ? T(1) / sqrt(nrm) : T(0);
+  // a row below 16 rounding units of the block's largest is the noise of a rank-
+  // deficient block: it was not made orthogonal (floor_) and may point along a
+  // kept vector, which the projection would then count twice
+  T top = nrm;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) top = fmax(top, __shfl_xor_sync(VMC_FULL_MASK, top, o));
+  const T least = std::is_same<T, float>::value ? T(1.9e-6) : T(3.6e-15);
+  const T inv = nrm > least * least * top ? T(1) / sqrt(nrm) : T(0);
 #pragma unroll
   for (int j = 0; j < 32; ++j) V[ln * 33 + j] = u[j] * inv;
   __syncwarp();
