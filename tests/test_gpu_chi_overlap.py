@@ -45,3 +45,16 @@ def test_states_of_rank_one(a, b, c, precision):
     st = overlap_model(a, b, c, precision).bind_state(x)
     assert float(st.sign[0]) == math.copysign(1.0, c)
     assert abs(float(st.logabs[0]) - math.log(a * a * b * 1e20)) <= 1e-5
+
+
+@pytest.mark.parametrize("a,b,c", [(1e-13, 1e-25, 1.0), (1e-18, 1e-3, 1.0),
+                                   (1e-12, 1e-30, -1.0)])
+def test_small_overlaps_of_normalised_states(a, b, c):
+    """FP32 tensors (2^-24 relative each, four of them), a few FP32 roundings of
+    the truncation: 1e-5 in the log-amplitude."""
+    x = torch.zeros(1, 16, dtype=torch.int64, device=DEV)
+    x[0, [0, 5, 10]] = 3
+    for precision in ("fp64", "fp32"):
+        st = overlap_model(a, b, c, precision).bind_state(x)
+        assert float(st.sign[0]) == math.copysign(1.0, c), precision
+        assert abs(float(st.logabs[0]) - math.log(a * a * b * 1e20)) <= 1e-5, precision

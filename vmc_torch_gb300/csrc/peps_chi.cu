@@ -833,44 +833,42 @@ __device__ __forceinline__ void chi_finish(double v, int et, int eb, uint64_t up
 
 // <a, b> by one warp.  FP32 states: an FP64 instruction costs a warp 64 clocks
 // on GB300 (two conversions and a multiply-add per element), so the products
-// are taken exactly as p + fma(a, b, -p) and summed in three FP32 words with
-// TwoSum (~2^-70 of the largest partial sum, finer than the FP64 sum), joined
-// in FP64 at the end.
-__device__ __forceinline__ float dot_two_sum(float& s, float x) {
-  const float t = s + x, bb = t - s;
-  const float e = (s - (t - bb)) + (x - bb);
-  s = t;
-  return e;
-}
-__device__ __forceinline__ void dot_add(float a, float b, float& s, float& c, float& d) {
-  const float p = a * b;
-  const float q = fmaf(a, b, -p);
-  const float e = dot_two_sum(s, p);
-  d += dot_two_sum(c, e);
-  d += dot_two_sum(c, q);
+// are taken exactly as p + fma(a, b, -p) and summed in three FP32 words (Sum3,
+// finer than the FP64 sum), joined in FP64 at the end.  The states' largest
+// entries are 1 to 2, but they need not meet: where the largest product lies
+// outside [2^-85, 2^100), so that FP32 loses error terms that count, the sum is
+// taken in FP64.
+constexpr unsigned DOT_LO = (127u - 85u) << 23, DOT_HI = (127u + 100u) << 23;
+
+__device__ __forceinline__ void dot_add(float a, float b, Sum3& S, float& mx) {
+  const float p = __fmul_rn(a, b);
+  mx = fmaxf(mx, fabsf(p));     // a NaN shows in the sum
+  S.add(p);
+  S.low(fmaf(a, b, -p));
 }
 template <typename T>
 __device__ __forceinline__ double warp_dot(const T* __restrict__ a, const T* __restrict__ b, int NS) {
   const int ln = threadIdx.x & 31;
-  double acc = 0.0;
   if constexpr (std::is_same<T, float>::value) {
-    float s = 0.f, c = 0.f, d = 0.f;
+    Sum3 S;
+    float mx = 0.f;
     if ((NS & 127) == 0) {     // states start at multiples of NS elements of an aligned workspace
 #pragma unroll 4
       for (int e = ln * 4; e < NS; e += 128) {
         const float4 x = *reinterpret_cast<const float4*>(a + e), y = *reinterpret_cast<const float4*>(b + e);
-        dot_add(x.x, y.x, s, c, d);
-        dot_add(x.y, y.y, s, c, d);
-        dot_add(x.z, y.z, s, c, d);
-        dot_add(x.w, y.w, s, c, d);
+        dot_add(x.x, y.x, S, mx);
+        dot_add(x.y, y.y, S, mx);
+        dot_add(x.z, y.z, S, mx);
+        dot_add(x.w, y.w, S, mx);
       }
     } else {
-      for (int e = ln; e < NS; e += 32) dot_add(a[e], b[e], s, c, d);
+      for (int e = ln; e < NS; e += 32) dot_add(a[e], b[e], S, mx);
     }
-    acc = (double)s + ((double)c + (double)d);
-  } else {
-    for (int e = ln; e < NS; e += 32) acc += (double)a[e] * (double)b[e];
+    const unsigned m = __reduce_max_sync(VMC_FULL_MASK, isfinite(S.s) ? __float_as_uint(mx) : 0x7fffffffu);
+    if (m >= DOT_LO && m < DOT_HI) return warp_sum(S.value());
   }
+  double acc = 0.0;
+  for (int e = ln; e < NS; e += 32) acc += (double)a[e] * (double)b[e];
   return warp_sum(acc);
 }
 
