@@ -542,11 +542,30 @@ __global__ void __launch_bounds__(sg::NTHR, 2) k_g_dh2(GradNet<float> net, int n
   }
 }
 
-__global__ void k_g_dz1(int64_t n, float s, GradWork w) {
+// The product runs over all orbitals, Gbar being zero at the empty ones and in
+// rows without an inverse; where an output weight there is not finite, 0 times
+// it is NaN, and the sum over the row's own orbitals is taken instead.
+__global__ void k_g_dz1(GradNet<float> net, int N, int nf, int64_t n, float s, const uint64_t* __restrict__ occ,
+                        GradWork w) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   float acc = w.dh[i];
   for (int z = 1; z < w.splits; ++z) acc += w.dh[z * n + i];
+  if (!isfinite(acc)) {
+    const int64_t b = i / HID, nout = (int64_t)2 * N * nf;
+    const uint64_t up = occ[2 * b], dn = occ[2 * b + 1];
+    bool inverse = false;     // A^-1 has a non-zero entry
+    acc = 0.f;
+    for (int o = 0; o < 2 * N; ++o) {
+      if (!orb_occupied(up, dn, N, o)) continue;
+      for (int64_t j = (int64_t)o * nf; j < (int64_t)(o + 1) * nf; ++j) {
+        const float g = w.gbar[b * nout + j];
+        inverse |= g != 0.f;
+        acc += g * net.outw[j * HID + (i - b * HID)];
+      }
+    }
+    if (!inverse) acc = 0.f;
+  }
   w.dz1[i] = s * acc * gelu_d<float>(w.z1[i]);
 }
 
@@ -729,7 +748,7 @@ extern "C" int vmc_nnbf_logpsi_grad_ws(const void* const* gnet, int n_sites, int
       k_g_invert<64, 4><<<one, 128, 0, st>>>(N, nf, s, (int)R, oc, w, of, ld_full, od, ld_dense, kg, la, sg_);
     const int kchunk = (int)(((nout + splits - 1) / splits + sg::BK - 1) / sg::BK * sg::BK);
     k_g_dh2<<<dim3(HID / sg::BN, mt, (unsigned)splits), sg::NTHR, 0, st>>>(g, (int)nout, (int)R, kchunk, w);
-    k_g_dz1<<<(unsigned)((R * HID + 255) / 256), 256, 0, st>>>(R * HID, s, w);
+    k_g_dz1<<<(unsigned)((R * HID + 255) / 256), 256, 0, st>>>(g, N, nf, R * HID, s, oc, w);
     k_g_dz0<<<dim3(HID / sg::BN, mt), sg::NTHR, 0, st>>>(g, (int)R, w);
     if (od) k_g_write<<<dim3((unsigned)R, 4), 256, 0, st>>>(N, nf, s, oc, w, od, ld_dense, 0);
     if (of) k_g_write<<<dim3((unsigned)R, 32), 256, 0, st>>>(N, nf, s, oc, w, of, ld_full, 1);
