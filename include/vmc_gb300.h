@@ -311,9 +311,14 @@ int vmc_sr_cholesky(double* T, int64_t n, int64_t ldt, int* d_info, void* stream
  *   kp a multiple of 32 >= K, padding zeroed; planes (16-byte aligned) holds
  *   7 * rows_pad * kp bf16.
  * vmc_sr_gram_f64_tc: T (ns, ns, FP64, ld ldt) = [T +] X X^T [+ shift I], the
- *   full symmetric matrix; digit products of levels 0..6 (28 of the 49; the rest
- *   is below 2^-56 of the largest entries' product), summed as integers, added
- *   in FP64 every 256 columns.  Rows and columns with a NaN or Inf come out NaN.
+ *   full symmetric matrix; digit products of levels 0..6 (28 of the 49), added in
+ *   FP64 every 256 columns.  Levels 0..4 are summed as exact integers; 5 and 6
+ *   (2^-54 and 2^-62 of 2^(E_i + E_j)) may lose a unit or two where 256 digits
+ *   share a sign.  Error per entry: at most 36 x 2^-56 max|X_i| max|X_j| for every
+ *   column, and the FP64 additions' roundings; vmc_sr_gram's is relative to the
+ *   sum of |x_ik x_jk| and smaller for rows whose large entries stand in
+ *   different columns.  Rows and columns with a NaN or Inf come out NaN; entries
+ *   below 2^-1022 count as zero.
  * vmc_sr_cholesky_tc: as vmc_sr_cholesky with the trailing updates done this
  *   way; work (256-byte aligned) of *bytes from vmc_sr_cholesky_tc_work_bytes.
  * d_err (device int) receives VMC_ERR_TIMEOUT if a bounded wait gave up. */

@@ -8,21 +8,31 @@
 // FP64's own 2^-53 for entries within a factor 8 of it), is written as seven
 // balanced base-256 digits d_0 .. d_6 in [-128, 128], each exact in BF16.  A
 // product x_i x_j is the sum of the digit products d_p d_q of level p + q with
-// weight 2^(-14 - 8 (p + q)); the 28 products of levels 0..6 are formed (what
-// is left out is below 2^-56 of the largest entries' product per term).  All
-// products of one level share a TMEM accumulator: integers of at most 2^14,
-// so 256 columns of K sum to at most 2^22 times the level's p + q + 1
-// products, within FP32's 2^24 exact integers for levels 0..3 in the worst
-// case (levels 4..6 for digits of random sign; there one unit is 2^-46 or
-// less of the result's scale).  Every 256 columns the seven levels are
-// combined as one 64-bit integer (unit 2^-54) and added in FP64.
+// weight 2^(-14 - 8 (p + q)); the 28 products of levels 0..6 are formed.  What is
+// left out is at most 6 x 2^-56 of 2^(E_i + E_j) per term (level 7), and the
+// operands' rounding 2 x 2^-56 of it: with 2^E at most twice the largest entry,
+// 36 x 2^-56 of the two rows' largest entries' product.  The error thus scales
+// with those, not with the sum of |x_ik x_jk| as that of FP64 multiply-adds
+// does: below theirs where the rows' entries are of one size, above where the
+// large entries of two rows stand in different columns (vmc_sr_gram is the
+// choice there); relative to sqrt(T_ii T_jj) it is below K 36 x 2^-56 always,
+// like the error that a Cholesky factorisation of T commits by itself.
+//
+// All products of one level share a TMEM accumulator: integers of at most 2^14,
+// so 256 columns of K sum to at most 2^22 times the level's products.  Levels 0
+// to 3 (one to four products) stay within FP32's 2^24 exact integers, level 4
+// (five) has two accumulators of three and two, and is exact as well.  Levels 5
+// and 6 (six and seven) pass 2^24 where digits share a sign, and lose a unit or
+// two in the additions beyond it, which is 2^-54 and 2^-62 of 2^(E_i + E_j).
+// (Level 4 in one accumulator lost units of 2^-46 there.)  Every 256 columns
+// the levels are combined as one 64-bit integer (unit 2^-54) and added in FP64.
 //
 // On GB300 FP64 arithmetic runs at 2 multiply-adds a clock per SM (1.25
 // TFLOP/s), BF16 tcgen05 at 1.9 PFLOP/s measured: 28 products leave 34
 // TFLOP/s per executed multiply-add pair of the FP64 result, 54x.
 //
-// Tile: 128 x 64 outputs per CTA (7 levels x 64 columns = 448 of the 512 TMEM
-// columns; 128 columns would not fit).  K atoms of 32 (SWIZZLE_64B) so that two
+// Tile: 128 x 64 outputs per CTA (8 accumulators x 64 columns: all 512 TMEM
+// columns).  K atoms of 32 (SWIZZLE_64B) so that two
 // stages of all seven planes of both operands (84 KB each) fit shared memory;
 // one 3-D TMA load per operand and stage brings the seven planes.  Warp 0
 // issues the copies, warp 1 (one thread) the MMAs, warps 2..5 combine.
@@ -36,6 +46,8 @@
 namespace {
 
 constexpr int ND = 7;                          // digits per entry, levels per product
+constexpr int SPLIT_LV = 4, SPLIT_P = 3;       // products p >= SPLIT_P of level SPLIT_LV: an accumulator of their own
+constexpr int NACC = ND + 1;
 constexpr int OM = 128, ON = 64;               // tile
 constexpr int OK = 32;                         // K atom (64 bytes of BF16)
 constexpr int APLANE = OM * OK * 2, BPLANE = ON * OK * 2;
@@ -205,9 +217,12 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
 #pragma unroll
             for (int p = 0; p <= lv; ++p)
 #pragma unroll
-              for (int kk = 0; kk < OK / 16; ++kk)
-                tc::mma_bf16(tbase + (uint32_t)(lv * ON), tc::sdesc_sw64(sa + p * APLANE + kk * 32),
-                             tc::sdesc_sw64(sb + (lv - p) * BPLANE + kk * 32), idesc, (a > a0 || p || kk) ? 1u : 0u);
+              for (int kk = 0; kk < OK / 16; ++kk) {
+                const bool own = lv == SPLIT_LV && p >= SPLIT_P;
+                tc::mma_bf16(tbase + (uint32_t)((own ? ND : lv) * ON), tc::sdesc_sw64(sa + p * APLANE + kk * 32),
+                             tc::sdesc_sw64(sb + (lv - p) * BPLANE + kk * 32), idesc,
+                             (a > a0 || p != (own ? SPLIT_P : 0) || kk) ? 1u : 0u);
+              }
           tc::mma_commit(&empty[s]);   // the stage is free once these MMAs have read it
         }
         if (ok) tc::mma_commit(tfull);
@@ -228,13 +243,14 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
       tc::fence_after_sync();
 #pragma unroll
       for (int g = 0; g < ON / 8; ++g) {
-        uint32_t v[ND][8];
-        tc::tmem_ld8x7(tbase + ((uint32_t)(quad * 32) << 16) + (uint32_t)(g * 8), ON, v);
+        uint32_t v[NACC][8];
+        tc::tmem_ld8x8(tbase + ((uint32_t)(quad * 32) << 16) + (uint32_t)(g * 8), ON, v);
 #pragma unroll
         for (int q = 0; q < 8; ++q) {
           int lv[ND];
 #pragma unroll
           for (int p = 0; p < ND; ++p) lv[p] = __float2int_rn(__uint_as_float(v[p][q]));
+          lv[SPLIT_LV] += __float2int_rn(__uint_as_float(v[ND][q]));
           // levels 0..3 in units of 2^-38, 4..6 in units of 2^-62; together in 2^-54
           const long long hi = ((((long long)lv[0] * 256 + lv[1]) * 256 + lv[2]) * 256) + lv[3];
           const long long lo = (((long long)lv[4] * 256 + lv[5]) * 256) + lv[6];

@@ -152,25 +152,27 @@ __device__ __forceinline__ void tmem_ld8x2(uint32_t taddr, uint32_t step, float 
   }
 }
 
-// Seven groups of 32 lanes x 8 columns, `step` columns apart (one group per
-// digit level of the fixed-point products), read in flight together.
-__device__ __forceinline__ void tmem_ld8x7(uint32_t taddr, uint32_t step, uint32_t (&r)[7][8]) {
+// Eight groups of 32 lanes x 8 columns, `step` columns apart (the accumulators of
+// the fixed-point products), read in flight together.
+__device__ __forceinline__ void tmem_ld8x8(uint32_t taddr, uint32_t step, uint32_t (&r)[8][8]) {
   asm volatile(
       "{\n .reg .b32 a;\n"
-      " mov.b32 a, %56;\n"
+      " mov.b32 a, %64;\n"
       " tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [a];\n"
-      " add.u32 a, a, %57;\n"
+      " add.u32 a, a, %65;\n"
       " tcgen05.ld.sync.aligned.32x32b.x8.b32 {%8,%9,%10,%11,%12,%13,%14,%15}, [a];\n"
-      " add.u32 a, a, %57;\n"
+      " add.u32 a, a, %65;\n"
       " tcgen05.ld.sync.aligned.32x32b.x8.b32 {%16,%17,%18,%19,%20,%21,%22,%23}, [a];\n"
-      " add.u32 a, a, %57;\n"
+      " add.u32 a, a, %65;\n"
       " tcgen05.ld.sync.aligned.32x32b.x8.b32 {%24,%25,%26,%27,%28,%29,%30,%31}, [a];\n"
-      " add.u32 a, a, %57;\n"
+      " add.u32 a, a, %65;\n"
       " tcgen05.ld.sync.aligned.32x32b.x8.b32 {%32,%33,%34,%35,%36,%37,%38,%39}, [a];\n"
-      " add.u32 a, a, %57;\n"
+      " add.u32 a, a, %65;\n"
       " tcgen05.ld.sync.aligned.32x32b.x8.b32 {%40,%41,%42,%43,%44,%45,%46,%47}, [a];\n"
-      " add.u32 a, a, %57;\n"
+      " add.u32 a, a, %65;\n"
       " tcgen05.ld.sync.aligned.32x32b.x8.b32 {%48,%49,%50,%51,%52,%53,%54,%55}, [a];\n"
+      " add.u32 a, a, %65;\n"
+      " tcgen05.ld.sync.aligned.32x32b.x8.b32 {%56,%57,%58,%59,%60,%61,%62,%63}, [a];\n"
       " tcgen05.wait::ld.sync.aligned;\n}\n"
       : "=r"(r[0][0]), "=r"(r[0][1]), "=r"(r[0][2]), "=r"(r[0][3]), "=r"(r[0][4]), "=r"(r[0][5]), "=r"(r[0][6]), "=r"(r[0][7]),
         "=r"(r[1][0]), "=r"(r[1][1]), "=r"(r[1][2]), "=r"(r[1][3]), "=r"(r[1][4]), "=r"(r[1][5]), "=r"(r[1][6]), "=r"(r[1][7]),
@@ -178,7 +180,8 @@ __device__ __forceinline__ void tmem_ld8x7(uint32_t taddr, uint32_t step, uint32
         "=r"(r[3][0]), "=r"(r[3][1]), "=r"(r[3][2]), "=r"(r[3][3]), "=r"(r[3][4]), "=r"(r[3][5]), "=r"(r[3][6]), "=r"(r[3][7]),
         "=r"(r[4][0]), "=r"(r[4][1]), "=r"(r[4][2]), "=r"(r[4][3]), "=r"(r[4][4]), "=r"(r[4][5]), "=r"(r[4][6]), "=r"(r[4][7]),
         "=r"(r[5][0]), "=r"(r[5][1]), "=r"(r[5][2]), "=r"(r[5][3]), "=r"(r[5][4]), "=r"(r[5][5]), "=r"(r[5][6]), "=r"(r[5][7]),
-        "=r"(r[6][0]), "=r"(r[6][1]), "=r"(r[6][2]), "=r"(r[6][3]), "=r"(r[6][4]), "=r"(r[6][5]), "=r"(r[6][6]), "=r"(r[6][7])
+        "=r"(r[6][0]), "=r"(r[6][1]), "=r"(r[6][2]), "=r"(r[6][3]), "=r"(r[6][4]), "=r"(r[6][5]), "=r"(r[6][6]), "=r"(r[6][7]),
+        "=r"(r[7][0]), "=r"(r[7][1]), "=r"(r[7][2]), "=r"(r[7][3]), "=r"(r[7][4]), "=r"(r[7][5]), "=r"(r[7][6]), "=r"(r[7][7])
       : "r"(taddr), "r"(step));
 }
 

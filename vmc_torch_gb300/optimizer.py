@@ -142,7 +142,12 @@ class MinSRGB300(PreconditionerGB300):
         up to ~2^-32 rounding.  "cuda" forms them on the CUDA cores with
         compensated (double-float) accumulation: the exact Gram of the FP32
         rows, ~10x slower.  FP64 O: "tensor" uses seven base-256 digits of
-        every entry (vmc_sr_gram_f64_tc, FP64 accuracy), "cuda" the FP64 cores."""
+        every entry (vmc_sr_gram_f64_tc): rows to 2^-56 of their largest
+        entry, errors of T_ij that scale with the largest entries of rows i
+        and j.  "cuda" uses the FP64 cores (errors relative to the sum of
+        |O_ik O_jk|), ~10x slower: the choice where rows have their large
+        entries in different columns and T itself is wanted, not only the
+        solution of the positive definite system."""
         if gram not in ("tensor", "cuda"):
             raise ValueError("gram must be 'tensor' or 'cuda'")
         self.record_stages = record_stages
