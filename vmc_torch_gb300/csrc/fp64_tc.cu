@@ -456,9 +456,18 @@ __global__ void k_syrk_df(const double* __restrict__ A, int64_t lda, int64_t n, 
 // a_ij -= u_i (u_j / d_k).  Eight steps are a phase with the register groups
 // left of or above them left out at compile time: ~15 FP64 instructions a warp
 // and step (with 16 lanes a row in k_trsm64: minSR of 2049 x 8192 7.98 -> 7.31 ms).
-template <int KP>
+//
+// Near the ends of FP64's range 1 / d is subnormal or overflows.  The steps do
+// not test for it (a scaled reciprocal in the loop: minSR of 2049 x 8192 7.33 ->
+// 7.66 ms); a tile that met such a pivot is factored again from C, with r =
+// 1 / (d sc) and a product with sc.
+__device__ __forceinline__ bool far_exponent(double d) {
+  const int e = (__double2hiint(d) >> 20) - 1023;
+  return e < -1000 || e > 1000;
+}
+template <int KP, bool FAR>
 __device__ __forceinline__ void potrf_phase(double (&a)[8][4], double (*uc)[NB], double* dk, double* rk, int tx, int ty,
-                                            int* __restrict__ info) {
+                                            bool& bad) {
 #pragma unroll 1
   for (int kk = 0; kk < 8; ++kk) {
     const int k = 8 * KP + kk;
@@ -466,10 +475,11 @@ __device__ __forceinline__ void potrf_phase(double (&a)[8][4], double (*uc)[NB],
     const double* u = uc[k & 1];
     double d = u[k];
     if (!(d > 0.0) || (__double2hiint(d) & 0x7ff00000) == 0x7ff00000) {
-      if (threadIdx.x == 0) atomicExch(info, 1);
+      bad = true;
       d = 1e-300;
     }
-    const double r = vmc::rcp_pos(d);
+    const double sc = FAR && far_exponent(d) ? (d < 1.0 ? 0x1p300 : 0x1p-300) : 1.0;
+    const double r = FAR ? 1.0 / (d * sc) : vmc::rcp_pos(d);
     if (threadIdx.x == 0) { dk[k] = d; rk[k] = r; }
     double ui[8];
 #pragma unroll
@@ -478,7 +488,8 @@ __device__ __forceinline__ void potrf_phase(double (&a)[8][4], double (*uc)[NB],
 #pragma unroll
     for (int jj = KP / 2; jj < 4; ++jj) {   // the group of the next column comes first
       const int c = tx + 16 * jj;
-      const double v = c > k ? u[c] * r : 0.0;
+      double v = c > k ? u[c] * r : 0.0;
+      if (FAR) v *= sc;
 #pragma unroll
       for (int i = 2 * jj > KP ? 2 * jj : KP; i < 8; ++i) a[i][jj] = fma(-ui[i], v, a[i][jj]);
       if (jj == jn && c == k + 1)
@@ -487,11 +498,9 @@ __device__ __forceinline__ void potrf_phase(double (&a)[8][4], double (*uc)[NB],
     }
   }
 }
-__global__ void __launch_bounds__(128) k_potrf64(double* __restrict__ C, int64_t ldc, int nb, int* __restrict__ info) {
-  __shared__ double uc[2][NB];
-  __shared__ double dk[NB], rk[NB];
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  double a[8][4];
+template <bool FAR>
+__device__ __forceinline__ void potrf_tile(const double* C, int64_t ldc, int nb, double (&a)[8][4], double (*uc)[NB],
+                                           double* dk, double* rk, int tx, int ty, bool& bad) {
 #pragma unroll
   for (int i = 0; i < 8; ++i)
 #pragma unroll
@@ -502,19 +511,31 @@ __global__ void __launch_bounds__(128) k_potrf64(double* __restrict__ C, int64_t
   if (tx == 0)
 #pragma unroll
     for (int i = 0; i < 8; ++i) uc[0][ty + 8 * i] = a[i][0];
-  potrf_phase<0>(a, uc, dk, rk, tx, ty, info);
-  potrf_phase<1>(a, uc, dk, rk, tx, ty, info);
-  potrf_phase<2>(a, uc, dk, rk, tx, ty, info);
-  potrf_phase<3>(a, uc, dk, rk, tx, ty, info);
-  potrf_phase<4>(a, uc, dk, rk, tx, ty, info);
-  potrf_phase<5>(a, uc, dk, rk, tx, ty, info);
-  potrf_phase<6>(a, uc, dk, rk, tx, ty, info);
-  potrf_phase<7>(a, uc, dk, rk, tx, ty, info);
+  bad = false;
+  potrf_phase<0, FAR>(a, uc, dk, rk, tx, ty, bad);
+  potrf_phase<1, FAR>(a, uc, dk, rk, tx, ty, bad);
+  potrf_phase<2, FAR>(a, uc, dk, rk, tx, ty, bad);
+  potrf_phase<3, FAR>(a, uc, dk, rk, tx, ty, bad);
+  potrf_phase<4, FAR>(a, uc, dk, rk, tx, ty, bad);
+  potrf_phase<5, FAR>(a, uc, dk, rk, tx, ty, bad);
+  potrf_phase<6, FAR>(a, uc, dk, rk, tx, ty, bad);
+  potrf_phase<7, FAR>(a, uc, dk, rk, tx, ty, bad);
   __syncthreads();
+}
+__global__ void __launch_bounds__(128) k_potrf64(double* __restrict__ C, int64_t ldc, int nb, int* __restrict__ info) {
+  __shared__ double uc[2][NB];
+  __shared__ double dk[NB], rk[NB];
+  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+  double a[8][4];
+  bool bad;
+  potrf_tile<false>(C, ldc, nb, a, uc, dk, rk, tx, ty, bad);
+  const bool far = __syncthreads_or(threadIdx.x < NB && far_exponent(dk[threadIdx.x]));
+  if (far) potrf_tile<true>(C, ldc, nb, a, uc, dk, rk, tx, ty, bad);
+  if (bad && threadIdx.x == 0) atomicExch(info, 1);
   if (threadIdx.x < NB) {
-    const double sq = sqrt(dk[threadIdx.x]);
+    const double d = dk[threadIdx.x], sq = sqrt(d);
     dk[threadIdx.x] = sq;
-    rk[threadIdx.x] *= sq;    // 1 / sqrt(d)
+    rk[threadIdx.x] = far ? 1.0 / sq : rk[threadIdx.x] * sq;    // 1 / sqrt(d)
   }
   __syncthreads();
 #pragma unroll
