@@ -112,6 +112,8 @@ int vmc_slater_logpsi_grad(const double* G, const uint8_t* slot_orb, int64_t B, 
  *   [5] out_b (2N*nf) f32/f64     [6] M_base (2N, nf) f32/f64
  * Workspace for R rows (caller-owned): H1, H2 (R, 256) bf16/f64; A (R, nf, nf) f32/f64
  * (scratch; the FP32 matrices are kept in blocks of 8 columns).
+ * The weights must not be written while a call that reads them runs; work queued
+ * on the stream before the call may write them.
  * The workspace is scratch: its contents on return are unspecified (the LU
  * reuses consumed orbital-matrix rows).
  * d_err (device int) receives VMC_ERR_TIMEOUT if a bounded device wait gave up,

@@ -35,8 +35,11 @@ namespace {
 
 // Programmatic dependent launch (single-stream sweeps, lanes of 32 orbitals): a kernel lets its
 // successor's CTAs be placed as soon as its own have started, and waits for
-// its predecessor's completion before it touches anything that one writes.  Both
-// are no-ops in a launch without the attribute.
+// its predecessor's completion before it touches anything that one writes.
+// The wait is a no-op in a launch without the attribute; the trigger still
+// releases a successor that has it.  What a kernel reads before its wait (the
+// hidden layer's weights) is ordered after the work queued before the call by
+// the call's first launch on a stream, which is always a plain one.
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
@@ -327,8 +330,8 @@ __global__ void __launch_bounds__(128, 2)
     tc::prefetch_tmap(&tmB);
     *sflag = 1;
   }
-  // the weights' tile, which no earlier kernel of the stream writes, may come
-  // before the predecessor's end
+  // the weights' tile, which no kernel of the call writes, may come before the
+  // predecessor's end
   auto load_b = [&] {
     tc::mbar_arrive_expect_tx(&bars[4], SMEM_HB);
 #pragma unroll
@@ -1844,8 +1847,8 @@ int vmc_nnbf_sweep(int prec, const void* const* net_ptrs, int n_sites, int nf, i
           const int par = (s * n_edges + e) & 1;
           int* cn = ccnt ? ccnt + 2 * g + par : nullptr;
           int* cx = ccnt ? ccnt + 2 * g + (par ^ 1) : nullptr;
-          launch(lane_pdl, k_prep_sweep<float>, gwg, 256, 0, gs, B, w0, w1, n_sites, occ, edges, e, s, n_edges,
-                 hopping_rate, seed, sweep_offset + (uint64_t)s, r_move, r_bit, r_acc, (const float*)z0, nf32.w0t,
+          launch(lane_pdl && (s || e), k_prep_sweep<float>, gwg, 256, 0, gs, B, w0, w1, n_sites, occ, edges, e, s,
+                 n_edges, hopping_rate, seed, sweep_offset + (uint64_t)s, r_move, r_bit, r_acc, (const float*)z0, nf32.w0t,
                  prop_occ, (PropRec*)rec, H1, cn, cmap, cprop, cx);
           int rc = launch_eval_rows(prec, w1 - w0, n_sites, nf, cn ? cprop + 2 * w0 : prop_occ + 2 * w0, net,
                                     bf_scale, wg, d_err, gs, LD_ACCEPT, lg, /*allow_pipe=*/false, cn, cn ? cmap + w0 : nullptr, &maps, lane_pdl);
@@ -1879,8 +1882,8 @@ int vmc_nnbf_sweep(int prec, const void* const* net_ptrs, int n_sites, int nf, i
       int* cx = ccnt ? ccnt + (par ^ 1) : nullptr;
       STAGE_BEGIN(0);
       if (prec == 0)
-        launch(pdl, k_prep_sweep<float>, gw, 256, 0, st, B, 0, B, n_sites, occ, edges, e, s, n_edges, hopping_rate,
-               seed, sweep_offset + (uint64_t)s, r_move, r_bit, r_acc, (const float*)z0, nf32.w0t, prop_occ,
+        launch(pdl && (s || e), k_prep_sweep<float>, gw, 256, 0, st, B, 0, B, n_sites, occ, edges, e, s, n_edges,
+               hopping_rate, seed, sweep_offset + (uint64_t)s, r_move, r_bit, r_acc, (const float*)z0, nf32.w0t, prop_occ,
                (PropRec*)rec, H1, cn, cmap, cprop, cx);
       else
         k_prep_sweep<double><<<gw, 256, 0, st>>>(B, 0, B, n_sites, occ, edges, e, s, n_edges, hopping_rate, seed,
@@ -1982,8 +1985,8 @@ int vmc_nnbf_local_energy(int prec, const void* const* net_ptrs, int n_sites, in
       double* co = coeff + (size_t)g * sub;
       const Work wg{(char*)H1 + (size_t)g * sub * HID * 2, (char*)H2 + (size_t)g * sub * HID * 2,
                     (float*)A + (size_t)g * sub * nf * nf};
-      launch(lane_pdl, k_prep_conn<float>, (unsigned)((R * 32 + 255) / 256), 256, 0, gs, R, n_sites, pairs + 2 * p0,
-             occ, edges, t, (const float*)z0, nf32.w0t, ro, co, wg.H1);
+      launch(lane_pdl && k >= G, k_prep_conn<float>, (unsigned)((R * 32 + 255) / 256), 256, 0, gs, R, n_sites,
+             pairs + 2 * p0, occ, edges, t, (const float*)z0, nf32.w0t, ro, co, wg.H1);
       LdArgs la{};
       la.pairs = pairs + 2 * p0;
       la.coeff = co;
