@@ -1472,54 +1472,107 @@ int num_sms() {
 
 void set_attrs();
 
-// Second stream for the chunk pipeline: the backflow GEMM of chunk c+1 runs
-// on it (high priority) while the LU of chunk c runs on the caller's stream;
-// the GEMM is tensor/epilogue work and the LU latency-bound CUDA-core work,
-// so the two share the SMs.  Events order the slot reuse of the two A
-// buffers.  VMC_GB300_SERIAL_CHUNKS=1 runs the chunks back to back instead.
+// Streams and events of a call whose parts run side by side.  aux, h2, g, lu: the
+// chunk pipeline, in which the backflow GEMM of chunk c+1 runs on a second
+// stream (high priority) while the LU of chunk c runs on the caller's; the GEMM
+// is tensor/epilogue work and the LU latency-bound CUDA-core work, so the two
+// share the SMs; events order the slot reuse of the two A buffers
+// (VMC_GB300_SERIAL_CHUNKS=1 runs the chunks back to back instead).  lane, fork,
+// join: the groups of walkers or connected configurations, one stream each.
 struct ChunkPipe {
-  int dev = -1;
   cudaStream_t aux = nullptr;
   cudaEvent_t h2 = nullptr, g[2] = {nullptr, nullptr}, lu[2] = {nullptr, nullptr};
-  bool ok = false;
-  // walker groups of a sweep (vmc_nnbf_sweep): one stream each, fork/join events
   static constexpr int kLanes = 4;
   cudaStream_t lane[kLanes] = {};
   cudaEvent_t fork = nullptr, join[kLanes] = {};
   bool lanes_ok = false;
+  int state = 0;       // 0 not created, 1 usable, -1 creation failed
+  bool busy = false;   // lent to a call
+
+  void create() {
+    int lo = 0, hi = 0;
+    cudaDeviceGetStreamPriorityRange(&lo, &hi);
+    bool ok = cudaStreamCreateWithPriority(&aux, cudaStreamNonBlocking, hi) == cudaSuccess;
+    ok = ok && cudaEventCreateWithFlags(&h2, cudaEventDisableTiming) == cudaSuccess;
+    for (int i = 0; i < 2; ++i) {
+      ok = ok && cudaEventCreateWithFlags(&g[i], cudaEventDisableTiming) == cudaSuccess;
+      ok = ok && cudaEventCreateWithFlags(&lu[i], cudaEventDisableTiming) == cudaSuccess;
+    }
+    lanes_ok = ok && cudaEventCreateWithFlags(&fork, cudaEventDisableTiming) == cudaSuccess;
+    for (int i = 0; i < kLanes; ++i) {
+      lanes_ok = lanes_ok && cudaStreamCreateWithFlags(&lane[i], cudaStreamNonBlocking) == cudaSuccess;
+      lanes_ok = lanes_ok && cudaEventCreateWithFlags(&join[i], cudaEventDisableTiming) == cudaSuccess;
+    }
+    state = ok ? 1 : -1;
+  }
 };
-ChunkPipe g_pipe[16];
+
+// A call borrows a set while it queues its work (another thread that recorded
+// the same events in between would have this call's streams wait for the
+// wrong point) and gives it back on return: what it queued stays ordered by the
+// streams themselves, and the caller's stream waits for it.  A stream that a
+// capture has joined belongs to it until it ends, beyond the call, so a set
+// whose streams take part in a capture is lent to calls of that capture only.
+// No set free: the call runs on its caller's stream alone.
+constexpr int kPipeDevices = 16, kPipes = 4;
+ChunkPipe g_pipe[kPipeDevices][kPipes];
 std::mutex g_pipe_mu;
 
-ChunkPipe* chunk_pipe() {
-  static const bool serial = [] {
-    const char* e = std::getenv("VMC_GB300_SERIAL_CHUNKS");
-    return e && e[0] == '1';
-  }();
-  if (serial) return nullptr;
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 16) return nullptr;
-  std::lock_guard<std::mutex> lk(g_pipe_mu);
-  ChunkPipe& p = g_pipe[dev];
-  if (p.dev == dev) return p.ok ? &p : nullptr;
-  p.dev = dev;
-  int lo = 0, hi = 0;
-  cudaDeviceGetStreamPriorityRange(&lo, &hi);
-  bool ok = cudaStreamCreateWithPriority(&p.aux, cudaStreamNonBlocking, hi) == cudaSuccess;
-  ok = ok && cudaEventCreateWithFlags(&p.h2, cudaEventDisableTiming) == cudaSuccess;
-  for (int i = 0; i < 2; ++i) {
-    ok = ok && cudaEventCreateWithFlags(&p.g[i], cudaEventDisableTiming) == cudaSuccess;
-    ok = ok && cudaEventCreateWithFlags(&p.lu[i], cudaEventDisableTiming) == cudaSuccess;
+class PipeLease {
+ public:
+  PipeLease() = default;
+  PipeLease(const PipeLease&) = delete;
+  PipeLease& operator=(const PipeLease&) = delete;
+  ~PipeLease() { release(); }
+  void release() {
+    if (!p_) return;
+    std::lock_guard<std::mutex> lk(g_pipe_mu);
+    p_->busy = false;
+    p_ = nullptr;
   }
-  bool lok = ok && cudaEventCreateWithFlags(&p.fork, cudaEventDisableTiming) == cudaSuccess;
-  for (int i = 0; i < ChunkPipe::kLanes; ++i) {
-    lok = lok && cudaStreamCreateWithFlags(&p.lane[i], cudaStreamNonBlocking) == cudaSuccess;
-    lok = lok && cudaEventCreateWithFlags(&p.join[i], cudaEventDisableTiming) == cudaSuccess;
+  ChunkPipe* acquire(cudaStream_t st) {
+    static const bool serial = [] {
+      const char* e = std::getenv("VMC_GB300_SERIAL_CHUNKS");
+      return e && e[0] == '1';
+    }();
+    int dev = 0;
+    if (serial || cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kPipeDevices) return nullptr;
+    const unsigned long long id = capture_id(st);
+    std::lock_guard<std::mutex> lk(g_pipe_mu);
+    for (ChunkPipe& p : g_pipe[dev]) {
+      if (p.busy || p.state < 0) continue;
+      if (p.state == 0) p.create();
+      if (p.state != 1 || !fits(p, id)) continue;
+      p.busy = true;
+      p_ = &p;
+      return p_;
+    }
+    return nullptr;
   }
-  p.lanes_ok = lok;
-  p.ok = ok;
-  return ok ? &p : nullptr;
-}
+
+ private:
+  ChunkPipe* p_ = nullptr;
+  // 0: not capturing
+  static unsigned long long capture_id(cudaStream_t st) {
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    unsigned long long id = 0;
+    if (cudaStreamGetCaptureInfo(st, &status, &id) != cudaSuccess) {
+      cudaGetLastError();   // the legacy stream beside another thread's capture
+      return 0;
+    }
+    if (status == cudaStreamCaptureStatusInvalidated) return ~0ull;
+    return status == cudaStreamCaptureStatusNone ? 0 : id;
+  }
+  static bool fits(const ChunkPipe& p, unsigned long long id) {
+    auto ok = [id](cudaStream_t s) {
+      const unsigned long long i = s ? capture_id(s) : 0;
+      return i == 0 || i == id;
+    };
+    bool all = ok(p.aux);
+    for (cudaStream_t s : p.lane) all = all && ok(s);
+    return all;
+  }
+};
 
 // Least walkers of a group: a group's kernels must still fill the GPU for most
 // of their time, or its second stream only adds gaps that a single stream of
@@ -1601,7 +1654,8 @@ int launch_eval_rows(int prec, int64_t R, int N, int nf, const uint64_t* row_occ
     const size_t lsmem = wpb * 128 * sizeof(float);  // two pivot-row slots per warp
     // chunk pipeline (two A slots inside the R-row workspace) unless the
     // stages are being timed one by one
-    ChunkPipe* pipe = (allow_pipe && n_chunks > 1 && !g_timer.acc) ? chunk_pipe() : nullptr;
+    PipeLease lease;
+    ChunkPipe* pipe = (allow_pipe && n_chunks > 1 && !g_timer.acc) ? lease.acquire(st) : nullptr;
     if (pipe) {
       if (cudaEventRecord(pipe->h2, st) != cudaSuccess || cudaStreamWaitEvent(pipe->aux, pipe->h2, 0) != cudaSuccess)
         return VMC_ERR_CUDA;
@@ -1800,15 +1854,17 @@ int vmc_nnbf_sweep(int prec, const void* const* net_ptrs, int n_sites, int nf, i
     if (cudaMemsetAsync(ccnt, 0, 2 * ChunkPipe::kLanes * sizeof(int), st) != cudaSuccess) return VMC_ERR_CUDA;
   }
   // walker groups on their own streams (mixed precision, untimed stages, B >= 2 groups)
+  PipeLease lease;
   ChunkPipe* pipe = nullptr;
   int G = 1;
   if (prec == 0 && !stage_ms && sweep_lanes() > 1 && B >= 2 * kLaneRows) {
-    pipe = chunk_pipe();
+    pipe = lease.acquire(st);
     if (pipe && pipe->lanes_ok) {
       G = sweep_lanes();
       if ((int64_t)G > B / kLaneRows) G = (int)(B / kLaneRows);
     } else {
       pipe = nullptr;
+      lease.release();
     }
   }
   if (G > 1) {
@@ -1955,13 +2011,16 @@ int vmc_nnbf_local_energy(int prec, const void* const* net_ptrs, int n_sites, in
   // Mixed precision with a workspace of >= 2 chunks: the pair chunks are
   // independent, so G streams each take every G-th sub-chunk with their own
   // slice of the workspace (the walker-group scheme of vmc_nnbf_sweep).
+  PipeLease lease;
   ChunkPipe* pipe = nullptr;
   int G = 1;
   if (prec == 0 && !g_timer.acc && sweep_lanes() > 1 && chunk >= 2 * kChunkRows && P > kChunkRows) {
-    pipe = chunk_pipe();
+    pipe = lease.acquire(st);
     if (pipe && pipe->lanes_ok) {
       G = sweep_lanes();
       if ((int64_t)G > chunk / kChunkRows) G = (int)(chunk / kChunkRows);
+    } else {
+      lease.release();
     }
   }
   if (G > 1) {
