@@ -264,19 +264,20 @@ class MinSRGB300(PreconditionerGB300):
         else:
             _lib.call("vmc_sr_cholesky", _lib.ptr(T), Ns, Ns, _lib.ptr(flag), s)
         stages.mark("cholesky")
-        check = getattr(build_gram, "check", None)
-        if check is not None:
-            check()
         x = torch.empty(Ns, dtype=torch.float64, device=dev)
 
         def rhs():
             _lib.call("vmc_sr_rhs", _lib.ptr(E), Ns, Ebar, _lib.ptr(x), s)
 
-        # the solves are queued behind the factorisation before its outcome is
-        # read, so that the GPU does not wait for the host in between
+        # the solves are queued behind the factorisation before its outcome, or
+        # the Gram matrix's status, is read, so that the GPU does not wait for
+        # the host in between
         rhs()
         _lib.call("vmc_sr_cholesky_solve", _lib.ptr(T), Ns, Ns, _lib.ptr(x), s)
         stages.mark("solve")
+        check = getattr(build_gram, "check", None)
+        if check is not None:
+            check()
         info, err = flag.tolist()
         if err != 0:
             raise ValueError("vmc_sr_cholesky_tc: %s" % _lib.message(err))
