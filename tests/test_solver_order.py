@@ -55,3 +55,25 @@ def test_a_failed_gram_raises_before_its_factor_is_used(monkeypatch):
     E = torch.zeros(4, dtype=torch.float64)
     with pytest.raises(ValueError, match="vmc_sr_gram_tc"):
         opt.MinSRGB300._factor_solve(gram, E, 0.0, 4, 1e-3, torch.device("cpu"), opt._Stages(False))
+
+
+def test_the_first_of_two_gram_products_is_not_forgotten(monkeypatch):
+    """The factored form makes two products; a status set by either is raised."""
+    calls = []
+
+    def call(name, *args):
+        if name == "vmc_sr_gram_tc":
+            calls.append(args[-2])
+            if len(calls) == 1:
+                args[-2][0] = 7
+
+    monkeypatch.setattr(opt, "_lib", types.SimpleNamespace(
+        call=call, ptr=lambda t: t, stream_of=lambda d: None, message=lambda v: "status %d" % v))
+    solver = opt.MinSRGB300()
+    dev = torch.device("cpu")
+    X, T = torch.ones(3, 5), torch.zeros(3, 3, dtype=torch.float64)
+    for _ in range(2):
+        solver._tc_gram(X, T, 1.0, None, 0.0, 0, dev)
+    assert len(calls) == 2
+    with pytest.raises(ValueError, match="status 7"):
+        solver._check_tc()

@@ -153,6 +153,7 @@ class MinSRGB300(PreconditionerGB300):
         self.record_stages = record_stages
         self.last_stages = None
         self.gram = gram
+        self._tc_err = None
 
     # digit planes of an FP64 Gram matrix held at a time
     SLAB_BYTES = 2 << 30
@@ -160,6 +161,12 @@ class MinSRGB300(PreconditionerGB300):
     # (vmc_sr_cholesky_tc): at 513 the two take the same time (1.13 ms: the
     # chain of 64-column tiles), at 2049 4.4 against 5.2 ms, at 8192 29 against 85
     CHOLESKY_TC_MIN = 513
+
+    def _status(self, dev):
+        """The device status word of a solve's tensor-core products."""
+        if self._tc_err is None or dev.index not in (None, self._tc_err.device.index):
+            self._tc_err = torch.zeros(1, dtype=torch.int32, device=dev)
+        return self._tc_err
 
     def _tc_gram(self, X, T, alpha, D, shift, accumulate, dev):
         """T [+]= alpha (X X^T) o D [+ shift I] on the tensor cores, X FP32 (Ns, K)."""
@@ -169,10 +176,9 @@ class MinSRGB300(PreconditionerGB300):
         planes = torch.empty(3 * rp * kp, dtype=torch.bfloat16, device=dev)
         rexp = torch.empty(rp, dtype=torch.int32, device=dev)
         _lib.call("vmc_split_bf16x3", _lib.ptr(X), Ns, K, X.stride(0), _lib.ptr(planes), rp, kp, _lib.ptr(rexp), s)
-        err = torch.zeros(1, dtype=torch.int32, device=dev)
+        err = self._status(dev)
         _lib.call("vmc_sr_gram_tc", _lib.ptr(planes), _lib.ptr(rexp), Ns, rp, kp, float(alpha), _lib.ptr(T),
                   T.stride(0), _lib.ptr(D), float(shift), int(accumulate), _lib.ptr(err), s)
-        self._tc_err = err
         del planes
 
     def _tc_gram_f64(self, X, T, shift, dev):
@@ -186,7 +192,7 @@ class MinSRGB300(PreconditionerGB300):
         kp = -(-min(K, slab) // 32) * 32
         planes = torch.empty(7 * rp * kp, dtype=torch.bfloat16, device=dev)
         rexp = torch.empty(rp, dtype=torch.int32, device=dev)
-        err = torch.zeros(1, dtype=torch.int32, device=dev)
+        err = self._status(dev)
         for a in range(0, K, slab):
             k = min(slab, K - a)
             kp = -(-k // 32) * 32
@@ -194,12 +200,11 @@ class MinSRGB300(PreconditionerGB300):
                       _lib.ptr(rexp), s)
             _lib.call("vmc_sr_gram_f64_tc", _lib.ptr(planes), _lib.ptr(rexp), Ns, rp, kp, _lib.ptr(T), T.stride(0),
                       float(shift) if a + k == K else 0.0, int(a > 0), _lib.ptr(err), s)
-        self._tc_err = err
 
     def _check_tc(self):
-        err = getattr(self, "_tc_err", None)
-        if err is not None and int(err.item()) != 0:
-            raise ValueError("vmc_sr_gram_tc: %s" % _lib.message(int(err.item())))
+        err = 0 if self._tc_err is None else int(self._tc_err.item())
+        if err != 0:
+            raise ValueError("vmc_sr_gram_tc: %s" % _lib.message(err))
 
     def solve(self, *, local_o, local_energies, energy_mean, total_samples, n_params, diag_shift, device=None,
               run_sr=True):
@@ -212,6 +217,7 @@ class MinSRGB300(PreconditionerGB300):
 
     def _solve(self, local_o, local_energies, energy_mean, n_params, diag_shift, device, run_sr, t0):
         dev = torch.device(device) if device is not None else torch.device("cuda")
+        self._tc_err = None
         E = torch.as_tensor(local_energies, device=dev, dtype=torch.float64).contiguous()
         if isinstance(local_o, FactoredO):
             return self._solve_factored(local_o, E, float(energy_mean), n_params, float(diag_shift), dev, run_sr, t0)
