@@ -1275,8 +1275,9 @@ __global__ void __launch_bounds__(512)
 // operands (3 to 8 multiply-adds per load), the cotangent chain GX3 -> GX2 stays
 // in registers, and the sums over slices that make up dZ/dA2, dZ/dA3, dZ/dM and
 // dZ/dN are 4 x 4 register tiles over a split of the long index, folded by
-// shuffles.  Two CTAs per SM (107 KB each); the left environments are read
-// from the workspace (L1/L2).
+// shuffles.  One CTA per SM: 119 KB of shared memory (two would fit below 113
+// KB each), so that a thread has 255 registers and nothing is spilled; the left
+// environments are read from the workspace (L1/L2).
 // ---------------------------------------------------------------------------
 namespace pg {
 
@@ -1286,6 +1287,7 @@ constexpr int o_Y = 0, o_X2 = o_Y + 4096, o_X3 = o_X2 + 4 * SS, o_G3 = o_X3 + 4 
               o_M = o_F + 4096, o_N = o_M + 1024, o_Nt = o_N + 1024, o_GM = o_Nt + 1024, o_GN = o_GM + 1024,
               o_GA2 = o_GN + 2048, o_GA3 = o_GA2 + 256, o_GT = o_GA3 + 256, o_red = o_GT + 1024, o_col = o_red + 32;
 constexpr size_t SMEM = (size_t)(o_col + 6 * 256) * 4 + 16 * sizeof(int);
+static_assert(SMEM <= 227 * 1024, "one CTA per SM");
 
 // 16 partial sums over the 16 lanes that differ in lane bits 0..3 -> the total
 // of value (lane & 15) in every lane
@@ -1390,7 +1392,7 @@ __device__ __forceinline__ void forward4(float* sm, const float* E, const float*
   }
 }
 
-__global__ void __launch_bounds__(NT, 2)
+__global__ void __launch_bounds__(NT, 1)
     k_peps_grad_tiled(const float* __restrict__ tens, int Ly, const uint64_t* __restrict__ occ, int64_t R,
                       float* __restrict__ O, int64_t ldo, float* __restrict__ env) {
   constexpr int Lx = 6, D4 = 256, ESZ = 4096;
