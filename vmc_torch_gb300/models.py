@@ -674,14 +674,21 @@ class FPEPS_GB300(WavefunctionModel_GB300):
         return [[k for k in range(Ly - 1, 0, -1) if (cuts[a] >> k) & 1] for a in range(Lx // 2)]
 
     def _chi_work(self, st, rows=None):
-        rows = int(rows or min(st.B, self.chi_rows))
+        """(workspace, rows) of the boundary states of ``rows`` walkers or hop
+        terms at a time (default: the state's walkers, chi_rows at most), 4
+        states each, or 4 per row of a side where they are cached row by row
+        (197 KB a walker at 6x6, D = 4 in FP32).  The state keeps the one for
+        its walkers; a larger one is the call's."""
+        own = int(min(st.B, self.chi_rows))
+        rows = int(rows or own)
         nbytes = ctypes.c_int64(0)
         _lib.call("vmc_peps_chi_work_bytes", self._prec, self.Lx, self.Ly, self.D, self.chi, rows,
                   ctypes.byref(nbytes))
         w = st.extra.get("chi_work")
         if w is None or w.numel() < nbytes.value:
             w = torch.empty(nbytes.value, dtype=torch.uint8, device=st.device)
-            st.extra["chi_work"] = w
+            if rows <= own:
+                st.extra["chi_work"] = w
         return w, rows
 
     @staticmethod
