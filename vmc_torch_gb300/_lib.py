@@ -134,6 +134,18 @@ def stream_of(device=None):
     return ctypes.c_void_p(torch.cuda.current_stream(device).cuda_stream)
 
 
+def most_rows(alloc, rows, least=1):
+    """(rows, alloc(rows)) of a workspace whose size is a choice, with rows halved
+    down to ``least`` while device memory does not allow them."""
+    while True:
+        try:
+            return rows, alloc(rows)
+        except torch.OutOfMemoryError:
+            if rows <= least:
+                raise
+        rows = max(least, rows // 2)
+
+
 def call(name, *args):
     """Call an entry point and raise on a non-zero status."""
     st = getattr(load(), name)(*args)

@@ -518,10 +518,13 @@ class NNBF_GB300(WavefunctionModel_GB300):
         if self._prec != 0:
             _lib.call("vmc_nnbf_logpsi_grad", self._prec, *args, s)
             return
-        rows = max(1, min(st.B, self.GRAD_ROWS))
-        nbytes = ctypes.c_int64(0)
-        _lib.call("vmc_nnbf_grad_work_bytes", self.n_sites, self.n_fermions, rows, ctypes.byref(nbytes))
-        work = torch.empty(nbytes.value, dtype=torch.uint8, device=st.device)
+
+        def alloc(rows):
+            nbytes = ctypes.c_int64(0)
+            _lib.call("vmc_nnbf_grad_work_bytes", self.n_sites, self.n_fermions, rows, ctypes.byref(nbytes))
+            return torch.empty(nbytes.value, dtype=torch.uint8, device=st.device)
+
+        rows, work = _lib.most_rows(alloc, max(1, min(st.B, self.GRAD_ROWS)))
         _lib.call("vmc_nnbf_logpsi_grad_ws", *args, _lib.ptr(work), rows, s)
 
     def logpsi_grad(self, st, out=None):
@@ -554,10 +557,15 @@ class NNBF_GB300(WavefunctionModel_GB300):
         x = st.extra
         row = self.n_fermions ** 2 * x["A"].element_size()
         rows = min(P, self.ELOC_ROWS, self.ELOC_BYTES // row)
-        if rows <= st.B:
-            return st.B, x["H1"], x["H2"], x["A"]
-        return rows, *(torch.empty((rows,) + t.shape[1:], dtype=t.dtype, device=st.device)
-                       for t in (x["H1"], x["H2"], x["A"]))
+
+        def alloc(rows):
+            own = x["H1"], x["H2"], x["A"]
+            if rows <= st.B:
+                return own
+            return tuple(torch.empty((rows,) + t.shape[1:], dtype=t.dtype, device=st.device) for t in own)
+
+        rows, work = _lib.most_rows(alloc, max(rows, st.B), st.B)
+        return rows, *work
 
     def local_energy(self, st, H):
         ts, arr = self.net(st.device)
@@ -680,15 +688,19 @@ class FPEPS_GB300(WavefunctionModel_GB300):
         (197 KB a walker at 6x6, D = 4 in FP32).  The state keeps the one for
         its walkers; a larger one is the call's."""
         own = int(min(st.B, self.chi_rows))
-        rows = int(rows or own)
-        nbytes = ctypes.c_int64(0)
-        _lib.call("vmc_peps_chi_work_bytes", self._prec, self.Lx, self.Ly, self.D, self.chi, rows,
-                  ctypes.byref(nbytes))
-        w = st.extra.get("chi_work")
-        if w is None or w.numel() < nbytes.value:
-            w = torch.empty(nbytes.value, dtype=torch.uint8, device=st.device)
-            if rows <= own:
-                st.extra["chi_work"] = w
+
+        def alloc(rows):
+            nbytes = ctypes.c_int64(0)
+            _lib.call("vmc_peps_chi_work_bytes", self._prec, self.Lx, self.Ly, self.D, self.chi, rows,
+                      ctypes.byref(nbytes))
+            w = st.extra.get("chi_work")
+            if w is None or w.numel() < nbytes.value:
+                w = torch.empty(nbytes.value, dtype=torch.uint8, device=st.device)
+                if rows <= own:
+                    st.extra["chi_work"] = w
+            return w
+
+        rows, w = _lib.most_rows(alloc, int(rows or own))
         return w, rows
 
     @staticmethod

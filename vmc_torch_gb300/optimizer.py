@@ -184,13 +184,14 @@ class MinSRGB300(PreconditionerGB300):
     def _tc_gram_f64(self, X, T, shift, dev):
         """T = X X^T + shift I on the tensor cores, X FP64 (Ns, K); the digit
         planes (14 bytes per entry) are made for at most SLAB_BYTES of
-        columns at a time."""
+        columns at a time, fewer where memory does not allow that."""
         s = _lib.stream_of(dev)
         Ns, K = X.shape
         rp = -(-Ns // 128) * 128
-        slab = max(256, self.SLAB_BYTES // (14 * rp) // 256 * 256)
-        kp = -(-min(K, slab) // 32) * 32
-        planes = torch.empty(7 * rp * kp, dtype=torch.bfloat16, device=dev)
+        n = min(-(-K // 256), max(1, self.SLAB_BYTES // (14 * rp) // 256))   # a slab's blocks of 256 columns
+        n, planes = _lib.most_rows(
+            lambda n: torch.empty(7 * rp * min(256 * n, -(-K // 32) * 32), dtype=torch.bfloat16, device=dev), n)
+        slab = 256 * n
         rexp = torch.empty(rp, dtype=torch.int32, device=dev)
         err = self._status(dev)
         for a in range(0, K, slab):
