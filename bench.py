@@ -717,13 +717,13 @@ def run_gb300(args):
     d2h = B * LX * LY * 8 + 2 * B * 8
     n_chunks = -(-B // 4096)
     # Launches of the timed steps.  The sweep runs G walker groups (the library
-    # splits B >= 8192 walkers into min(VMC_GB300_SWEEP_LANES, B // 4096)
+    # splits B >= 4096 walkers into min(VMC_GB300_SWEEP_LANES, B // 2048)
     # groups, default 4), each launching per edge a prep kernel, the hidden
     # GEMM and (backflow GEMM + LU) per 4096-row chunk of the group; per step
     # also the refresh (prep, hidden GEMM, n_chunks x (backflow GEMM + LU)) and
     # the unpack of the configurations.
     lanes = max(1, min(4, int(os.environ.get("VMC_GB300_SWEEP_LANES", "4"))))
-    G = min(lanes, B // 4096) if B >= 2 * 4096 and lanes > 1 else 1
+    G = min(lanes, B // 2048) if B >= 2 * 2048 and lanes > 1 else 1
     bg = -(-B // G)
     per_edge = sum(2 + 2 * -(-min(bg, B - g * bg) // 4096) for g in range(G) if g * bg < B)
     gpu_launches = args.steps * (E * per_edge + 2 + 2 * n_chunks + 1)

@@ -120,14 +120,15 @@ int vmc_slater_logpsi_grad(const double* G, const uint8_t* slot_orb, int64_t B, 
  * and VMC_ERR_ARGS if a configuration evaluated from scratch has an occupation
  * bit at or above n_sites or other than nf electrons (its result is then
  * meaningless; bits above n_sites are ignored, never used as indices).
- * Streams: work is enqueued on `stream`; for R > 4096 (mixed precision) the
- * call may fork part of it onto library-owned streams (one high-priority stream
- * for the next chunk's backflow GEMM, up to four for independent walker groups),
- * created once per device and shared by all callers, and joins them back into
- * `stream` by events before it returns, on error paths too.  Calls issued
- * concurrently from several host threads therefore share those streams.
- * Environment: VMC_GB300_SERIAL_CHUNKS=1 / VMC_GB300_SWEEP_LANES=1 keep all
- * work on `stream`.
+ * Streams: work is enqueued on `stream`; for R > 4096 (sweeps: B >= 4096; local
+ * energies: chunk >= 8192; mixed precision) the call may fork part of it onto
+ * library-owned streams (one high-priority stream for the chunk pipeline, up to
+ * four for groups of walkers or connected configurations), which it joins back
+ * into `stream` by events before it returns, on error paths too.  There are four
+ * sets of them per device; a call borrows one while it queues its work, and
+ * stays on `stream` when none is free.  A set that a stream capture has joined is
+ * lent to calls of that capture only.  VMC_GB300_SERIAL_CHUNKS=1 keeps all work
+ * on `stream`, VMC_GB300_SWEEP_LANES=1 the groups.
  * Amplitude results: a singular orbital matrix gives sign 0 and logabs -inf; a
  * NaN or Inf entry (non-finite parameters) gives NaN for both, as the
  * reference's NaN amplitude.  Metropolis tests never accept a NaN ratio; from a
@@ -323,6 +324,9 @@ int vmc_sr_cholesky(double* T, int64_t n, int64_t ldt, int* d_info, void* stream
  *   below 2^-1022 count as zero.
  * vmc_sr_cholesky_tc: as vmc_sr_cholesky with the trailing updates done this
  *   way; work (256-byte aligned) of *bytes from vmc_sr_cholesky_tc_work_bytes.
+ *   From order 2560, and not under stream capture, the panels are factored on a
+ *   high-priority stream of the library, one call at a time, joined back into
+ *   `stream` before the call returns.
  * d_err (device int) receives VMC_ERR_TIMEOUT if a bounded wait gave up. */
 int vmc_split_f64(const double* X, int64_t rows, int64_t K, int64_t ldx, void* planes, int64_t rows_pad, int64_t kp,
                   int* row_exp, void* stream);

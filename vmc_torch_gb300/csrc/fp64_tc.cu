@@ -601,7 +601,7 @@ int factor_step(double* T, int64_t ldt, int64_t n, int64_t k0, int* d_info, cuda
       g_trsm_attr[dev] = true;
     }
     // a row's chain is the shorter the more lanes share it, while the CTAs fit
-    // the GPU at once: 16 lanes to two CTAs an SM
+    // the GPU at once: 16 lanes to two CTAs of 8 rows on each of 152 SMs
     if (rest <= 2432) k_trsm64<16><<<(unsigned)((rest + 7) / 8), 128, TRSM_SMEM, st>>>(D, ldt, rest);
     else k_trsm64<4><<<(unsigned)((rest + 31) / 32), 128, TRSM_SMEM, st>>>(D, ldt, rest);
   }

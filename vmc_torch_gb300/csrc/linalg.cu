@@ -62,7 +62,7 @@ struct TileAcc {
 // respectively one passes over 3.8 GB take 1.7 and 0.6 at the measured rate.
 constexpr int CW = 8;                    // warps a CTA
 constexpr int CB = 128;                  // rows a block of the loops below
-constexpr int64_t CWIDE = 128 * 304;     // columns from which NC = 4
+constexpr int64_t CWIDE = 128 * 304;     // columns from which NC = 4: two CTAs on each of 152 SMs
 
 // Terms of a group of rows are summed in FP32 words while the largest lies in
 // [2^-85, 2^96): sums of 2^28 rows stay below FP32's largest number, and what

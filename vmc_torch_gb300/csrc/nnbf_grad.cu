@@ -639,7 +639,7 @@ __global__ void __launch_bounds__(256) k_g_write(int N, int nf, float s, const u
   }
 }
 
-// Slices of dh2's K: enough CTAs for two per SM, at most 16.
+// Slices of dh2's K: enough CTAs for two on each of 152 SMs, at most 16.
 int g_splits(int64_t R) {
   const int64_t tiles = (R + sg::BM - 1) / sg::BM * (HID / sg::BN);
   int64_t z = 304 / tiles;

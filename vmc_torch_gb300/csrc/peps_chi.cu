@@ -29,8 +29,8 @@
 // singular vectors.  Otherwise the block's Gram matrix by two-sided Jacobi.
 // The chi largest singular values over both blocks select the kept vectors U
 // and the state becomes U U^T M, the SVD truncation.  Precision "fp64" runs
-// everything in FP64, "fp32" the state and the Jacobi in FP32 with FP64
-// accumulation of the final overlap.
+// everything in FP64, "fp32" the state and the Jacobi in FP32 with the final
+// overlap to FP64 accuracy.
 //
 // Log-derivatives: the cotangent of each side's truncation against the other
 // side's truncated state (first-order change of the kept singular subspace),

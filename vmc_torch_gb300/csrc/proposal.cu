@@ -723,7 +723,7 @@ int vmc_prop_train_step(int n_sites, const int32_t* edges, int n_edges, const ui
   float* DL = LG + (size_t)R * PLOG;    // R x 256 dlogits
   auto tiles = [](int v) { return (unsigned)((v + sg::BM - 1) / sg::BM); };
   // weight gradients: K = R (the batch), split so that the few tiles of a
-  // 512-wide product make about four CTAs per SM; the partial sums land
+  // 512-wide product make about four CTAs on each of 152 SMs; the partial sums land
   // atomically in the cleared gradient vector
   auto wgrad = [&](int M, int N, const float* A, int lda, const float* Bm, int ldb, float* C) {
     const int t = (int)(tiles(M) * tiles(N));
