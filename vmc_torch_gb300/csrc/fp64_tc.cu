@@ -422,13 +422,10 @@ __global__ void k_syrk_df(const double* __restrict__ A, int64_t lda, int64_t n, 
       for (int q = 0; q < 4; ++q)
 #pragma unroll
         for (int r = 0; r < 4; ++r) {
-          const float p = ah[q] * bh[r];
+          const float p = __fmul_rn(ah[q], bh[r]);
           const float e = fmaf(ah[q], bh[r], -p);
           sm[q][r] += e + fmaf(ah[q], bl[r], al[q] * bh[r]);
-          const float s2 = hs[q][r] + p;
-          const float bb = s2 - hs[q][r];
-          hc[q][r] += (hs[q][r] - (s2 - bb)) + (p - bb);
-          hs[q][r] = s2;
+          hc[q][r] += vmc::two_sum(hs[q][r], p);
         }
     }
     __syncthreads();

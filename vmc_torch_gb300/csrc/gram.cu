@@ -143,14 +143,6 @@ __device__ __forceinline__ void tile_of(int t, int& bi, int& bj) {
   bj = t - i * (i + 1) / 2;
 }
 
-// a + b rounded into a, the rounding error returned
-__device__ __forceinline__ float two_sum(float& a, float b) {
-  const float s = __fadd_rn(a, b), bb = __fsub_rn(s, a);
-  const float e = __fadd_rn(__fsub_rn(a, __fsub_rn(s, bb)), __fsub_rn(b, bb));
-  a = s;
-  return e;
-}
-
 // t 2^e in the exponent field: t is 0, not finite, or of an exponent between
 // FP32's least and 2^31, and |e| < 300
 __device__ __forceinline__ double scale2(double t, int e) {
@@ -261,7 +253,7 @@ __global__ void __launch_bounds__(GR_THREADS, 1)
 #pragma unroll
         for (int q = 0; q < 8; ++q) {
           float h = hi[g * 8 + q];
-          const float e = two_sum(h, v[q]), f = two_sum(h, w[q]);
+          const float e = vmc::two_sum(h, v[q]), f = vmc::two_sum(h, w[q]);
           hi[g * 8 + q] = h;
           lo[g * 8 + q] += e + f;
         }
